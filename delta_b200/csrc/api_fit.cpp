@@ -440,17 +440,17 @@ struct Engine {
       launch_stamped_assemble(c.stream, G, n_units, nf, k, d_fold, As, rs, ds2, d_dsd, Mg, rg, yg);
       DGPU_CUDA(cudaStreamSynchronize(c.stream));
     } else {
-      uint8_t* fm = static_cast<uint8_t*>(c.slot(kSlotSeedNeg, std::max(n_units, 1)));
+      uint8_t* fm = static_cast<uint8_t*>(c.slot(kSlotSeedNeg, std::max<size_t>(static_cast<size_t>(G) * n_units, 1)));
       const auto hm = down(c, mask, n_units);
+      std::vector<uint8_t> m(static_cast<size_t>(G) * n_units);
+      for (int g = 0; g < G; ++g)
+        for (int u = 0; u < n_units; ++u) m[static_cast<size_t>(g) * n_units + u] = (hm[u] && fold[u] == g) ? 1 : 0;
+      DGPU_CUDA(h2d_async(fm, m.data(), m.size(), c.stream));
       for (int g = 0; g < G; ++g) {
-        std::vector<uint8_t> m(n_units);
-        for (int u = 0; u < n_units; ++u) m[u] = (hm[u] && fold[u] == g) ? 1 : 0;
-        DGPU_CUDA(h2d_async(fm, m.data(), n_units, c.stream));
+        const uint8_t* fg = fm + static_cast<size_t>(g) * n_units;
         long long* dummy = nall + 1;
-        launch_rhs(c, N, nc, k, SS, R, fm, nullptr, rg + static_cast<size_t>(g) * P, yg + g, dummy);
-        launch_normal_equations(c, prec, N, nc, k, SS, R, fm,
-                                Mg + g * PP);
-        DGPU_CUDA(cudaStreamSynchronize(c.stream));
+        launch_rhs(c, N, nc, k, SS, R, fg, nullptr, rg + static_cast<size_t>(g) * P, yg + g, dummy);
+        launch_normal_equations(c, prec, N, nc, k, SS, R, fg, Mg + g * PP);
       }
     }
     launch_fold_train(c.stream, G, PP, Mg, Mall, Mt);

@@ -85,7 +85,7 @@ enum Slot : int {
   kSlotFit0, kSlotFit1, kSlotFit2, kSlotFit3, kSlotFit4, kSlotFit5, kSlotFit6, kSlotFit7,
   kSlotFit8, kSlotFit9, kSlotFit10, kSlotFit11, kSlotFit12, kSlotFit13, kSlotFit14, kSlotFit15,
   kSlotFft0, kSlotFft1, kSlotFft2, kSlotFft3, kSlotFft4, kSlotFft5,
-  kSlotGlsPart, kSlotLdlt,
+  kSlotGlsPart, kSlotLdlt, kSlotRowList,
   kSlotGrad0, kSlotGrad1, kSlotGrad2, kSlotGrad3, kSlotGrad4, kSlotGrad5, kSlotGrad6, kSlotGrad7,
   kSlotBatch0, kSlotBatch1, kSlotBatch2, kSlotBatch3, kSlotBatch4, kSlotBatch5, kSlotBatch6, kSlotBatch7,
   kSlotBatch8, kSlotBatch9, kSlotBatch10, kSlotBatch11,
