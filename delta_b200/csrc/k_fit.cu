@@ -346,6 +346,8 @@ k_normal_kron(int64_t N, int nc, int k, int SS, FitRows R, const uint8_t* __rest
 // a 32 MT x 48 tile; MT is picked so that the last tile row wastes least.
 // Two CTAs per SM: one generates its operands while the other multiplies, and
 // the raw rows of the next chunk arrive by cp.async meanwhile.
+// m8n8k4 rounds like four FMAs in k order, so each output is the sequential FMA
+// chain over its split's rows that the SIMT kernels form.
 // Only active rows are visited: k_row_list compacts them in row order, so a
 // cross-validation fold costs its own fifth of the rows. 1.9e5 rows x 435 x
 // 136 products: 3.39 ms with the SIMT kernel this replaced, 0.97 ms now (25
@@ -377,10 +379,11 @@ k_row_count(int64_t N, int SS, const uint8_t* __restrict__ valid, const uint8_t*
   }
 }
 
-// list[1..] = the active rows in row order, list[0] = how many.
+// list = the active rows in row order; starts[z] = position of the first one at
+// or after row z rps (rps a multiple of 32), starts[ceil(N / rps)] = how many.
 __global__ void __launch_bounds__(256)
 k_row_list(int64_t N, int SS, const uint8_t* __restrict__ valid, const uint8_t* __restrict__ accepted,
-           const int* __restrict__ counts, int* __restrict__ list) {
+           const int* __restrict__ counts, int64_t rps, int* __restrict__ list, int* __restrict__ starts) {
   __shared__ int ws[8], wc[8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int before = 0;
@@ -407,10 +410,12 @@ k_row_list(int64_t N, int SS, const uint8_t* __restrict__ valid, const uint8_t* 
   }
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    if (act[i] & (1u << lane)) list[1 + at + __popc(act[i] & ((1u << lane) - 1u))] = static_cast<int>(base + 32 * i + lane);
+    const int64_t r0 = base + 32 * i;
+    if (lane == 0 && r0 < N && r0 % rps == 0) starts[r0 / rps] = at;
+    if (act[i] & (1u << lane)) list[at + __popc(act[i] & ((1u << lane) - 1u))] = static_cast<int>(r0 + lane);
     at += __popc(act[i]);
   }
-  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) list[0] = total;
+  if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) starts[(N + rps - 1) / rps] = total;
 }
 
 constexpr int kNdK = 32;   // rows per chunk
@@ -435,8 +440,9 @@ inline size_t normal_dmma_smem(int mt, int nf, int k) {
 
 template <int MT>
 __global__ void __launch_bounds__(256, 2)
-k_normal_dmma(int nc, int k, FitRows R, const int* __restrict__ list, const int2* __restrict__ upairs, int Mu,
-              const int2* __restrict__ vpairs, int Nv, double* __restrict__ gpart) {
+k_normal_dmma(int nc, int k, FitRows R, const int* __restrict__ list, const int* __restrict__ starts,
+              const int2* __restrict__ upairs, int Mu, const int2* __restrict__ vpairs, int Nv,
+              double* __restrict__ gpart) {
   extern __shared__ __align__(16) double nsm[];
   constexpr int BM = 32 * MT, LU = BM + 4;
   const int nf = nc + 1, raw = nf + k + 1;  // a staged row: b (nc, then 1), d (k), w
@@ -445,9 +451,7 @@ k_normal_dmma(int nc, int k, FitRows R, const int* __restrict__ list, const int2
   double* rows = Vs + kNdK * kNdLv;  // 2 x kNdK x raw
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane >> 2, kq = lane & 3;
   const int u0 = blockIdx.x * BM, v0 = blockIdx.y * kNdN;
-  const int n = list[0];
-  const int per = ((n + static_cast<int>(gridDim.z) - 1) / static_cast<int>(gridDim.z) + kNdK - 1) / kNdK * kNdK;
-  const int rbeg = min(n, static_cast<int>(blockIdx.z) * per), rend = min(n, rbeg + per);
+  const int rbeg = starts[blockIdx.z], rend = starts[blockIdx.z + 1];
   // This lane's operand columns: U lane + 32 i, V lane and (lanes below 16) 32 + lane.
   int2 up[MT], vp[2];
 #pragma unroll
@@ -461,7 +465,7 @@ k_normal_dmma(int nc, int k, FitRows R, const int* __restrict__ list, const int2
     for (int rr = warp; rr < kNdK; rr += 8) {
       const int r = r0 + rr;
       if (r >= rend) break;
-      const size_t row = static_cast<size_t>(list[1 + r]);
+      const size_t row = static_cast<size_t>(list[r]);
       double* o = dst + rr * raw;
       for (int c = lane; c < nc; c += 32) cp_async8(o + c, R.bn + row * nc + c);
       for (int m = lane; m < k; m += 32) cp_async8(o + nf + m, R.d + row * k + m);
@@ -528,32 +532,29 @@ k_normal_dmma(int nc, int k, FitRows R, const int* __restrict__ list, const int2
   }
 }
 
-// Partial sums of the splits into gpart (slot kSlotFit11); returns the number of splits.
-static int launch_normal_dmma(Context& c, int64_t N, int nc, int k, int SS, const FitRows& R, const uint8_t* accepted,
-                              const int2* upairs, int Mu, const int2* vpairs, int Nv, double** gpart) {
+// Partial sums of nsplit splits of rps rows into gpart.
+static void launch_normal_dmma(Context& c, int64_t N, int nc, int k, int SS, const FitRows& R, const uint8_t* accepted,
+                               const int2* upairs, int Mu, const int2* vpairs, int Nv, int64_t rps, int nsplit,
+                               double* gpart) {
   cudaStream_t st = c.stream;
   if (N >= (int64_t(1) << 31) - kListRows) fail(DGPU_ERR_INVALID, "fit: too many rows");
   const int nblk = static_cast<int>((N + kListRows - 1) / kListRows);
-  int* counts = static_cast<int*>(c.slot(kSlotRowList, sizeof(int) * (static_cast<size_t>(nblk) + 1 + N)));
-  int* list = counts + nblk;
+  int* counts = static_cast<int*>(c.slot(kSlotRowList, sizeof(int) * (static_cast<size_t>(nblk) + nsplit + 1 + N)));
+  int* starts = counts + nblk;
+  int* list = starts + nsplit + 1;
   k_row_count<<<nblk, 256, 0, st>>>(N, SS, R.valid, accepted, counts);
   DGPU_LAUNCH("k_row_count");
-  k_row_list<<<nblk, 256, 0, st>>>(N, SS, R.valid, accepted, counts, list);
+  k_row_list<<<nblk, 256, 0, st>>>(N, SS, R.valid, accepted, counts, rps, list, starts);
   DGPU_LAUNCH("k_row_list");
   // Tile height 32 MT with the least padding of Mu (the taller one on a tie).
   int mt = 1;
   for (int t = 2; t <= 7; ++t)
     if ((Mu + 32 * t - 1) / (32 * t) * (32 * t) <= (Mu + 32 * mt - 1) / (32 * mt) * (32 * mt)) mt = t;
-  const int gx = (Mu + 32 * mt - 1) / (32 * mt), gy = (Nv + kNdN - 1) / kNdN;
-  // One wave of two CTAs per SM, at least two chunks of rows each.
-  const int64_t want = std::max<int64_t>(1, 148 * 2 / (gx * gy)), most = std::max<int64_t>(1, N / (2 * kNdK));
-  const int nsplit = static_cast<int>(std::min(want, most));
-  *gpart = static_cast<double*>(c.slot(kSlotFit11, sizeof(double) * static_cast<size_t>(nsplit) * Mu * Nv));
   const size_t smem = normal_dmma_smem(mt, nc + 1, k);
-  const dim3 grid(gx, gy, nsplit);
+  const dim3 grid((Mu + 32 * mt - 1) / (32 * mt), (Nv + kNdN - 1) / kNdN, nsplit);
   auto go = [&](auto kern) {
     ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
-    kern<<<grid, 256, smem, st>>>(nc, k, R, list, upairs, Mu, vpairs, Nv, *gpart);
+    kern<<<grid, 256, smem, st>>>(nc, k, R, list, starts, upairs, Mu, vpairs, Nv, gpart);
   };
   switch (mt) {
     case 1: go(k_normal_dmma<1>); break;
@@ -565,7 +566,6 @@ static int launch_normal_dmma(Context& c, int64_t N, int nc, int k, int SS, cons
     default: go(k_normal_dmma<7>); break;
   }
   DGPU_LAUNCH("k_normal_dmma");
-  return nsplit;
 }
 
 // G = sum_z gpart[z] (fixed order), then M[p][q] = G[{c,c'}][{m,m'}].
@@ -613,21 +613,20 @@ void launch_normal_equations(Context& c, int prec, int64_t N, int nc, int k, int
     launch_normal_tc(c, N, nc, k, SS, R, accepted, dpairs, Mu, dpairs + Mu, Nv, kSlotFit11, g,
                      prec == DGPU_PREC_TF32);
   } else {
-    double* gpart = nullptr;
-    int nsplit;
+    const int gx = (Mu + kNeT - 1) / kNeT, gy = (Nv + kNeT - 1) / kNeT;
+    // Split K (rows) so the grid covers the GPU a few times over (the FP64
+    // kernel's taller tiles: about once, two CTAs per SM).
+    const int64_t target_splits = std::max<int64_t>(1, (148 * 6) / (gx * gy));
+    int64_t rps = std::max<int64_t>(kNeR * 8, (N + target_splits - 1) / target_splits);
+    rps = (rps + kNeR - 1) / kNeR * kNeR;
+    const int nsplit = static_cast<int>((N + rps - 1) / rps);
+    double* gpart = static_cast<double*>(c.slot(kSlotFit11, sizeof(double) * static_cast<size_t>(nsplit) * Mu * Nv));
     if (prec == DGPU_PREC_FP32) {
-      const int gx = (Mu + kNeT - 1) / kNeT, gy = (Nv + kNeT - 1) / kNeT;
-      // Split K (rows) so the grid covers the GPU a few times over.
-      const int64_t target_splits = std::max<int64_t>(1, (148 * 6) / (gx * gy));
-      int64_t rps = std::max<int64_t>(kNeR * 8, (N + target_splits - 1) / target_splits);
-      rps = (rps + kNeR - 1) / kNeR * kNeR;
-      nsplit = static_cast<int>((N + rps - 1) / rps);
-      gpart = static_cast<double*>(c.slot(kSlotFit11, sizeof(double) * static_cast<size_t>(nsplit) * Mu * Nv));
       k_normal_kron<<<dim3(gx, gy, nsplit), 256, 0, st>>>(N, nc, k, SS, R, accepted, dpairs, Mu, dpairs + Mu, Nv, rps,
                                                           gpart);
       DGPU_LAUNCH("k_normal_kron");
     } else {
-      nsplit = launch_normal_dmma(c, N, nc, k, SS, R, accepted, dpairs, Mu, dpairs + Mu, Nv, &gpart);
+      launch_normal_dmma(c, N, nc, k, SS, R, accepted, dpairs, Mu, dpairs + Mu, Nv, rps, nsplit, gpart);
     }
     k_reduce_g<<<std::min(148 * 4, (Mu * Nv + 255) / 256), 256, 0, st>>>(nsplit, Mu * Nv, gpart, g);
     DGPU_LAUNCH("k_reduce_g");
