@@ -995,7 +995,7 @@ int dgpu_stamp_gcv(dgpu_context* ctx, int mem, int64_t width, int64_t height, co
     launch_quad_err(c, 1, P, work, M, nullptr, rhs, nullptr, ywy, raw);
     launch_gcv_stats(st, P, k, rk, X, E.d_fk, lam, raw, n, work, scal);
     const int nq = m - 1;
-    double* out6 = static_cast<double*>(c.slot(kSlotGrad7, sizeof(double) * (6 * static_cast<size_t>(gcv_rows_blocks(N)) + 8)));
+    double* out6 = static_cast<double*>(c.slot(kSlotGrad7, sizeof(double) * (gcv_rows_doubles(N, nc, k) + 8)));
     if (grad_gcv || grad_rss) {
       GcvRowsArgs a;
       a.N = N;
@@ -1014,8 +1014,7 @@ int dgpu_stamp_gcv(dgpu_context* ctx, int mem, int64_t width, int64_t height, co
       a.X = X;
       a.scal = scal;
       a.scale = scale;
-      a.partial = out6 + 8;
-      launch_gcv_rows(st, a, out6);
+      launch_gcv_rows(st, a, out6 + 8, out6);
     }
     GcvScalars hs{};
     double g6[6] = {0, 0, 0, 0, 0, 0};

@@ -28,7 +28,7 @@ struct GcvRowsArgs {
   const double* X = nullptr;        // P x (1 + nq): [theta | H], row-major
   const GcvScalars* scal = nullptr;
   double scale = 1.0;
-  double* partial = nullptr;        // gcv_rows_blocks x 6
+  double* partial = nullptr;        // 6 per block of 128 rows (set by launch_gcv_rows)
 };
 
 int gcv_rhs_cols(int P, int k, int r);
@@ -40,7 +40,8 @@ size_t gcv_stats_doubles(int P, int k, int r);
 void launch_gcv_theta(cudaStream_t st, int P, int k, int r, const double* X, const double* fk, double* work);
 void launch_gcv_stats(cudaStream_t st, int P, int k, int r, const double* X, const double* fk, double lam,
                       const double* raw, const long long* n, double* work, GcvScalars* scal);
-int gcv_rows_blocks(int64_t N);
-void launch_gcv_rows(cudaStream_t st, const GcvRowsArgs& a, double* out6);
+// work: gcv_rows_doubles of device memory, 16-byte aligned.
+size_t gcv_rows_doubles(int64_t N, int nc, int k);
+void launch_gcv_rows(cudaStream_t st, const GcvRowsArgs& a, double* work, double* out6);
 
 }  // namespace dgpu

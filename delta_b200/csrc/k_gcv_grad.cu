@@ -16,8 +16,8 @@
 // Back through X: Xbar = 2 W X Mbar + W t bbar^T, and per row
 // Ubar_c = sum_j d_j Xbar_(c,j); then dx += sum_c Ubar_c dU_c/ddx with
 // dU_c/ddx = -s B^x_n,c (the B_n of the x-derivative taps), dy alike, and
-// ds += sum_c Ubar_c u_c / s. The H H^T part is applied column by column of H
-// (Y_q = X_row h_q, then Y_q (d-contracted h_q)), so no P x P matrix is formed.
+// ds += sum_c Ubar_c u_c / s. The H H^T part is one product over all rows (see
+// k_gcv_edf).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -130,59 +130,58 @@ __global__ void k_gcv_scalars(int P, double lam, const double* __restrict__ sums
 }
 
 constexpr int kGrRows = 128;  // rows (threads) per block
-constexpr int kGrQc = 8;      // columns of H staged per step
 constexpr int kGrMaxK = 32;
 
-// Per block: {dGCV/ddx, dGCV/ddy, dGCV/ds, dRSS/ddx, dRSS/ddy, dRSS/ds} over its rows.
+// RSS part, a thread per row. Per block: {alpha dRSS/ddx, ddy, ds, dRSS/ddx, ddy, ds}
+// over its rows.
 __global__ void __launch_bounds__(kGrRows) k_gcv_rows(GcvRowsArgs a) {
   extern __shared__ __align__(16) double gsm[];
-  const int nc = a.nc, nf = nc + 1, k = a.k, P = nf * k, nq = a.nq, m = nq + 1;
-  double* sh = gsm;                             // P x kGrQc
-  double* su = sh + static_cast<size_t>(P) * kGrQc;  // nc x rows: u
-  double* sx = su + static_cast<size_t>(nc) * kGrRows;
-  double* sy = sx + static_cast<size_t>(nc) * kGrRows;
+  const int nc = a.nc, nf = nc + 1, k = a.k, P = nf * k;
+  double* st = gsm;    // theta
+  double* sz = st + P;  // z
   const int tid = threadIdx.x;
   const int64_t row = static_cast<int64_t>(blockIdx.x) * kGrRows + tid;
   const bool live = row < a.N && a.valid[row] && a.w[row] > 0.0;
   const GcvScalars S = *a.scal;
   const double wr = live ? a.w[row] : 0.0, tr = live ? a.t[row] : 0.0;
+  for (int p = tid; p < P; p += kGrRows) {
+    st[p] = a.theta[p];
+    sz[p] = a.z[p];
+  }
   double d[kGrMaxK];
 #pragma unroll
   for (int j = 0; j < kGrMaxK; ++j) d[j] = (live && j < k) ? a.d[row * k + j] : 0.0;
-  for (int c = 0; c < nc; ++c) {
-    su[c * kGrRows + tid] = live ? a.bn[row * nc + c] : 0.0;
-    sx[c * kGrRows + tid] = live ? a.bnx[row * nc + c] : 0.0;
-    sy[c * kGrRows + tid] = live ? a.bny[row * nc + c] : 0.0;
-  }
+  __syncthreads();
   double g[6] = {0, 0, 0, 0, 0, 0};
   const double inv_s = 1.0 / a.scale;
   if (live) {
-    // X theta and X z.
-    double xt = 0.0, xz = 0.0;
-    for (int c = 0; c < nf; ++c) {
-      double dt = 0.0, dz = 0.0;
+    const double* bn = a.bn + row * nc;
+    const double* bnx = a.bnx + row * nc;
+    const double* bny = a.bny + row * nc;
+    auto dots = [&](int c, double& dt, double& dz) {
+      dt = dz = 0.0;
 #pragma unroll
       for (int j = 0; j < kGrMaxK; ++j)
         if (j < k) {
-          dt = fma(d[j], a.theta[c * k + j], dt);
-          dz = fma(d[j], a.z[c * k + j], dz);
+          dt = fma(d[j], st[c * k + j], dt);
+          dz = fma(d[j], sz[c * k + j], dz);
         }
-      const double u = c < nc ? su[c * kGrRows + tid] : 1.0;
+    };
+    // X theta and X z.
+    double xt = 0.0, xz = 0.0;
+    for (int c = 0; c < nf; ++c) {
+      double dt, dz;
+      dots(c, dt, dz);
+      const double u = c < nc ? bn[c] : 1.0;
       xt = fma(u, dt, xt);
       xz = fma(u, dz, xz);
     }
     for (int c = 0; c < nc; ++c) {
-      double dt = 0.0, dz = 0.0;
-#pragma unroll
-      for (int j = 0; j < kGrMaxK; ++j)
-        if (j < k) {
-          dt = fma(d[j], a.theta[c * k + j], dt);
-          dz = fma(d[j], a.z[c * k + j], dz);
-        }
+      double dt, dz;
+      dots(c, dt, dz);
       // RSS part (alpha = 1): 2 w (X Mbar)_c + w t bbar_c, d-contracted.
       const double ur = 2.0 * wr * (xt * dt - 0.5 * (xz * dt + xt * dz)) + wr * tr * (-2.0 * dt + dz);
-      const double u = su[c * kGrRows + tid];
-      const double bx = sx[c * kGrRows + tid], by = sy[c * kGrRows + tid];
+      const double u = bn[c], bx = bnx[c], by = bny[c];
       g[3] -= ur * bx;
       g[4] -= ur * by;
       g[5] += ur * u * inv_s;
@@ -190,41 +189,6 @@ __global__ void __launch_bounds__(kGrRows) k_gcv_rows(GcvRowsArgs a) {
       g[0] -= ug * bx;
       g[1] -= ug * by;
       g[2] += ug * u * inv_s;
-    }
-  }
-  // dedf part of GCV: 2 w beta lambda sum_q Y_q (d-contracted h_q), Y_q = X_row h_q.
-  const double coef = 2.0 * wr * S.beta * S.lam;
-  for (int q0 = 0; q0 < nq; q0 += kGrQc) {
-    const int qn = min(kGrQc, nq - q0);
-    __syncthreads();
-    for (int e = tid; e < P * kGrQc; e += blockDim.x) {
-      const int p = e / kGrQc, qq = e - p * kGrQc;
-      sh[e] = qq < qn ? a.X[static_cast<size_t>(p) * m + 1 + q0 + qq] : 0.0;
-    }
-    __syncthreads();
-    if (!live) continue;
-    for (int qq = 0; qq < qn; ++qq) {
-      double yq = 0.0, sxq = 0.0, syq = 0.0, suq = 0.0;
-      for (int c = 0; c < nf; ++c) {
-        const double* hc = sh + static_cast<size_t>(c) * k * kGrQc + qq;
-        double dh = 0.0;
-#pragma unroll
-        for (int j = 0; j < kGrMaxK; ++j)
-          if (j < k) dh = fma(d[j], hc[j * kGrQc], dh);
-        if (c < nc) {
-          const double u = su[c * kGrRows + tid];
-          yq = fma(u, dh, yq);
-          suq = fma(u, dh, suq);
-          sxq = fma(sx[c * kGrRows + tid], dh, sxq);
-          syq = fma(sy[c * kGrRows + tid], dh, syq);
-        } else {
-          yq += dh;
-        }
-      }
-      const double cy = coef * yq;
-      g[0] -= cy * sxq;
-      g[1] -= cy * syq;
-      g[2] += cy * suq * inv_s;
     }
   }
   // Fixed-order block reduction.
@@ -240,6 +204,264 @@ __global__ void __launch_bounds__(kGrRows) k_gcv_rows(GcvRowsArgs a) {
     for (int w = 0; w < kGrRows / 32; ++w) t += red[tid][w];
     a.partial[static_cast<size_t>(blockIdx.x) * 6 + tid] = t;
   }
+}
+
+// ---------------------------------------------------------------------------
+// edf part of the GCV gradient.
+//
+// Per row, with K = H H^T and S_cc' = sum_mm' K_(c,m)(c',m') d_m d_m' (symmetric
+// in c, c'), the row's share of dedf/ddx is -2 w beta lambda sum_cc' bx_c S_cc' u_c'.
+// S over all rows is one product of the rows' design pairs V[i][{m,m'}] =
+// d_m d_m' (k (k+1) / 2 wide) with the packed Kp[{m,m'}][{c,c'}], so it runs on
+// the FP64 tensor cores and each S value is used where it is made: it meets
+// the weights of its pair (bx_c u_c' + bx_c' u_c for dx, alike for dy and the
+// scale) in the epilogue and is not stored. Contracting each row with the
+// nf r columns of H instead (X_row h_q, then its d-contraction) takes 3.5 times
+// the products on the vector pipe: 22.9 ms at 1.9e5 rows, P = 464; this way
+// 1.35 ms, bound by the DMMA pipe (13 GFMA with padding, 0.72 ms at 37 TFLOP/s).
+//
+// A CTA takes 128 rows x 16 NT pairs of components, eight warps of 32 x 8 NT,
+// the design pairs in chunks of 16: V is generated into one buffer while the
+// tensor cores read the other; Kp (zero padded) arrives by cp.async.
+// ---------------------------------------------------------------------------
+constexpr int kGeK = 16;             // design pairs per chunk
+constexpr int kGeLa = kGrRows + 4;   // row strides = 4 mod 16 doubles: conflict-free fragment loads
+
+__host__ __device__ inline int ge_pairs(int n) { return n * (n + 1) / 2; }
+__host__ __device__ inline int ge_pad(int n, int to) { return (n + to - 1) / to * to; }
+
+// (a, b), a <= b, of the idx-th pair in row-major order over the upper triangle of n.
+__device__ __forceinline__ int2 pair_of(int idx, int n) {
+  int a = 0, left = n;
+  while (idx >= left) {
+    idx -= left;
+    ++a;
+    --left;
+  }
+  return make_int2(a, a + idx);
+}
+
+__device__ __forceinline__ void dmma_gcv(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
+// K = H H^T (P x P), H the last nq columns of X (row stride m = nq + 1): a
+// 32 x 32 tile per CTA of four warps.
+__global__ void __launch_bounds__(128) k_hht(int P, int m, const double* __restrict__ X, double* __restrict__ K) {
+  __shared__ double A[32][36], B[32][36];
+  const int p0 = blockIdx.x * 32, q0 = blockIdx.y * 32, tid = threadIdx.x;
+  const int warp = tid >> 5, lane = tid & 31, q = lane >> 2, kq = lane & 3;
+  const int wr = (warp >> 1) * 16, wc = (warp & 1) * 16;
+  double acc[2][2][2] = {};
+  for (int c0 = 1; c0 < m; c0 += 32) {
+    __syncthreads();
+    for (int e = tid; e < 32 * 32; e += 128) {
+      const int r = e >> 5, c = e & 31;
+      A[r][c] = (p0 + r < P && c0 + c < m) ? X[static_cast<size_t>(p0 + r) * m + c0 + c] : 0.0;
+      B[r][c] = (q0 + r < P && c0 + c < m) ? X[static_cast<size_t>(q0 + r) * m + c0 + c] : 0.0;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k0 = 0; k0 < 32; k0 += 4) {
+      const double a0 = A[wr + q][k0 + kq], a1 = A[wr + 8 + q][k0 + kq];
+      const double b0 = B[wc + q][k0 + kq], b1 = B[wc + 8 + q][k0 + kq];
+      dmma_gcv(acc[0][0], a0, b0);
+      dmma_gcv(acc[0][1], a0, b1);
+      dmma_gcv(acc[1][0], a1, b0);
+      dmma_gcv(acc[1][1], a1, b1);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int r = p0 + wr + 8 * i + q, c = q0 + wc + 8 * j + 2 * kq + e;
+        if (r < P && c < P) K[static_cast<size_t>(r) * P + c] = acc[i][j][e];
+      }
+}
+
+// Kp[{m,m'}][{c,c'}] (vp x sp, zero padded): K_(c,m)(c',m') + K_(c,m')(c',m), once when m = m'.
+__global__ void __launch_bounds__(128) k_pack_k(int nf, int k, int sp, const double* __restrict__ K,
+                                                double* __restrict__ kp) {
+  const int v = blockIdx.x, P = nf * k;
+  const int2 mm = v < ge_pairs(k) ? pair_of(v, k) : make_int2(-1, -1);
+  for (int s = threadIdx.x; s < sp; s += blockDim.x) {
+    double x = 0.0;
+    if (mm.x >= 0 && s < ge_pairs(nf)) {
+      const int2 cc = pair_of(s, nf);
+      x = K[static_cast<size_t>(cc.x * k + mm.x) * P + cc.y * k + mm.y];
+      if (mm.x != mm.y) x += K[static_cast<size_t>(cc.x * k + mm.y) * P + cc.y * k + mm.x];
+    }
+    kp[static_cast<size_t>(v) * sp + s] = x;
+  }
+}
+
+template <int NT>
+__host__ __device__ constexpr int ge_lb() { return 16 * NT + 4; }
+// Main loop: 2 x V chunk, 2 x Kp chunk, the rows' design values (k x 128), the
+// pair table; epilogue, in the same memory: u, bx, by (nc x 128 each).
+template <int NT>
+size_t ge_smem(int nc, int k) {
+  const size_t main = sizeof(double) * (2 * kGeK * (kGeLa + ge_lb<NT>()) + static_cast<size_t>(k) * kGeLa) +
+                      sizeof(int2) * ge_pad(ge_pairs(k), kGeK);
+  return std::max(main, sizeof(double) * 3 * nc * kGeLa);
+}
+
+template <int NT>
+__global__ void __launch_bounds__(256, 2) k_gcv_edf(GcvRowsArgs a, const double* __restrict__ kp, int sp, int vp,
+                                                    double* __restrict__ part) {
+  extern __shared__ __align__(16) double gsm[];
+  constexpr int LB = ge_lb<NT>();
+  const int nc = a.nc, nf = nc + 1, k = a.k;
+  double* As = gsm;                        // 2 x kGeK x kGeLa
+  double* Bs = As + 2 * kGeK * kGeLa;      // 2 x kGeK x LB
+  double* sd = Bs + 2 * kGeK * LB;         // k x kGeLa
+  int2* pt = reinterpret_cast<int2*>(sd + k * kGeLa);
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane >> 2, kq = lane & 3;
+  const int64_t row0 = static_cast<int64_t>(blockIdx.x) * kGrRows;
+  const int s0 = blockIdx.y * 16 * NT;
+  const int myrow = tid & (kGrRows - 1);
+  auto live_row = [&](int r) { return row0 + r < a.N && a.valid[row0 + r] && a.w[row0 + r] > 0.0; };
+  auto load_b = [&](int v0, int buf) {
+    for (int e = tid; e < kGeK * 8 * NT; e += 256) {  // 16-byte pieces
+      const int r = e / (8 * NT), c = 2 * (e - r * 8 * NT);
+      const double* src = kp + static_cast<size_t>(v0 + r) * sp + s0 + c;
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(static_cast<uint32_t>(
+                       __cvta_generic_to_shared(Bs + (buf * kGeK + r) * LB + c))), "l"(src) : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  load_b(0, 0);
+  for (int e = tid; e < kGrRows * k; e += 256) {
+    const int r = e / k, j = e - r * k;
+    sd[j * kGeLa + r] = live_row(r) ? a.d[(row0 + r) * k + j] : 0.0;
+  }
+  for (int v = tid; v < vp; v += 256) pt[v] = v < ge_pairs(k) ? pair_of(v, k) : make_int2(-1, -1);
+  __syncthreads();
+  auto gen = [&](int v0, int buf) {
+    const int h = (tid >> 7) * (kGeK / 2);
+#pragma unroll
+    for (int j = 0; j < kGeK / 2; ++j) {
+      const int2 p = pt[v0 + h + j];
+      As[(buf * kGeK + h + j) * kGeLa + myrow] = p.x >= 0 ? sd[p.x * kGeLa + myrow] * sd[p.y * kGeLa + myrow] : 0.0;
+    }
+  };
+  gen(0, 0);
+  double acc[4][NT][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int wm = (warp >> 1) * 32, wn = (warp & 1) * 8 * NT;
+  int buf = 0;
+  for (int v0 = 0; v0 < vp; v0 += kGeK, buf ^= 1) {
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();  // this chunk is in place; the other buffers are read
+    if (v0 + kGeK < vp) {
+      load_b(v0 + kGeK, buf ^ 1);
+      gen(v0 + kGeK, buf ^ 1);
+    }
+#pragma unroll
+    for (int k0 = 0; k0 < kGeK; k0 += 4) {
+      const double* A = As + (buf * kGeK + k0 + kq) * kGeLa + wm + q;
+      const double* B = Bs + (buf * kGeK + k0 + kq) * LB + wn + q;
+      double af[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) af[i] = A[8 * i];
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        const double bf = B[8 * j];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) dmma_gcv(acc[i][j], af[i], bf);
+      }
+    }
+  }
+  __syncthreads();
+  double* su = gsm;  // nc x kGeLa each
+  double* sx = su + nc * kGeLa;
+  double* sy = sx + nc * kGeLa;
+  for (int e = tid; e < kGrRows * nc; e += 256) {
+    const int r = e / nc, c = e - r * nc;
+    const bool live = live_row(r);
+    const int64_t at = (row0 + r) * nc + c;
+    su[c * kGeLa + r] = live ? a.bn[at] : 0.0;
+    sx[c * kGeLa + r] = live ? a.bnx[at] : 0.0;
+    sy[c * kGeLa + r] = live ? a.bny[at] : 0.0;
+  }
+  __syncthreads();
+  double g[3] = {0.0, 0.0, 0.0};
+  double rx[4] = {}, ry[4] = {}, rs[4] = {};
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int s = s0 + wn + 8 * j + 2 * kq + e;
+      if (s >= ge_pairs(nf)) continue;
+      const int2 cc = pair_of(s, nf);
+      if (cc.x >= nc) continue;  // the background with itself: no kernel component
+      const double* p0 = su + cc.x * kGeLa + wm + q;
+      const int step = nc * kGeLa;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const double v = acc[i][j][e];
+        const double u0 = p0[8 * i], x0 = p0[step + 8 * i], y0 = p0[2 * step + 8 * i];
+        if (cc.y == nc) {  // u_c' = 1, no component
+          rx[i] = fma(v, x0, rx[i]);
+          ry[i] = fma(v, y0, ry[i]);
+          rs[i] = fma(v, u0, rs[i]);
+        } else if (cc.x == cc.y) {
+          rx[i] = fma(v, x0 * u0, rx[i]);
+          ry[i] = fma(v, y0 * u0, ry[i]);
+          rs[i] = fma(v, u0 * u0, rs[i]);
+        } else {
+          const double* p1 = su + cc.y * kGeLa + wm + q;
+          const double u1 = p1[8 * i], x1 = p1[step + 8 * i], y1 = p1[2 * step + 8 * i];
+          rx[i] = fma(v, fma(x0, u1, x1 * u0), rx[i]);
+          ry[i] = fma(v, fma(y0, u1, y1 * u0), ry[i]);
+          rs[i] = fma(v, 2.0 * u0 * u1, rs[i]);
+        }
+      }
+    }
+  const GcvScalars S = *a.scal;
+  const double inv_s = 1.0 / a.scale;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = wm + 8 * i + q;
+    const double coef = live_row(r) ? 2.0 * a.w[row0 + r] * S.beta * S.lam : 0.0;
+    g[0] = fma(-coef, rx[i], g[0]);
+    g[1] = fma(-coef, ry[i], g[1]);
+    g[2] = fma(coef * inv_s, rs[i], g[2]);
+  }
+  __shared__ double red[3][8];
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    double v = g[i];
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (lane == 0) red[i][warp] = v;
+  }
+  __syncthreads();
+  if (tid < 3) {
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) t += red[tid][w];
+    part[(static_cast<size_t>(blockIdx.y) * gridDim.x + blockIdx.x) * 3 + tid] = t;
+  }
+}
+
+// out6 = the column sums of the row partials, plus the edf partials in the
+// first three (fixed order: lanes stride the rows, then a shuffle tree).
+__global__ void __launch_bounds__(192) k_gcv_sum(const double* __restrict__ part, int nrows,
+                                                 const double* __restrict__ edf, int nedf, double* __restrict__ out6) {
+  const int i = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  double t = 0.0;
+  for (int r = lane; r < nrows; r += 32) t += part[static_cast<size_t>(r) * 6 + i];
+  if (i < 3)
+    for (int r = lane; r < nedf; r += 32) t += edf[static_cast<size_t>(r) * 3 + i];
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) out6[i] = t;
 }
 
 // Fixed-order column sums (one thread per column, rows in order).
@@ -290,19 +512,49 @@ size_t gcv_stats_doubles(int P, int k, int r) {
   return 2 * static_cast<size_t>(P) + 4 * static_cast<size_t>(nq) + 8;
 }
 
+namespace {
 int gcv_rows_blocks(int64_t N) { return static_cast<int>((N + kGrRows - 1) / kGrRows); }
+// Pairs of components per CTA: the width with the least padding, the wider one on a tie.
+int ge_nt(int nf) { return ge_pad(ge_pairs(nf), 96) <= ge_pad(ge_pairs(nf), 48) ? 6 : 3; }
+}  // namespace
 
-void launch_gcv_rows(cudaStream_t st, const GcvRowsArgs& a, double* out6) {
+size_t gcv_rows_doubles(int64_t N, int nc, int k) {
+  const int nf = nc + 1, bn = 16 * ge_nt(nf);
+  const size_t P = static_cast<size_t>(nf) * k, sp = ge_pad(ge_pairs(nf), bn), vp = ge_pad(ge_pairs(k), kGeK);
+  return P * P + sp * vp + (6 + 3 * sp / bn) * static_cast<size_t>(gcv_rows_blocks(N)) + 2;
+}
+
+void launch_gcv_rows(cudaStream_t st, const GcvRowsArgs& a, double* work, double* out6) {
   if (a.k > kGrMaxK) fail(DGPU_ERR_INVALID, "stamp_gcv: at most 32 knots are supported");
-  const int P = (a.nc + 1) * a.k;
-  const size_t smem = sizeof(double) * (static_cast<size_t>(P) * kGrQc + 3 * static_cast<size_t>(a.nc) * kGrRows);
-  if (smem > 200 * 1024) fail(DGPU_ERR_INVALID, "stamp_gcv: basis too large for the row contraction");
+  const int nf = a.nc + 1, P = nf * a.k;
+  if (sizeof(double) * (8 * static_cast<size_t>(P) + 3 * static_cast<size_t>(a.nc) * kGrRows) > 200 * 1024)
+    fail(DGPU_ERR_INVALID, "stamp_gcv: basis too large for the row contraction");
+  const int nt = ge_nt(nf), bn = 16 * nt, nb = gcv_rows_blocks(a.N);
+  const int sp = ge_pad(ge_pairs(nf), bn), vp = ge_pad(ge_pairs(a.k), kGeK);
+  double* kp = work;  // 16-byte rows for cp.async: first, sp is a multiple of 48
+  double* K = kp + static_cast<size_t>(sp) * vp;
+  double* edf = K + static_cast<size_t>(P) * P;
+  GcvRowsArgs r = a;
+  r.partial = edf + 3 * static_cast<size_t>(sp / bn) * nb;
+  k_hht<<<dim3((P + 31) / 32, (P + 31) / 32), 128, 0, st>>>(P, a.nq + 1, a.X, K);
+  DGPU_LAUNCH("k_hht");
+  k_pack_k<<<vp, 128, 0, st>>>(nf, a.k, sp, K, kp);
+  DGPU_LAUNCH("k_pack_k");
+  const size_t smem = sizeof(double) * 2 * static_cast<size_t>(P);
   ensure_dynamic_smem(reinterpret_cast<const void*>(k_gcv_rows), smem);
-  const int nb = gcv_rows_blocks(a.N);
-  k_gcv_rows<<<nb, kGrRows, smem, st>>>(a);
+  k_gcv_rows<<<nb, kGrRows, smem, st>>>(r);
   DGPU_LAUNCH("k_gcv_rows");
-  k_colsum<<<1, 32, 0, st>>>(a.partial, nb, 6, out6);
-  DGPU_LAUNCH("k_colsum");
+  auto go = [&](auto kern, size_t bytes) {
+    ensure_dynamic_smem(reinterpret_cast<const void*>(kern), bytes);
+    kern<<<dim3(nb, sp / bn), 256, bytes, st>>>(a, kp, sp, vp, edf);
+  };
+  if (nt == 6)
+    go(k_gcv_edf<6>, ge_smem<6>(a.nc, a.k));
+  else
+    go(k_gcv_edf<3>, ge_smem<3>(a.nc, a.k));
+  DGPU_LAUNCH("k_gcv_edf");
+  k_gcv_sum<<<1, 192, 0, st>>>(r.partial, nb, edf, (sp / bn) * nb, out6);
+  DGPU_LAUNCH("k_gcv_sum");
 }
 
 }  // namespace dgpu
