@@ -48,3 +48,23 @@ def test_fp64_normal_equations_at_tile_edges(nc, side, n):
     tol = 10 * np.sqrt(n) * np.finfo(float).eps * cond
     assert np.linalg.norm(got - want) <= tol * np.linalg.norm(want)
 
+
+
+# Unknowns below, at and past the 32-column panels of the LDL^T, up to 23
+# panels. One component is zero at every row, so the Cholesky fails and the
+# system goes through the fallback; its zero pivots are the diagonal's ties.
+# The other unknowns are well determined (the bound of the fallback's own test).
+@pytest.mark.parametrize("nc,side,n", [(3, 3, 900), (6, 3, 1500), (7, 4, 2500), (12, 5, 4000), (28, 5, 6000)])
+def test_ldlt_fallback_at_panel_edges(nc, side, n):
+    rng = np.random.default_rng(nc)
+    knots = nr.grid_knots(0, 0, 100, 80, side, side)
+    pts = np.column_stack([rng.uniform(0, 100, n), rng.uniform(0, 80, n)])
+    bn = rng.normal(size=(n, nc))
+    bn[:, 2] = 0.0
+    w = rng.uniform(0.5, 2.0, n)
+    t = bn.sum(1) + 0.5 + 0.1 * rng.normal(size=n)
+    got = _core.solve_gls(knots, pts, t, w, bn, 0.1)
+    want = nr.solve_gls(knots, pts, t, w, bn, 0.1)
+    assert got["used_ldlt"]
+    np.testing.assert_allclose(got["theta"], want["theta"], rtol=1e-7, atol=1e-9)
+    np.testing.assert_allclose(got["effective_dof"], want["effective_dof"], rtol=1e-8)
