@@ -99,9 +99,7 @@ int dgpu_kernel_chi2(dgpu_context* ctx, int mem, int64_t width, int64_t height, 
 
     const bool want_theta = grad_theta != nullptr;
     const bool want_ref = grad_reference != nullptr;
-    const int nb = chi2_tile_blocks(w, h);
-    double* part = static_cast<double*>(c.slot(kSlotGrad3, sizeof(double) * (4 * static_cast<size_t>(nb) + 4)));
-    double* sums = part + 4 * static_cast<size_t>(nb);
+    const bool grad = want_theta || want_ref || grad_shift != nullptr || grad_scale != nullptr;
     Chi2Args a;
     a.w = w;
     a.h = h;
@@ -121,11 +119,14 @@ int dgpu_kernel_chi2(dgpu_context* ctx, int mem, int64_t width, int64_t height, 
     a.dgy = d_taps + 3 * nt;
     a.scale = static_cast<float>(scale);
     a.q = want_theta ? static_cast<float*>(c.slot(kSlotGrad4, sizeof(float) * n * nf)) : nullptr;
-    a.p = want_ref ? static_cast<float*>(c.slot(kSlotGrad5, sizeof(float) * n)) : nullptr;
+    a.p = want_theta || want_ref ? static_cast<float*>(c.slot(kSlotGrad5, sizeof(float) * n)) : nullptr;
+    const int nb = chi2_tile_blocks(a, grad);
+    double* part = static_cast<double*>(c.slot(kSlotGrad3, sizeof(double) * (4 * static_cast<size_t>(nb) + 4)));
+    double* sums = part + 4 * static_cast<size_t>(nb);
     a.partial = part;
     {
       StageTimer t(c, "gradient: chi2 tiles");
-      launch_chi2_tile(s, a);
+      launch_chi2_tile(s, a, grad);
       launch_sum_rows(s, part, nb, 4, sums);
     }
     std::vector<double> gth;
@@ -137,7 +138,7 @@ int dgpu_kernel_chi2(dgpu_context* ctx, int mem, int64_t width, int64_t height, 
       const size_t pairs = static_cast<size_t>(nf) * tp.k;
       double* tpart = static_cast<double*>(c.slot(kSlotGrad6, sizeof(double) * (pairs * tb + pairs)));
       d_gth = tpart + pairs * tb;
-      launch_theta_grad(s, w, h, nf, tp.k, a.q, D, tpart);
+      launch_theta_grad(s, w, h, nf, tp.k, a.q, a.p, D, tpart);
       launch_sum_rows(s, tpart, tb, static_cast<int>(pairs), d_gth);
       gth.resize(pairs);
     }
@@ -156,7 +157,7 @@ int dgpu_kernel_chi2(dgpu_context* ctx, int mem, int64_t width, int64_t height, 
       r.gx = a.gx;
       r.gy = a.gy;
       r.out = static_cast<float*>(out_buf(c, mem, grad_reference, 4 * n, kSlotGrad7));
-      launch_adjoint_reference(s, r);
+      launch_adjoint_reference(s, r, b.n_max);
       stage_out(c, mem, grad_reference, r.out, 4 * n);
     }
     double hs[4];

@@ -25,8 +25,8 @@ struct Chi2Args {
   const float* gy = nullptr;   // g_n(v - dy)
   const float* dgy = nullptr;  // g_n'(v - dy)
   float scale = 1.0f;
-  float* q = nullptr;          // optional: nf x (w*h), dchi2 / da_c(x)
-  float* p = nullptr;          // optional: w*h, rbar * s (for the reference adjoint)
+  float* q = nullptr;          // optional: nf x (w*h), C_c(x) and, last, rbar(x)
+  float* p = nullptr;          // optional: w*h, rbar * s; dchi2 / da_c(x) = p C_c for c < nc, rbar for the background
   double* partial = nullptr;   // chi2_tile_blocks x 4: chi2, d/ds, d/ddx, d/ddy
 };
 
@@ -44,12 +44,16 @@ struct AdjRefArgs {
 };
 
 size_t chi2_tile_smem(int n_max, int ks);
-int chi2_tile_blocks(int w, int h);
-void launch_chi2_tile(cudaStream_t st, const Chi2Args& a);
+// grad false: only chi^2 is wanted (the other sums may be left at zero).
+int chi2_tile_blocks(const Chi2Args& a, bool grad);
+void launch_chi2_tile(cudaStream_t st, const Chi2Args& a, bool grad);
+// The tiles of the common basis shapes (k_grad_tile.cu); false: not one of
+// them. Sets the number of tiles; launches only when a.partial is set.
+bool launch_chi2_fast(cudaStream_t st, const Chi2Args& a, bool grad, int* blocks);
 void launch_sum_rows(cudaStream_t st, const double* part, int nrows, int ncols, double* out);
 int theta_grad_blocks();
-void launch_theta_grad(cudaStream_t st, int w, int h, int nf, int k, const float* q, const DevFields& D,
+void launch_theta_grad(cudaStream_t st, int w, int h, int nf, int k, const float* q, const float* p, const DevFields& D,
                        double* part);
-void launch_adjoint_reference(cudaStream_t st, const AdjRefArgs& a);
+void launch_adjoint_reference(cudaStream_t st, const AdjRefArgs& a, int n_max);
 
 }  // namespace dgpu

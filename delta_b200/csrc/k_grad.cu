@@ -19,7 +19,9 @@
 //   dchi2/ddx  -= rbar s sum_c a_c C^x_c     (dy alike)
 //   q_c(x)      = rbar s C_c (c < nc),  q_nc = rbar   (dchi2/da_c(x))
 // chi^2 and the scalar gradients are reduced per CTA in FP64 and summed in a
-// fixed order. q is written out (nf values per pixel) for the field adjoint.
+// fixed order. C_c (c < nc), rbar and p = rbar s are written out for the adjoints.
+// k_grad_tile.cu holds the same tiles for the common basis shapes; this kernel
+// serves the others (n_max 0, 1, 7, 8; fewer than 9 or more than 40 taps).
 //
 // k_theta_grad: dchi2/dtheta_{c,j} = sum_x q_c(x) D_j(x), where D_j(x) is the
 // same lattice blend applied to the j-th design function (the fields of the
@@ -161,8 +163,7 @@ __global__ void __launch_bounds__(kGThreads) k_chi2_tile(Chi2Args a) {
       g_dy -= static_cast<double>(rb) * static_cast<double>(s) * static_cast<double>(my);
     }
     if (a.q) {
-      const float f = rb * s;
-      for (int c = 0; c < a.nc; ++c) a.q[static_cast<size_t>(c) * N + idx] = f * cv[c];
+      for (int c = 0; c < a.nc; ++c) a.q[static_cast<size_t>(c) * N + idx] = cv[c];
       a.q[static_cast<size_t>(a.nc) * N + idx] = rb;
     }
     if (a.p) a.p[idx] = rb * s;
@@ -188,62 +189,131 @@ __global__ void __launch_bounds__(kGThreads) k_chi2_tile(Chi2Args a) {
   }
 }
 
-// out[c] = sum over rows r of part[r * ncols + c], rows in order (one thread per column).
-__global__ void k_sum_rows(const double* __restrict__ part, int nrows, int ncols, double* __restrict__ out) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
-  if (c >= ncols) return;
+// out[c] = sum over rows r of part[r * ncols + c], a CTA per column: threads
+// stride the rows, then a fixed tree. (One thread per column over the 8192 tiles
+// of a 2048^2 frame was a 0.4 ms chain of dependent loads.)
+__global__ void __launch_bounds__(256) k_sum_rows(const double* __restrict__ part, int nrows, int ncols,
+                                                  double* __restrict__ out) {
+  __shared__ double red[8];
   double t = 0.0;
-  for (int r = 0; r < nrows; ++r) t += part[static_cast<size_t>(r) * ncols + c];
-  out[c] = t;
+  for (int r = threadIdx.x; r < nrows; r += 256) t += part[static_cast<size_t>(r) * ncols + blockIdx.x];
+  t = warp_sum_d(t);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = t;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    t = 0.0;
+    for (int i = 0; i < 8; ++i) t += red[i];
+    out[blockIdx.x] = t;
+  }
 }
 
-constexpr int kTgChunk = 256;
-constexpr int kTgStride = kTgChunk + 1;  // padded rows: a warp reads 16+ rows at one column
-constexpr int kTgThreads = 512;
+// sum_x q_f(x) D_j(x) on the FP64 tensor cores: fields x design functions with
+// the pixels as the inner dimension, exact products of float32 values. A warp
+// takes 32 pixels at a time, lane = pixel: the planes of the next 32 arrive by
+// cp.async (coalesced, one plane per instruction) while it blends D, brings both
+// into the fragment layout through shared memory and multiplies; q_c = p C_c is
+// rounded to float32 as it is read. One tile of 32 fields x 8 NT design
+// functions per CTA (blockIdx.y, .z), its warps' sums added in order. Floor:
+// reading the planes (nf + 1 floats per pixel: 0.5 GB at 2048^2, 29 fields, 75 us
+// at 6.5 TB/s). One FP64 FMA chain per thread and pair took 1.53 ms, this 0.22 ms.
+constexpr int kTgWarps = 8;
+constexpr int kTgLd = 36;  // conflict-free fragments
 
-// Per block: sum over its pixel chunks of q_c(x) D_j(x) -> part[block][c * k + j].
-__global__ void __launch_bounds__(kTgThreads) k_theta_grad(int w, int h, int nf, int k, const float* __restrict__ q,
-                                                           DevFields D, double* __restrict__ part) {
+__device__ __forceinline__ void dmma_grad(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
+// One float to shared memory, 0 when !in (src is then not read).
+__device__ __forceinline__ void cp_async4(float* dst, const float* src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(dst))),
+               "l"(src), "r"(in ? 4 : 0)
+               : "memory");
+}
+
+template <int NT>
+__global__ void __launch_bounds__(kTgWarps * 32, 2)
+k_theta_grad(int w, int h, int nf, int k, const float* __restrict__ q, const float* __restrict__ p, DevFields D,
+             double* __restrict__ part) {
   extern __shared__ __align__(16) float sm[];
-  float* sq = sm;                    // nf x chunk (row stride kTgStride)
-  float* sd = sq + nf * kTgStride;   // k x chunk
-  const size_t N = static_cast<size_t>(w) * h;
-  const int pairs = nf * k;
-  double acc[(64 * 64 + kTgThreads - 1) / kTgThreads];
-  const int per = (pairs + kTgThreads - 1) / kTgThreads;
-  for (int i = 0; i < per; ++i) acc[i] = 0.0;
-  for (size_t base = static_cast<size_t>(blockIdx.x) * kTgChunk; base < N;
-       base += static_cast<size_t>(gridDim.x) * kTgChunk) {
-    const int n = static_cast<int>(min(static_cast<size_t>(kTgChunk), N - base));
-    __syncthreads();
-    for (int i = threadIdx.x; i < nf * kTgChunk; i += blockDim.x) {
-      const int c = i / kTgChunk, pp = i - c * kTgChunk;
-      sq[c * kTgStride + pp] = pp < n ? q[static_cast<size_t>(c) * N + base + pp] : 0.0f;
+  constexpr int NJ = 8 * NT, kBuf = 33 * kTgLd, kWarpFloats = 2 * kBuf + NJ * kTgLd;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, r = lane >> 2, kq = lane & 3;
+  float* sq = sm + warp * kWarpFloats;  // 2 x (32 planes, then p) x kTgLd
+  float* sd = sq + 2 * kBuf;            // NJ x kTgLd
+  const int f0 = blockIdx.z * 32, j0 = blockIdx.y * NJ, nfl = min(32, nf - f0), nj = min(NJ, k - j0);
+  const int nc = nf - 1 - f0;           // planes below nc are C_c (times p), plane nc is rbar
+  const int64_t N = static_cast<int64_t>(w) * h;
+  for (int i = lane; i < kWarpFloats; i += 32) sq[i] = 0.0f;  // planes past the last stay zero
+  __syncwarp();
+  auto load = [&](int64_t b, int buf) {
+    const int64_t px = min(b + lane, N - 1);
+    const bool in = b + lane < N;
+    float* dst = sq + buf * kBuf + lane;
+    const float* src = q + static_cast<size_t>(f0) * N + px;
+    for (int f = 0; f < nfl; ++f) cp_async4(dst + f * kTgLd, src + static_cast<size_t>(f) * N, in);
+    cp_async4(dst + 32 * kTgLd, p + px, in);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  double acc[4][NT][2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < NT; ++j) acc[i][j][0] = acc[i][j][1] = 0.0;
+  const int64_t step = static_cast<int64_t>(gridDim.x) * kTgWarps * 32;
+  int64_t b = (static_cast<int64_t>(blockIdx.x) * kTgWarps + warp) * 32;
+  if (b < N) load(b, 0);
+  for (int buf = 0; b < N; b += step, buf ^= 1) {
+    if (b + step < N) load(b + step, buf ^ 1);
+    const int64_t px = min(b + lane, N - 1);
+    const int y = static_cast<int>(px / w), x = static_cast<int>(px - static_cast<int64_t>(y) * w);
+    if (D.exact) {
+      for (int j = 0; j < nj; ++j) sd[j * kTgLd + lane] = __ldg(D.full + static_cast<size_t>(j0 + j) * N + px);
+    } else {
+      const size_t plane = static_cast<size_t>(D.ncx) * D.ncy;
+      const float* c0 = D.latf + j0 * plane + static_cast<size_t>(D.celly[y]) * D.ncx + D.cellx[x];
+      const float fy = D.wy[y], wx = D.wx[x];
+#pragma unroll 8
+      for (int j = 0; j < nj; ++j, c0 += plane)
+        sd[j * kTgLd + lane] = cell_blend(__ldg(c0), __ldg(c0 + 1), __ldg(c0 + D.ncx), __ldg(c0 + D.ncx + 1), fy, wx);
     }
-    for (int i = threadIdx.x; i < k * kTgChunk; i += blockDim.x) {
-      const int j = i / kTgChunk, pp = i - j * kTgChunk;
-      float v = 0.0f;
-      if (pp < n) {
-        const size_t idx = base + pp;
-        v = field_point(D, j, static_cast<int>(idx % w), static_cast<int>(idx / w));
+    if (b + step < N)
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    else
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+    const float* cur = sq + buf * kBuf;
+#pragma unroll
+    for (int k0 = 0; k0 < 32; k0 += 4) {
+      const float pv = cur[32 * kTgLd + k0 + kq];
+      double bf[NT];
+#pragma unroll
+      for (int j = 0; j < NT; ++j) bf[j] = static_cast<double>(sd[(8 * j + r) * kTgLd + k0 + kq]);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float v = cur[(8 * i + r) * kTgLd + k0 + kq];
+        const double af = static_cast<double>(8 * i + r < nc ? pv * v : v);
+#pragma unroll
+        for (int j = 0; j < NT; ++j) dmma_grad(acc[i][j], af, bf[j]);
       }
-      sd[j * kTgStride + pp] = v;
     }
-    __syncthreads();
-    for (int i = 0; i < per; ++i) {
-      const int t = threadIdx.x + i * kTgThreads;
-      if (t >= pairs) break;
-      const int c = t / k, j = t - c * k;
-      const float* a0 = sq + c * kTgStride;
-      const float* b0 = sd + j * kTgStride;
-      double s = 0.0;
-      for (int pp = 0; pp < n; ++pp) s = fma(static_cast<double>(a0[pp]), static_cast<double>(b0[pp]), s);
-      acc[i] += s;
-    }
+    __syncwarp();
   }
-  for (int i = 0; i < per; ++i) {
-    const int t = threadIdx.x + i * kTgThreads;
-    if (t < pairs) part[static_cast<size_t>(blockIdx.x) * pairs + t] = acc[i];
+  __syncthreads();
+  double* red = reinterpret_cast<double*>(sm);  // warps x 32 x NJ
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) red[(warp * 32 + 8 * i + r) * NJ + 8 * j + 2 * kq + e] = acc[i][j][e];
+  __syncthreads();
+  for (int e = threadIdx.x; e < 32 * NJ; e += kTgWarps * 32) {
+    const int f = e / NJ, j = e - f * NJ;
+    if (f0 + f >= nf || j0 + j >= k) continue;
+    double t = 0.0;
+    for (int i = 0; i < kTgWarps; ++i) t += red[i * 32 * NJ + e];
+    part[static_cast<size_t>(blockIdx.x) * nf * k + (f0 + f) * k + j0 + j] = t;
   }
 }
 
@@ -310,7 +380,185 @@ __global__ void __launch_bounds__(kGThreads) k_adjoint_reference(AdjRefArgs a) {
   }
 }
 
-void launch_chi2_tile(cudaStream_t st, const Chi2Args& a) {
+// The reference adjoint for up to 40 taps (KSP = 8 KB, zero padded): grouped by
+// nx, sum_ny first. Both correlations are linear, so
+//   dchi2/dR = sum_nx g_nx (*)_x [ sum_ny g_ny (*)_y (p a_{nx,ny}) ]
+// needs one x correlation per nx instead of one per component. A CTA of 256
+// threads takes 128 window columns (a pair per lane, packed FMAs) by 32 output
+// rows, 8 rows per thread; a_c p is blended into one window buffer while the
+// other is read, the y sums stay in registers over the group's components, and
+// the x correlation reads them from shared memory, one row per lane. FP32 FMA
+// bound: about 1200 FMA per pixel at 28 components of 23 taps (0.14 ms for
+// 2048^2 at 37.2 TFMA/s); one x and one y correlation per component with a
+// scalar load per tap took 2.70 ms, this 0.44 ms.
+constexpr int kArCols = 128;           // window columns of a tile
+constexpr int kArRows = 32;            // output rows of a tile
+constexpr int kArLdI = kArCols + 4;    // y sums: conflict-free 16-byte reads, a row per lane
+
+template <int KB>
+__global__ void __launch_bounds__(256, 2) k_adjoint_f(AdjRefArgs a, int n_max) {
+  constexpr int KSP = 8 * KB, TW = kArCols - KSP, WR = kArRows + KSP;  // output columns, window rows
+  extern __shared__ __align__(16) float smem[];
+  float* pw = smem;                    // WR x kArCols: p
+  float* pc = pw + WR * kArCols;       // 2 x WR x kArCols: p a_c
+  float* ys = pc + 2 * WR * kArCols;   // kArRows x kArLdI: sum_ny g_ny (*)_y (p a_c)
+  float* gx = ys + kArRows * kArLdI;   // (n_max + 1) x KSP
+  float* gy = gx + (n_max + 1) * KSP;
+  const int ks = a.ks, kh = (ks - 1) / 2, w = a.w, h = a.h, tid = threadIdx.x;
+  const DevFields& F = a.F;
+  const int bx = blockIdx.x * TW, by = blockIdx.y * kArRows;
+  for (int i = tid; i < (n_max + 1) * KSP; i += 256) {
+    const int q = i / KSP, j = i - q * KSP;
+    gx[i] = j < ks ? a.gx[q * ks + j] : 0.0f;
+    gy[i] = j < ks ? a.gy[q * ks + j] : 0.0f;
+  }
+  for (int i = tid; i < WR * kArCols; i += 256) {
+    const int r = i / kArCols, c = i - r * kArCols;
+    const int yy = by - kh + r, xx = bx - kh + c;
+    pw[i] = (yy >= 0 && yy < h && xx >= 0 && xx < w) ? a.p[static_cast<size_t>(yy) * w + xx] : 0.0f;
+  }
+  // This thread's window columns (a pair) and rows: WR / 4 in the blend, 8 in the y correlation.
+  const int cp = 2 * (tid & 63), rg = tid >> 6;
+  int xc[2], jx[2];
+  float wx[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    xc[u] = min(max(bx - kh + cp + u, 0), w - 1);
+    jx[u] = F.exact ? 0 : F.cellx[xc[u]];
+    wx[u] = F.exact ? 0.0f : F.wx[xc[u]];
+  }
+  auto blend = [&](int c, float* dst) {
+    int cj = -1;
+    float a00[2], e[2], t[2], g[2];
+    for (int r = rg * (WR / 4); r < (rg + 1) * (WR / 4); ++r) {
+      const int yy = min(max(by - kh + r, 0), h - 1);
+      const float2 pv = *reinterpret_cast<const float2*>(pw + r * kArCols + cp);
+      float f[2];
+      if (F.exact) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u) f[u] = __ldg(F.full + (static_cast<size_t>(c) * h + yy) * w + xc[u]);
+      } else {
+        const int jy = F.celly[yy];
+        const float fy = F.wy[yy];
+        if (jy != cj) {
+          cj = jy;
+          const float* r0 = F.latf + (static_cast<size_t>(c) * F.ncy + cj) * F.ncx;
+          const float* r1 = r0 + F.ncx;
+#pragma unroll
+          for (int u = 0; u < 2; ++u) {
+            const float b00 = __ldg(r0 + jx[u]), b01 = __ldg(r0 + jx[u] + 1);
+            const float b10 = __ldg(r1 + jx[u]), b11 = __ldg(r1 + jx[u] + 1);
+            a00[u] = b00;
+            e[u] = b10 - b00;
+            t[u] = b01 - b00;
+            g[u] = (b11 - b10) - t[u];
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+          f[u] = __fmaf_rn(__fmaf_rn(g[u], fy, t[u]), wx[u], __fmaf_rn(e[u], fy, a00[u]));
+      }
+      *reinterpret_cast<float2*>(dst + r * kArCols + cp) = make_float2(pv.x * f[0], pv.y * f[1]);
+    }
+  };
+  // x correlation items: lane = row, 8 output columns per warp and step.
+  constexpr int kGroups = TW / 8, kItems = (kGroups + 7) / 8;
+  const int lane = tid & 31, warp = tid >> 5;
+  float out[kItems][8];
+#pragma unroll
+  for (int n = 0; n < kItems; ++n)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) out[n][i] = 0.0f;
+  auto comp = [](int nx, int ny) { return (nx + ny) * (nx + ny + 1) / 2 + ny; };
+  __syncthreads();
+  blend(comp(0, 0), pc);
+  int buf = 0;
+  for (int nx = 0; nx <= n_max; ++nx) {
+    float2 acc[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] = make_float2(0.0f, 0.0f);
+    for (int ny = 0; ny <= n_max - nx; ++ny) {
+      __syncthreads();  // this component's window is complete, the other buffer is read
+      const float* cur = pc + buf * WR * kArCols;
+      buf ^= 1;
+      if (ny < n_max - nx)
+        blend(comp(nx, ny + 1), pc + buf * WR * kArCols);
+      else if (nx < n_max)
+        blend(comp(nx + 1, 0), pc + buf * WR * kArCols);
+      const float* col = cur + rg * 8 * kArCols + cp;
+      const float* g = gy + ny * KSP;
+#pragma unroll
+      for (int j0 = 0; j0 < KSP; j0 += 8) {
+        float2 v[15];
+#pragma unroll
+        for (int t = 0; t < 15; ++t) v[t] = *reinterpret_cast<const float2*>(col + (j0 + t) * kArCols);
+        const float4 ka = *reinterpret_cast<const float4*>(g + j0), kb = *reinterpret_cast<const float4*>(g + j0 + 4);
+        const float kv[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
+#pragma unroll
+        for (int jj = 0; jj < 8; ++jj)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) acc[i] = __ffma2_rn(make_float2(kv[jj], kv[jj]), v[i + jj], acc[i]);
+      }
+    }
+    // (the x pass of the previous nx finished reading ys before this nx's first barrier)
+#pragma unroll
+    for (int i = 0; i < 8; ++i) *reinterpret_cast<float2*>(ys + (rg * 8 + i) * kArLdI + cp) = acc[i];
+    __syncthreads();
+#pragma unroll
+    for (int n = 0; n < kItems; ++n) {
+      const int grp = warp + 8 * n;
+      if (grp >= kGroups) break;
+      const float* row = ys + lane * kArLdI + 8 * grp;
+#pragma unroll
+      for (int j0 = 0; j0 < KSP; j0 += 8) {
+        float v[16];
+#pragma unroll
+        for (int t = 0; t < 16; t += 4) {
+          const float4 q = *reinterpret_cast<const float4*>(row + j0 + t);
+          v[t] = q.x, v[t + 1] = q.y, v[t + 2] = q.z, v[t + 3] = q.w;
+        }
+        const float4 ka = *reinterpret_cast<const float4*>(gx + nx * KSP + j0);
+        const float4 kb = *reinterpret_cast<const float4*>(gx + nx * KSP + j0 + 4);
+        const float kv[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
+#pragma unroll
+        for (int jj = 0; jj < 8; ++jj)
+#pragma unroll
+          for (int i = 0; i < 8; ++i) out[n][i] = __fmaf_rn(kv[jj], v[i + jj], out[n][i]);
+      }
+    }
+  }
+  const int y = by + lane;
+  if (y >= h) return;
+#pragma unroll
+  for (int n = 0; n < kItems; ++n) {
+    const int grp = warp + 8 * n;
+    if (grp >= kGroups) break;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int x = bx + 8 * grp + i;
+      if (x >= w) break;
+      const size_t idx = static_cast<size_t>(y) * w + x;
+      const float rv = __ldg(a.ref + idx);
+      const bool replaced = (a.rmask && __ldg(a.rmask + idx) != 0) || !isfinite(rv);
+      a.out[idx] = replaced ? 0.0f : out[n][i];
+    }
+  }
+}
+
+template <int KB>
+static void launch_adjoint_f(cudaStream_t st, const AdjRefArgs& a, int n_max) {
+  constexpr int KSP = 8 * KB;
+  const size_t smem = sizeof(float) * (3 * static_cast<size_t>(kArRows + KSP) * kArCols + kArRows * kArLdI +
+                                       2 * static_cast<size_t>(n_max + 1) * KSP);
+  auto kern = k_adjoint_f<KB>;
+  ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
+  kern<<<dim3(ceil_div(a.w, kArCols - KSP), ceil_div(a.h, kArRows)), 256, smem, st>>>(a, n_max);
+  DGPU_LAUNCH("k_adjoint_f");
+}
+
+void launch_chi2_tile(cudaStream_t st, const Chi2Args& a, bool grad) {
+  int blocks;
+  if (launch_chi2_fast(st, a, grad, &blocks)) return;
   const dim3 grid(ceil_div(a.w, kGTW), ceil_div(a.h, kGTH));
   const size_t smem = chi2_tile_smem(a.n_max, a.ks);
   ensure_dynamic_smem(reinterpret_cast<const void*>(k_chi2_tile), smem);
@@ -318,25 +566,45 @@ void launch_chi2_tile(cudaStream_t st, const Chi2Args& a) {
   DGPU_LAUNCH("k_chi2_tile");
 }
 
-int chi2_tile_blocks(int w, int h) { return ceil_div(w, kGTW) * ceil_div(h, kGTH); }
+int chi2_tile_blocks(const Chi2Args& a, bool grad) {
+  Chi2Args q = a;
+  q.partial = nullptr;
+  int blocks;
+  return launch_chi2_fast(nullptr, q, grad, &blocks) ? blocks : ceil_div(a.w, kGTW) * ceil_div(a.h, kGTH);
+}
 
 void launch_sum_rows(cudaStream_t st, const double* part, int nrows, int ncols, double* out) {
-  k_sum_rows<<<ceil_div(ncols, 128), 128, 0, st>>>(part, nrows, ncols, out);
+  k_sum_rows<<<ncols, 256, 0, st>>>(part, nrows, ncols, out);
   DGPU_LAUNCH("k_sum_rows");
 }
 
 int theta_grad_blocks() { return 148 * 2; }
 
-void launch_theta_grad(cudaStream_t st, int w, int h, int nf, int k, const float* q, const DevFields& D,
+void launch_theta_grad(cudaStream_t st, int w, int h, int nf, int k, const float* q, const float* p, const DevFields& D,
                        double* part) {
   if (nf * k > 64 * 64) fail(DGPU_ERR_INVALID, "gradient: too many field coefficients");
-  const size_t smem = sizeof(float) * static_cast<size_t>(nf + k) * kTgStride;
-  ensure_dynamic_smem(reinterpret_cast<const void*>(k_theta_grad), smem);
-  k_theta_grad<<<theta_grad_blocks(), kTgThreads, smem, st>>>(w, h, nf, k, q, D, part);
+  auto go = [&](auto kern, int nt) {
+    const size_t smem = std::max(sizeof(float) * kTgWarps * (66 + 8 * nt) * kTgLd, sizeof(double) * kTgWarps * 32 * 8 * nt);
+    ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
+    kern<<<dim3(theta_grad_blocks(), ceil_div(k, 8 * nt), ceil_div(nf, 32)), kTgWarps * 32, smem, st>>>(w, h, nf, k, q, p,
+                                                                                                  D, part);
+  };
+  if (k <= 16)
+    go(k_theta_grad<2>, 2);
+  else
+    go(k_theta_grad<4>, 4);
   DGPU_LAUNCH("k_theta_grad");
 }
 
-void launch_adjoint_reference(cudaStream_t st, const AdjRefArgs& a) {
+void launch_adjoint_reference(cudaStream_t st, const AdjRefArgs& a, int n_max) {
+  switch ((a.ks + 7) / 8) {
+    case 1: return launch_adjoint_f<1>(st, a, n_max);
+    case 2: return launch_adjoint_f<2>(st, a, n_max);
+    case 3: return launch_adjoint_f<3>(st, a, n_max);
+    case 4: return launch_adjoint_f<4>(st, a, n_max);
+    case 5: return launch_adjoint_f<5>(st, a, n_max);
+    default: break;  // longer taps: the generic kernel
+  }
   const dim3 grid(ceil_div(a.w, kGTW), ceil_div(a.h, kGTH));
   const size_t smem = adjoint_ref_smem(a.ks);
   ensure_dynamic_smem(reinterpret_cast<const void*>(k_adjoint_reference), smem);
