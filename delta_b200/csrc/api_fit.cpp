@@ -132,9 +132,10 @@ struct Engine {
     int *ok, *midx, *ridx;
     double* partial;
   };
-  Work work(int nsys, int nm = 1) {
+  Work work(int nsys, int nm = 1, bool want_edf = true) {
     Work w{};
-    w.A = static_cast<double*>(c.slot(kSlotFft0, sizeof(double) * solve_work_doubles(P, nf, rk, nsys, nm)));
+    w.A = static_cast<double*>(
+        c.slot(kSlotFft0, sizeof(double) * solve_work_doubles(P, nf, want_edf ? rk : 0, nsys, nm)));
     const size_t small = sizeof(double) * (static_cast<size_t>(nsys) * P + 6 * nsys) + sizeof(int) * 3 * nsys + 64;
     char* sm = static_cast<char*>(c.slot(kSlotFft1, small));
     w.theta = reinterpret_cast<double*>(sm);
@@ -151,12 +152,13 @@ struct Engine {
   }
 
   void solve(const Work& w, int nsys, const double* M, const int* midx, const double* rhs, const int* ridx,
-             int nm = 1) {
+             int nm = 1, bool want_edf = true) {
     SolveBatch b;
     b.P = P;
     b.k = k;
     b.nf = nf;
-    b.r = rk;
+    b.r = want_edf ? rk : 0;
+    b.want_edf = want_edf ? 1 : 0;
     b.nsys = nsys;
     b.M = M;
     b.m_index = midx;
@@ -427,18 +429,20 @@ struct Engine {
       launch_stamp_moments(c.stream, n_units, nc, SS, R, mask, As, rs, ds2, cen);
       const auto hc = down(c, cen, static_cast<size_t>(n_units) * 3);
       std::vector<double> dsd(static_cast<size_t>(n_units) * k, 0.0);
-      std::vector<int> f2(n_units, -1);
-      for (int u = 0; u < n_units; ++u) {
-        const double cnt = hc[3 * u + 2];
-        if (cnt <= 0.0 || fold[u] < 0) continue;
-        tp.design_row(hc[3 * u] / cnt, hc[3 * u + 1] / cnt, dsd.data() + static_cast<size_t>(u) * k);
-        f2[u] = fold[u];
+      std::vector<int> members(G + 1, 0);  // offsets of the folds, then their stamps in order
+      for (int g = 0; g < G; ++g) {
+        for (int u = 0; u < n_units; ++u) {
+          const double cnt = hc[3 * u + 2];
+          if (cnt <= 0.0 || fold[u] != g) continue;
+          tp.design_row(hc[3 * u] / cnt, hc[3 * u + 1] / cnt, dsd.data() + static_cast<size_t>(u) * k);
+          members.push_back(u);
+        }
+        members[g + 1] = static_cast<int>(members.size()) - (G + 1);
       }
       double* d_dsd = up(c, kSlotFit13, dsd.data(), dsd.size());
-      int* d_fold = static_cast<int*>(c.slot(kSlotBlockCounts, sizeof(int) * std::max(n_units, 1)));
-      DGPU_CUDA(h2d_async(d_fold, f2.data(), sizeof(int) * n_units, c.stream));
-      launch_stamped_assemble(c.stream, G, n_units, nf, k, d_fold, As, rs, ds2, d_dsd, Mg, rg, yg);
-      DGPU_CUDA(cudaStreamSynchronize(c.stream));
+      int* d_members = static_cast<int*>(c.slot(kSlotBlockCounts, sizeof(int) * members.size()));
+      DGPU_CUDA(h2d_async(d_members, members.data(), sizeof(int) * members.size(), c.stream));
+      launch_stamped_assemble(c.stream, G, nf, k, d_members + G + 1, d_members, As, rs, ds2, d_dsd, Mg, rg, yg);
     } else {
       uint8_t* fm = static_cast<uint8_t*>(c.slot(kSlotSeedNeg, std::max<size_t>(static_cast<size_t>(G) * n_units, 1)));
       const auto hm = down(c, mask, n_units);
@@ -465,7 +469,7 @@ struct Engine {
     }
     std::vector<double> curve(nl, kInf);
     std::vector<char> done(nl, 0);
-    Work w = work(std::max(nl * G, 1), G);
+    Work w = work(std::max(nl * G, 1), G, false);  // held-out errors need theta alone
     // Mixed precision, row folds: held-out errors around per-fold anchors
     // (th0[g], with the FP64 residual sums r0[g], s0[g] over fold g's rows).
     double* th0 = nullptr;
@@ -484,7 +488,7 @@ struct Engine {
         }
       DGPU_CUDA(h2d_async(w.lam, lam.data(), sizeof(double) * ns, c.stream));
       DGPU_CUDA(h2d_async(w.midx, mi.data(), sizeof(int) * ns, c.stream));
-      solve(w, ns, Mt, w.midx, rt, w.midx, G);
+      solve(w, ns, Mt, w.midx, rt, w.midx, G, false);
       return ns;
     };
     auto evaluate = [&](const std::vector<int>& idx) {

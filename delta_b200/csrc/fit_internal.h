@@ -77,6 +77,9 @@ struct SolveBatch {
   int* ok = nullptr;                // nsys: 1 Cholesky, 2 LDLT fallback, 0 failed
   unsigned* status = nullptr;
   double* partial = nullptr;        // nsys x 8 per-rank trace partials
+  // 0: no degrees of freedom wanted (edf stays unset): the rows F^T are not
+  // appended, which halves the work. r is then 0 for the workspace too.
+  int want_edf = 1;
   // 1: leave systems whose Cholesky failed at ok = 0 (no LDLT fallback): a
   // reduced-precision attempt that will be redone in FP64 anyway.
   int skip_ldlt = 0;

@@ -18,7 +18,7 @@ void launch_gcv_finish(cudaStream_t st, int nsys, const double* raw, const doubl
 void launch_fold_train(cudaStream_t st, int groups, size_t len, const double* part, double* all, double* train);
 void launch_stamp_moments(cudaStream_t st, int n_stamps, int nc, int SS, const FitRows& R, const uint8_t* accepted,
                           double* As, double* rs, double* ds2, double* cen);
-void launch_stamped_assemble(cudaStream_t st, int groups, int nstamp, int nf, int k, const int* fold,
+void launch_stamped_assemble(cudaStream_t st, int groups, int nf, int k, const int* list, const int* offs,
                              const double* As, const double* rs, const double* ds2, const double* dsd, double* Mg,
                              double* rg, double* yg);
 void launch_refine_update(cudaStream_t st, int P, int k, const double* pen, double lam, const double* theta,

@@ -167,107 +167,224 @@ void launch_fold_train(cudaStream_t st, int groups, size_t len, const double* pa
 }
 
 // Per-stamp moments over the stamp's active rows: A_s = sum w b b^T (nf x nf,
-// full), r_s = sum w t b, ds2_s = sum w t^2, pixel-centroid sums.
-__global__ void __launch_bounds__(256)
+// full), r_s = sum w t b, ds2_s = sum w t^2, pixel-centroid sums. A CTA per stamp:
+// with t appended to the row, [b, t], all three are one product (w [b, t])^T
+// [b, t] with the rows as the inner dimension, on the FP64 tensor cores, each
+// entry the FMA chain over the rows in order. Rows arrive by cp.async, kSmRows at a
+// time. Bound by reading the rows (230 bytes each; 200 stamps of 961 rows, 29
+// fields: 44 MB, 7 us at 6.5 TB/s) and one chain of DMMAs per entry; a thread per entry walking the rows took
+// 2.1 ms, this 0.09 ms.
+constexpr int kSmRows = 64;
+constexpr int kSmThreads = 512;
+
+__host__ __device__ inline int sm_ld(int nf) { return ((nf + 1 + 7) / 8 * 8 + 11) / 16 * 16 + 4; }  // >= nf + 1 rounded to 8, = 4 mod 16
+size_t stamp_moments_smem(int nf) { return sizeof(double) * kSmRows * (3 * static_cast<size_t>(sm_ld(nf)) + 2); }
+
+__device__ __forceinline__ void dmma_gls(double (&d)[2], double a, double b) {
+  asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+      : "+d"(d[0]), "+d"(d[1])
+      : "d"(a), "d"(b));
+}
+
+__global__ void __launch_bounds__(kSmThreads)
 k_stamp_moments(int nc, int SS, FitRows R, const uint8_t* __restrict__ accepted, double* __restrict__ As,
                 double* __restrict__ rs, double* __restrict__ ds2, double* __restrict__ cen) {
-  const int s = blockIdx.x, nf = nc + 1;
-  const bool act_stamp = accepted[s] != 0;
-  // entries: nf*nf (A) + nf (r) + 1 (ds2) + 3 (sx, sy, count); one thread per
-  // entry, rows summed in order.
-  const int ne = nf * nf + nf + 4;
-  for (int e = threadIdx.x; e < ne; e += blockDim.x) {
-    double acc = 0.0;
-    if (act_stamp) {
-      for (int i = 0; i < SS; ++i) {
-        const size_t row = static_cast<size_t>(s) * SS + i;
-        if (!R.valid[row]) continue;
-        const double w = R.w[row], t = R.t[row];
-        double v;
-        if (e < nf * nf) {
-          const int a = e / nf, b = e % nf;
-          const double ba = a < nc ? R.bn[row * nc + a] : 1.0;
-          const double bb = b < nc ? R.bn[row * nc + b] : 1.0;
-          v = w * ba * bb;
-        } else if (e < nf * nf + nf) {
-          const int a = e - nf * nf;
-          const double ba = a < nc ? R.bn[row * nc + a] : 1.0;
-          v = w * t * ba;
-        } else if (e == nf * nf + nf) {
-          v = w * t * t;
-        } else if (e == nf * nf + nf + 1) {
-          v = static_cast<double>(R.px[row]);
-        } else if (e == nf * nf + nf + 2) {
-          v = static_cast<double>(R.py[row]);
-        } else {
-          v = 1.0;
+  extern __shared__ __align__(16) double smm[];
+  const int s = blockIdx.x, nf = nc + 1, ld = sm_ld(nf), nt = (nf + 1 + 7) / 8;  // tiles of 8 per side
+  double* rows = smm;                          // 2 x kSmRows x ld: b (background 1), t, zeros
+  double* wrow = rows + 2 * kSmRows * ld;      // kSmRows x ld: w [b, t]
+  double* wv = wrow + kSmRows * ld;            // 2 x kSmRows: w
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, q = lane >> 2, kq = lane & 3;
+  constexpr int kWarps = kSmThreads / 32;
+  const size_t base = static_cast<size_t>(s) * SS;
+  const bool on = accepted[s] != 0;
+  const int n = on ? SS : 0;
+  auto active = [&](int i) { return i < n && R.valid[base + i]; };
+  // Inactive rows stay out of shared memory (zeros there) and out of every sum.
+  auto stage = [&](int i0, int buf) {
+    for (int rr = warp; rr < kSmRows; rr += kWarps) {
+      double* o = rows + (buf * kSmRows + rr) * ld;
+      const size_t row = base + i0 + rr;
+      if (active(i0 + rr)) {
+        for (int c = lane; c < nc; c += 32)
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(o + c))),
+                       "l"(R.bn + row * nc + c) : "memory");
+        if (lane == 0) {
+          o[nc] = 1.0;
+          o[nf] = R.t[row];
+          wv[buf * kSmRows + rr] = R.w[row];
         }
-        acc += v;
+      } else {
+        for (int c = lane; c < ld; c += 32) o[c] = 0.0;
+        if (lane == 0) wv[buf * kSmRows + rr] = 0.0;
+      }
+      for (int c = nf + 1 + lane; c < ld; c += 32) o[c] = 0.0;
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  // This warp's output tiles: warp, warp + kWarps, ... of nt x nt, kMost at a time.
+  constexpr int kMost = 4;
+  double cx = 0.0, cy = 0.0, cn = 0.0;
+  for (int t0 = 0; t0 < nt * nt; t0 += kMost * kWarps) {
+    double acc[kMost][2];
+#pragma unroll
+    for (int u = 0; u < kMost; ++u) acc[u][0] = acc[u][1] = 0.0;
+    __syncthreads();
+    if (n > 0) stage(0, 0);
+    int buf = 0;
+    for (int i0 = 0; i0 < n; i0 += kSmRows) {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+      __syncthreads();  // this chunk is in place, the previous one is read
+      const double* cur = rows + buf * kSmRows * ld;
+      const double* cw = wv + buf * kSmRows;
+      for (int e = tid; e < kSmRows * 8 * nt; e += kSmThreads) {
+        const int rr = e / (8 * nt), c = e - rr * 8 * nt;
+        wrow[rr * ld + c] = cw[rr] * cur[rr * ld + c];
+      }
+      if (t0 == 0 && tid < kSmRows && active(i0 + tid)) {
+        cx += static_cast<double>(R.px[base + i0 + tid]);
+        cy += static_cast<double>(R.py[base + i0 + tid]);
+        cn += 1.0;
+      }
+      buf ^= 1;
+      if (i0 + kSmRows < n) stage(i0 + kSmRows, buf);
+      __syncthreads();
+#pragma unroll
+      for (int u = 0; u < kMost; ++u) {
+        const int t = t0 + u * kWarps + warp;
+        if (t >= nt * nt) break;
+        const double* A = wrow + kq * ld + 8 * (t / nt) + q;
+        const double* B = cur + kq * ld + 8 * (t % nt) + q;
+#pragma unroll
+        for (int k0 = 0; k0 < kSmRows; k0 += 4) dmma_gls(acc[u], A[k0 * ld], B[k0 * ld]);
       }
     }
-    const double tot = acc;
-    if (e < nf * nf)
-      As[static_cast<size_t>(s) * nf * nf + e] = tot;
-    else if (e < nf * nf + nf)
-      rs[static_cast<size_t>(s) * nf + (e - nf * nf)] = tot;
-    else if (e == nf * nf + nf)
-      ds2[s] = tot;
-    else
-      cen[static_cast<size_t>(s) * 3 + (e - nf * nf - nf - 1)] = tot;
+#pragma unroll
+    for (int u = 0; u < kMost; ++u) {
+      const int t = t0 + u * kWarps + warp;
+      if (t >= nt * nt) break;
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int a = 8 * (t / nt) + q, b = 8 * (t % nt) + 2 * kq + e;
+        if (a < nf && b < nf)
+          As[(static_cast<size_t>(s) * nf + a) * nf + b] = acc[u][e];
+        else if (a == nf && b < nf)
+          rs[static_cast<size_t>(s) * nf + b] = acc[u][e];
+        else if (a == nf && b == nf)
+          ds2[s] = acc[u][e];
+      }
+    }
   }
+  // Centroid sums: whole numbers, exact in any order.
+  __shared__ double red[3][2];
+  if (warp < 2) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      cx += __shfl_xor_sync(0xffffffffu, cx, o);
+      cy += __shfl_xor_sync(0xffffffffu, cy, o);
+      cn += __shfl_xor_sync(0xffffffffu, cn, o);
+    }
+    if (lane == 0) {
+      red[0][warp] = cx;
+      red[1][warp] = cy;
+      red[2][warp] = cn;
+    }
+  }
+  __syncthreads();
+  if (tid < 3) cen[static_cast<size_t>(s) * 3 + tid] = red[tid][0] + red[tid][1];
 }
 
 void launch_stamp_moments(cudaStream_t st, int n_stamps, int nc, int SS, const FitRows& R, const uint8_t* accepted,
                           double* As, double* rs, double* ds2, double* cen) {
   if (n_stamps == 0) return;
-  k_stamp_moments<<<n_stamps, 256, 0, st>>>(nc, SS, R, accepted, As, rs, ds2, cen);
+  const size_t smem = stamp_moments_smem(nc + 1);
+  ensure_dynamic_smem(reinterpret_cast<const void*>(k_stamp_moments), smem);
+  k_stamp_moments<<<n_stamps, kSmThreads, smem, st>>>(nc, SS, R, accepted, As, rs, ds2, cen);
   DGPU_LAUNCH("k_stamp_moments");
 }
 
 // Fold assembly M_g = sum_{s in g} A_s (x) d_s d_s^T, rf_g(c-block) = sum r_s(c) d_s,
-// ysq_g = sum ds2_s (src/solve.cpp:605-629).
-__global__ void k_stamped_assemble(int groups, int nstamp, int nf, int k, const int* __restrict__ fold,
-                                   const double* __restrict__ As, const double* __restrict__ rs,
-                                   const double* __restrict__ ds2, const double* __restrict__ dsd,
-                                   double* __restrict__ Mg, double* __restrict__ rg, double* __restrict__ yg) {
-  const int P = nf * k;
-  const size_t per = static_cast<size_t>(P) * P + P + 1;
-  const size_t total = static_cast<size_t>(groups) * per;
-  for (size_t e = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < total;
-       e += static_cast<size_t>(gridDim.x) * blockDim.x) {
-    const int g = static_cast<int>(e / per);
-    const size_t o = e - static_cast<size_t>(g) * per;
-    double acc = 0.0;
-    if (o < static_cast<size_t>(P) * P) {
-      const int p = static_cast<int>(o / P), q = static_cast<int>(o % P);
-      const int c = p / k, m = p % k, c2 = q / k, m2 = q % k;
-      for (int s = 0; s < nstamp; ++s) {
-        if (fold[s] != g) continue;
-        acc += As[static_cast<size_t>(s) * nf * nf + c * nf + c2] * (dsd[static_cast<size_t>(s) * k + m] *
-                                                                       dsd[static_cast<size_t>(s) * k + m2]);
+// ysq_g = sum ds2_s (src/solve.cpp:605-629), the stamps of a fold in order:
+// list[offs[g] .. offs[g + 1]). A CTA takes kSaPairs field pairs (c, c') of one
+// fold, a thread one design pair (m, m') of them at a time, so a product d_m d_m'
+// serves kSaPairs sums; the last CTA of a fold forms rf and ysq. (A thread per
+// entry of M scanning every stamp took 0.22 ms at 5 folds of 40 stamps, P =
+// 725; this 0.03 ms.)
+constexpr int kSaPairs = 8;
+constexpr int kSaStamps = 64;  // stamps staged at a time
+
+__global__ void __launch_bounds__(256)
+k_stamped_assemble(int nf, int k, const int* __restrict__ list, const int* __restrict__ offs,
+                   const double* __restrict__ As, const double* __restrict__ rs, const double* __restrict__ ds2,
+                   const double* __restrict__ dsd, double* __restrict__ Mg, double* __restrict__ rg,
+                   double* __restrict__ yg) {
+  extern __shared__ __align__(16) double sa[];
+  double* sA = sa;                          // kSaStamps x kSaPairs
+  double* sd = sA + kSaStamps * kSaPairs;   // kSaStamps x k
+  const int g = blockIdx.y, P = nf * k, tid = threadIdx.x;
+  const int b0 = offs[g], b1 = offs[g + 1];
+  if (blockIdx.x == gridDim.x - 1) {
+    for (int p = tid; p <= P; p += 256) {
+      const int c = p / k, m = p - c * k;
+      double acc = 0.0;
+      for (int i = b0; i < b1; ++i) {
+        const int s = list[i];
+        if (p < P)
+          acc += rs[static_cast<size_t>(s) * nf + c] * dsd[static_cast<size_t>(s) * k + m];
+        else
+          acc += ds2[s];
       }
-      Mg[static_cast<size_t>(g) * P * P + o] = acc;
-    } else if (o < static_cast<size_t>(P) * P + P) {
-      const int p = static_cast<int>(o - static_cast<size_t>(P) * P);
-      const int c = p / k, m = p % k;
-      for (int s = 0; s < nstamp; ++s)
-        if (fold[s] == g) acc += rs[static_cast<size_t>(s) * nf + c] * dsd[static_cast<size_t>(s) * k + m];
-      rg[static_cast<size_t>(g) * P + p] = acc;
-    } else {
-      for (int s = 0; s < nstamp; ++s)
-        if (fold[s] == g) acc += ds2[s];
-      yg[g] = acc;
+      if (p < P)
+        rg[static_cast<size_t>(g) * P + p] = acc;
+      else
+        yg[g] = acc;
     }
+    return;
+  }
+  const int e0 = blockIdx.x * kSaPairs, ne = min(kSaPairs, nf * nf - e0);
+  for (int mm0 = 0; mm0 < k * k; mm0 += 256) {
+    const int mm = mm0 + tid, m = mm / k, m2 = mm - m * k;
+    const bool in = mm < k * k;
+    double acc[kSaPairs];
+#pragma unroll
+    for (int e = 0; e < kSaPairs; ++e) acc[e] = 0.0;
+    for (int i0 = b0; i0 < b1; i0 += kSaStamps) {
+      const int n = min(kSaStamps, b1 - i0);
+      __syncthreads();
+      for (int t = tid; t < n * kSaPairs; t += 256) {
+        const int i = t / kSaPairs, e = t - i * kSaPairs;
+        sA[t] = e < ne ? As[static_cast<size_t>(list[i0 + i]) * nf * nf + e0 + e] : 0.0;
+      }
+      for (int t = tid; t < n * k; t += 256) {
+        const int i = t / k;
+        sd[t] = dsd[static_cast<size_t>(list[i0 + i]) * k + (t - i * k)];
+      }
+      __syncthreads();
+      if (in)
+        for (int i = 0; i < n; ++i) {
+          const double dd = sd[i * k + m] * sd[i * k + m2];
+#pragma unroll
+          for (int e = 0; e < kSaPairs; ++e) acc[e] = fma(sA[i * kSaPairs + e], dd, acc[e]);
+        }
+    }
+    if (in)
+      for (int e = 0; e < ne; ++e) {
+        const int c = (e0 + e) / nf, c2 = (e0 + e) - c * nf;
+        double v = 0.0;
+#pragma unroll
+        for (int x = 0; x < kSaPairs; ++x) v = x == e ? acc[x] : v;
+        Mg[static_cast<size_t>(g) * P * P + static_cast<size_t>(c * k + m) * P + c2 * k + m2] = v;
+      }
   }
 }
 
-void launch_stamped_assemble(cudaStream_t st, int groups, int nstamp, int nf, int k, const int* fold,
+void launch_stamped_assemble(cudaStream_t st, int groups, int nf, int k, const int* list, const int* offs,
                              const double* As, const double* rs, const double* ds2, const double* dsd, double* Mg,
                              double* rg, double* yg) {
-  const size_t P = static_cast<size_t>(nf) * k;
-  const size_t total = static_cast<size_t>(groups) * (P * P + P + 1);
-  const int blocks = static_cast<int>(std::min<size_t>((total + 255) / 256, 148 * 16));
-  k_stamped_assemble<<<std::max(blocks, 1), 256, 0, st>>>(groups, nstamp, nf, k, fold, As, rs, ds2, dsd, Mg, rg, yg);
+  const size_t smem = sizeof(double) * kSaStamps * (kSaPairs + static_cast<size_t>(k));
+  ensure_dynamic_smem(reinterpret_cast<const void*>(k_stamped_assemble), smem);
+  k_stamped_assemble<<<dim3((nf * nf + kSaPairs - 1) / kSaPairs + 1, groups), 256, smem, st>>>(nf, k, list, offs, As, rs,
+                                                                                      ds2, dsd, Mg, rg, yg);
   DGPU_LAUNCH("k_stamped_assemble");
 }
 

@@ -558,9 +558,11 @@ __global__ void k_ldlt_finish(SolveBatch b, int s0, LdltWork wk) {
   const int* perm = wk.i + blockIdx.x * (static_cast<size_t>(P) + 1);
   if (threadIdx.x != 0 || !perm[P]) return;
   const double* zc = wk.d + blockIdx.x * ldlt_sys_doubles(P) + 2 * PP + P;
-  double e = 0.0;
-  for (int c = 0; c < P; ++c) e += zc[c];
-  b.edf[s] = e;
+  if (b.want_edf) {
+    double e = 0.0;
+    for (int c = 0; c < P; ++c) e += zc[c];
+    b.edf[s] = e;
+  }
   b.ok[s] = 2;
 }
 
@@ -718,9 +720,11 @@ void launch_ldlt_fallback(Context& c, const SolveBatch& b) {
     const int m = std::min(chunk, b.nsys - s0);
     k_ldlt_factor<<<m, kLdltThreads, kLdltDynSmem, c.stream>>>(b, s0, wk);
     DGPU_LAUNCH("k_ldlt_factor");
-    k_ldlt_trace<<<dim3(m, (b.P + kLdltTraceThreads - 1) / kLdltTraceThreads), kLdltTraceThreads, 0, c.stream>>>(
-        b, s0, wk);
-    DGPU_LAUNCH("k_ldlt_trace");
+    if (b.want_edf) {
+      k_ldlt_trace<<<dim3(m, (b.P + kLdltTraceThreads - 1) / kLdltTraceThreads), kLdltTraceThreads, 0, c.stream>>>(
+          b, s0, wk);
+      DGPU_LAUNCH("k_ldlt_trace");
+    }
     k_ldlt_finish<<<m, 32, 0, c.stream>>>(b, s0, wk);
     DGPU_LAUNCH("k_ldlt_finish");
   }

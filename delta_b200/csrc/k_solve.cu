@@ -603,7 +603,7 @@ __global__ void __launch_bounds__(kSolveThreads, 2) k_solve_cluster(SolveBatch b
   if (tid == 0) {
     double t2 = 0.0;
     for (int q = 0; q < cn; ++q) t2 += b.partial[static_cast<size_t>(s) * cn + q];
-    b.edf[s] = static_cast<double>(y.P) - y.lam * t2;
+    if (b.want_edf) b.edf[s] = static_cast<double>(y.P) - y.lam * t2;
     b.ok[s] = s_ok;
   }
   // theta = L^-T y, y = E row 0: column tiles from the last, each
