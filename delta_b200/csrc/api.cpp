@@ -711,12 +711,10 @@ int dgpu_catalog_fetch(dgpu_context* ctx, const dgpu_catalog_columns* o, int cou
 int dgpu_catalog_labels(dgpu_context* ctx, int mem, int32_t* labels, int64_t n) {
   return guarded(ctx, [&](Context& c) {
     if (n != c.cat_npix) fail(DGPU_ERR_CAPACITY, "catalog_labels: size does not match the last catalog");
-    const void* src = c.slot_ptr[kSlotLabels];
-    if (!src) fail(DGPU_ERR_RUNTIME, "catalog_labels: no catalog has been built");
-    if (mem == DGPU_MEM_DEVICE)
-      DGPU_CUDA(cudaMemcpyAsync(labels, src, sizeof(int32_t) * n, cudaMemcpyDeviceToDevice, c.stream));
-    else
-      DGPU_CUDA(cudaMemcpyAsync(labels, src, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, c.stream));
+    if (!c.slot_ptr[kSlotLabels]) fail(DGPU_ERR_RUNTIME, "catalog_labels: no catalog has been built");
+    int* dst = static_cast<int*>(out_buf(c, mem, labels, sizeof(int32_t) * n, kSlotScratch0));
+    expand_labels(c, n, dst);
+    stage_out(c, mem, labels, dst, sizeof(int32_t) * n);
     DGPU_CUDA(cudaStreamSynchronize(c.stream));
   });
 }

@@ -418,6 +418,8 @@ void launch_basis_convolve(cudaStream_t s, int w, int h, const float* img, const
 
 // Catalog (k_ccl.cu)
 struct CatalogDevResult;
+// Label image (n int32, device) of the last run_catalog, which saw n pixels.
+void expand_labels(Context& c, int64_t n, int* labels);
 int run_catalog(Context& c, int w, int h, const float* score, const float* diff,
                 const uint8_t* mask, const dgpu_catalog_params& p, const float* variance,
                 const float* psf, int psf_size, const double* bright_x, const double* bright_y,

@@ -1,16 +1,22 @@
 // Connected-component source catalog (src/catalog.cpp:61-697) on sm_100a.
 //
-// Seeds -> 8-connected union-find labelling with atomicMin linking (every
-// parent index is below its child, so each component's root is its minimum
-// linear index) -> roots ranked in raster order by a block count + scan, which
-// reproduces the reference's final numbering exactly (label = rank of the
-// component's first pixel in raster order, src/catalog.cpp:124-260) ->
-// per-label reductions with atomics (count, |score|-weighted sums in FP64,
-// peak with the lowest-index tie-break of src/catalog.cpp:362-371, mask OR over
-// footprint + 8-ring) -> per-component finishing (centroid, FWHM consistency,
-// aperture flux, quality bits, dipole flag, optional PSF-shape fit and
-// bright-star distance). Every data-dependent loop is capped; hitting a cap
-// sets the context status word and the call reports DGPU_ERR_LIMIT.
+// Seeds are rare (a few thousand of 1.7e7 pixels), so one pass over the score and
+// mask packs both polarities into bitmaps and everything after it works on the
+// raster-ordered list of the wanted polarity's seed pixels: 8-connected
+// union-find over list positions with atomicMin linking (every parent is below
+// its child, so each component's root is its first pixel in raster order) ->
+// roots ranked in list order, which reproduces the reference's final numbering
+// exactly (label = rank of the component's first pixel in raster order,
+// src/catalog.cpp:124-260) -> per-label reductions with atomics (count,
+// |score|-weighted sums in FP64, peak with the lowest-index tie-break of
+// src/catalog.cpp:362-371, mask OR over footprint + 8-ring, dipole contact) ->
+// per-component finishing (centroid, FWHM consistency, aperture flux, quality
+// bits, dipole flag, optional PSF-shape fit and bright-star distance). A
+// neighbour's list position is the number of seeds before its bitmap word plus
+// the set bits below its own. The label image itself is written only where it
+// is asked for (expand_labels). Every data-dependent loop is capped; hitting a
+// cap sets the context status word and the call reports DGPU_ERR_LIMIT.
+// Floor at 4096^2: reading 5 bytes a pixel, 13 us at 6.5 TB/s.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -21,18 +27,195 @@
 namespace dgpu {
 
 
-__global__ void k_seed(int64_t n, const float* __restrict__ score, const uint8_t* __restrict__ mask,
-                       int exclude, float thr_pos, float thr_neg, uint8_t* __restrict__ seeds) {
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const float v = score[i];
-    const bool fin = isfinite(v);
-    const bool good = !(exclude && mask != nullptr && mask[i] != 0);
-    uint8_t s = 0;
-    if (fin && v >= thr_pos && good) s |= 1;
-    if (fin && v <= -thr_neg && good) s |= 2;
-    seeds[i] = s;
+constexpr int kSeedBlock = 8192;  // pixels per block of the seed pass
+constexpr int kRankBlock = 1024;  // list entries per block of the ranking
+static_assert(kSeedBlock == 8 * 8 * 128, "eight warps of eight groups of 128 pixels");
+
+// The catalog's work arrays, sized for every pixel a seed: bitmaps of the
+// labelled polarity and the other one, the number of listed seeds before each
+// word, the seed list, the union-find parents (list positions), the rank of each
+// root, per-block counts of the seed pass and of the ranking, and
+// {arrival counters (2), seeds, roots}.
+struct SeedList {
+  unsigned* bits;
+  unsigned* other;
+  int* before;
+  int* list;
+  int* parent;
+  int* rank;
+  int* seed_counts;
+  int* root_counts;
+  int* heads;  // [0], [1]: blocks arrived; [2]: seeds; [3]: roots
+
+  static int64_t words(int64_t n) { return (n + 31) / 32; }
+  static int64_t blocks(int64_t n) { return (n + kSeedBlock - 1) / kSeedBlock; }
+  static int64_t ranks(int64_t n) { return (n + kRankBlock - 1) / kRankBlock; }
+  static size_t ints(int64_t n) {
+    return static_cast<size_t>(3 * words(n) + 3 * n + blocks(n) + ranks(n)) + 4;
   }
+  static SeedList at(int* p, int64_t n) {
+    SeedList l;
+    l.heads = p;
+    l.bits = reinterpret_cast<unsigned*>(p + 4);
+    l.other = l.bits + words(n);
+    l.before = reinterpret_cast<int*>(l.other + words(n));
+    l.list = l.before + words(n);
+    l.parent = l.list + n;
+    l.rank = l.parent + n;
+    l.seed_counts = l.rank + n;
+    l.root_counts = l.seed_counts + blocks(n);
+    return l;
+  }
+};
+
+// Exclusive scan of counts[0 .. nb) in place by one block of 256 threads;
+// returns the total to every thread.
+__device__ int block_scan(int* counts, int nb) {
+  __shared__ int part[8];
+  __shared__ int total;
+  const int per = (nb + 255) / 256, lo = min(nb, static_cast<int>(threadIdx.x) * per), hi = min(nb, lo + per);
+  int s = 0;
+#pragma unroll 8
+  for (int i = lo; i < hi; ++i) s += __ldcg(counts + i);
+  int v = s;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += u;
+  }
+  if (lane == 31) part[warp] = v;
+  __syncthreads();
+  int run = v - s;
+  for (int i = 0; i < warp; ++i) run += part[i];
+  if (threadIdx.x == 255) total = run + s;
+  for (int i = lo; i < hi; ++i) {
+    const int c = __ldcg(counts + i);
+    counts[i] = run;
+    run += c;
+  }
+  __syncthreads();
+  return total;
+}
+
+// Does this block arrive last? (Every block's writes before the call are then
+// visible to it; no block waits for another.)
+__device__ bool last_block(int* arrived) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(arrived, 1) == static_cast<int>(gridDim.x) - 1;
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+
+// Bits 0-7 of x to every fourth bit.
+__device__ __forceinline__ unsigned spread4(unsigned x) {
+  x = (x | (x << 12)) & 0x000f000fu;
+  x = (x | (x << 6)) & 0x03030303u;
+  return (x | (x << 3)) & 0x11111111u;
+}
+
+// Bitmaps of both polarities and the labelled one's count per block; the last
+// block scans the counts. A lane takes four adjacent pixels of each group of 128
+// (one 16-byte and one 4-byte load where `vec` says that the images are aligned
+// for it), all eight groups of its warp in flight.
+__global__ void __launch_bounds__(256)
+k_seed_bits(int64_t n, int nb, const float* __restrict__ score, const uint8_t* __restrict__ mask, bool vec,
+            float thr_pos, float thr_neg, bool negative, SeedList sl) {
+  __shared__ int wc[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t base = static_cast<int64_t>(blockIdx.x) * kSeedBlock + warp * 1024 + 4 * lane;
+  float v[8][4];
+  unsigned m[8];  // a byte per pixel, non-zero: excluded
+#pragma unroll
+  for (int g = 0; g < 8; ++g) {
+    const int64_t i = base + 128 * g;
+    if (vec && i + 3 < n) {
+      const float4 t = __ldcs(reinterpret_cast<const float4*>(score + i));
+      v[g][0] = t.x, v[g][1] = t.y, v[g][2] = t.z, v[g][3] = t.w;
+      m[g] = mask != nullptr ? __ldcs(reinterpret_cast<const unsigned*>(mask + i)) : 0u;
+    } else {
+      m[g] = 0u;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        v[g][u] = i + u < n ? __ldcs(score + i + u) : __int_as_float(0x7fc00000);
+        if (mask != nullptr && i + u < n) m[g] |= static_cast<unsigned>(__ldcs(mask + i + u)) << (8 * u);
+      }
+    }
+  }
+  int count = 0;
+#pragma unroll
+  for (int g = 0; g < 8; ++g) {
+    unsigned p[4], q[4];  // one bit per lane, by pixel of the four
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const bool good = isfinite(v[g][u]) && ((m[g] >> (8 * u)) & 0xffu) == 0;
+      p[u] = __ballot_sync(0xffffffffu, good && v[g][u] >= thr_pos);
+      q[u] = __ballot_sync(0xffffffffu, good && v[g][u] <= -thr_neg);
+    }
+    // Word `lane` (0-3) of the group: pixel 4 k + u of it is bit k of byte `lane` of ballot u.
+    const int64_t i = base - 4 * lane + 128 * g + 32 * lane;
+    if (lane < 4 && i < n) {
+      unsigned pw = 0, qw = 0;
+      if (p[0] | p[1] | p[2] | p[3] | q[0] | q[1] | q[2] | q[3])
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          pw |= spread4((p[u] >> (8 * lane)) & 0xffu) << u;
+          qw |= spread4((q[u] >> (8 * lane)) & 0xffu) << u;
+        }
+      sl.bits[i >> 5] = negative ? qw : pw;
+      sl.other[i >> 5] = negative ? pw : qw;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) count += __popc(negative ? q[u] : p[u]);
+  }
+  if (lane == 0) wc[warp] = count;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    int t = 0;
+    for (int i = 0; i < 8; ++i) t += wc[i];
+    sl.seed_counts[blockIdx.x] = t;
+  }
+  if (last_block(&sl.heads[0])) {
+    const int total = block_scan(sl.seed_counts, nb);
+    if (threadIdx.x == 0) sl.heads[2] = total;
+  }
+}
+
+// The seed list in raster order, each seed its own parent.
+__global__ void __launch_bounds__(kSeedBlock / 32)
+k_seed_list(int64_t n, int nb, SeedList sl) {
+  const int b = blockIdx.x;
+  const int at0 = sl.seed_counts[b], at1 = b + 1 < nb ? sl.seed_counts[b + 1] : sl.heads[2];
+  if (at0 == at1) return;
+  __shared__ int wt[kSeedBlock / 32 / 32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t word = static_cast<int64_t>(b) * (kSeedBlock / 32) + threadIdx.x;
+  unsigned bits = word * 32 < n ? sl.bits[word] : 0u;
+  int v = __popc(bits);
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v += u;
+  }
+  if (lane == 31) wt[warp] = v;
+  __syncthreads();
+  int at = at0 + v - __popc(bits);
+  for (int i = 0; i < warp; ++i) at += wt[i];
+  if (word * 32 < n) sl.before[word] = at;
+  while (bits) {
+    sl.list[at] = static_cast<int>(word * 32) + __ffs(bits) - 1;
+    sl.parent[at] = at;
+    ++at;
+    bits &= bits - 1;
+  }
+}
+
+__device__ __forceinline__ bool has_bit(const unsigned* bits, int i) { return (bits[i >> 5] >> (i & 31)) & 1u; }
+__device__ __forceinline__ int list_pos(const SeedList& sl, int i) {
+  return sl.before[i >> 5] + __popc(sl.bits[i >> 5] & ((1u << (i & 31)) - 1u));
 }
 
 __device__ __forceinline__ int find_root(const int* L, int i, unsigned* st, int cap) {
@@ -62,114 +245,96 @@ __device__ void unite(int* L, int a, int b, unsigned* st, int cap) {
   set_status(st, kStatusLoopLimit);
 }
 
-__global__ void k_label_init(int64_t n, const uint8_t* __restrict__ seeds, uint8_t bit, int* __restrict__ L) {
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x)
-    L[i] = (seeds[i] & bit) ? static_cast<int>(i) : -1;
-}
-
-__global__ void k_label_merge(int w, int h, const uint8_t* __restrict__ seeds, uint8_t bit, int* L,
-                              unsigned* st, int cap) {
-  const int64_t n = static_cast<int64_t>(w) * h;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    if (!(seeds[i] & bit)) continue;
-    const int x = static_cast<int>(i % w), y = static_cast<int>(i / w);
-    const int me = static_cast<int>(i);
-    if (x > 0 && (seeds[i - 1] & bit)) unite(L, me, me - 1, st, cap);
-    if (y > 0) {
-      const int64_t a = i - w;
-      if (x > 0 && (seeds[a - 1] & bit)) unite(L, me, static_cast<int>(a - 1), st, cap);
-      if (seeds[a] & bit) unite(L, me, static_cast<int>(a), st, cap);
-      if (x + 1 < w && (seeds[a + 1] & bit)) unite(L, me, static_cast<int>(a + 1), st, cap);
+__global__ void k_label_merge(int w, SeedList sl, unsigned* st, int cap) {
+  const int n = sl.heads[2];
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+    const int i = sl.list[e], x = i % w;
+    if (x > 0 && has_bit(sl.bits, i - 1)) unite(sl.parent, e, e - 1, st, cap);
+    if (i >= w) {
+      const int a = i - w;
+      if (x > 0 && has_bit(sl.bits, a - 1)) unite(sl.parent, e, list_pos(sl, a - 1), st, cap);
+      if (has_bit(sl.bits, a)) unite(sl.parent, e, list_pos(sl, a), st, cap);
+      if (x + 1 < w && has_bit(sl.bits, a + 1)) unite(sl.parent, e, list_pos(sl, a + 1), st, cap);
     }
   }
 }
 
-__global__ void k_label_flatten(int64_t n, int* L, unsigned* st, int cap) {
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    if (L[i] >= 0) L[i] = find_root(L, static_cast<int>(i), st, cap);
-  }
-}
-
-constexpr int kRankBlock = 1024;
-
-__global__ void k_root_count(int64_t n, const int* __restrict__ L, int* __restrict__ counts) {
-  __shared__ int s;
-  if (threadIdx.x == 0) s = 0;
-  __syncthreads();
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * kRankBlock + threadIdx.x;
-  const bool root = i < n && L[i] == static_cast<int>(i);
-  const unsigned bal = __ballot_sync(0xffffffffu, root);
-  if ((threadIdx.x & 31) == 0 && bal) atomicAdd(&s, __popc(bal));
-  __syncthreads();
-  if (threadIdx.x == 0) counts[blockIdx.x] = s;
-}
-
-// Exclusive scan of per-block root counts in one CTA; writes the total.
-__global__ void k_scan_counts(int nb, int* counts, int* total) {
-  __shared__ int part[1024];
-  const int per = (nb + blockDim.x - 1) / blockDim.x;
-  const int lo = threadIdx.x * per, hi = min(nb, lo + per);
-  int s = 0;
-  for (int i = lo; i < hi; ++i) s += counts[i];
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (int off = 1; off < static_cast<int>(blockDim.x); off <<= 1) {
-    const int v = threadIdx.x >= static_cast<unsigned>(off) ? part[threadIdx.x - off] : 0;
+// Parents to roots; the roots of each block of list entries are counted and the
+// last block scans the counts.
+__global__ void __launch_bounds__(256) k_label_flatten(SeedList sl, unsigned* st, int cap) {
+  __shared__ int wc[8];
+  const int n = sl.heads[2], nb = (n + kRankBlock - 1) / kRankBlock;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+    int count = 0;
+    for (int e0 = b * kRankBlock + warp * 128; e0 < b * kRankBlock + (warp + 1) * 128; e0 += 32) {
+      const int e = e0 + lane;
+      int r = -1;
+      if (e < n) {
+        r = find_root(sl.parent, e, st, cap);
+        sl.parent[e] = r;
+      }
+      count += __popc(__ballot_sync(0xffffffffu, e < n && r == e));
+    }
+    if (lane == 0) wc[warp] = count;
     __syncthreads();
-    part[threadIdx.x] += v;
+    if (threadIdx.x == 0) {
+      int t = 0;
+      for (int i = 0; i < 8; ++i) t += wc[i];
+      sl.root_counts[b] = t;
+    }
     __syncthreads();
   }
-  int run = part[threadIdx.x] - s;
-  for (int i = lo; i < hi; ++i) {
-    const int c = counts[i];
-    counts[i] = run;
-    run += c;
+  if (last_block(&sl.heads[1])) {
+    const int total = block_scan(sl.root_counts, nb);
+    if (threadIdx.x == 0) sl.heads[3] = total;
   }
-  if (threadIdx.x == blockDim.x - 1) *total = part[threadIdx.x];
 }
 
-// rank_at[root] = raster rank of the root (0-based).
-__global__ void k_root_rank(int64_t n, const int* __restrict__ L, const int* __restrict__ offsets,
-                            int* __restrict__ rank_at) {
-  __shared__ int warp_tot[kRankBlock / 32];
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * kRankBlock + threadIdx.x;
-  const bool root = i < n && L[i] == static_cast<int>(i);
-  const unsigned bal = __ballot_sync(0xffffffffu, root);
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  if (lane == 0) warp_tot[wid] = __popc(bal);
-  __syncthreads();
-  if (wid == 0) {
-    int v = warp_tot[lane];
-    for (int o = 1; o < 32; o <<= 1) {
-      const int u = __shfl_up_sync(0xffffffffu, v, o);
-      if (lane >= o) v += u;
+// rank[root] = raster rank of the root (0-based).
+__global__ void __launch_bounds__(256) k_root_rank(SeedList sl) {
+  __shared__ int wc[8];
+  const int n = sl.heads[2], nb = (n + kRankBlock - 1) / kRankBlock;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int b = blockIdx.x; b < nb; b += gridDim.x) {
+    unsigned roots[4];
+    int count = 0;
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const int e = b * kRankBlock + warp * 128 + g * 32 + lane;
+      roots[g] = __ballot_sync(0xffffffffu, e < n && sl.parent[e] == e);
+      count += __popc(roots[g]);
     }
-    warp_tot[lane] = v - warp_tot[lane];  // exclusive
+    __syncthreads();
+    if (lane == 0) wc[warp] = count;
+    __syncthreads();
+    int at = sl.root_counts[b];
+    for (int i = 0; i < warp; ++i) at += wc[i];
+#pragma unroll
+    for (int g = 0; g < 4; ++g) {
+      const int e = b * kRankBlock + warp * 128 + g * 32 + lane;
+      if (roots[g] & (1u << lane)) sl.rank[e] = at + __popc(roots[g] & ((1u << lane) - 1u));
+      at += __popc(roots[g]);
+    }
   }
-  __syncthreads();
-  if (root) rank_at[i] = offsets[blockIdx.x] + warp_tot[wid] + __popc(bal & ((1u << lane) - 1));
 }
 
-// Only a root carries a rank, so a pixel maps to a label only through a root:
-// one left pointing at a non-root (a capped search gave up) gets label 0 and
-// the bounds status, which keeps every label within [1, number of roots].
-__global__ void k_label_final(int64_t n, const int* __restrict__ L, const int* __restrict__ rank_at,
-                              int* __restrict__ labels, unsigned* st) {
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int r = L[i];
-    int lbl = 0;
-    if (r >= 0) {
-      if (L[r] == r)
-        lbl = rank_at[r] + 1;
-      else
-        set_status(st, kStatusBounds);
-    }
-    labels[i] = lbl;
-  }
+// Component (label - 1) of list entry e. Only a root carries a rank, so an entry
+// maps to a component only through a root: one left pointing at a non-root (a
+// capped search gave up) gets -1 and the bounds status, which keeps every
+// component within [0, number of roots).
+__device__ __forceinline__ int component_of(const SeedList& sl, int e, unsigned* st) {
+  const int r = sl.parent[e];
+  if (sl.parent[r] == r) return sl.rank[r];
+  set_status(st, kStatusBounds);
+  return -1;
+}
+
+// The label image: zeros, then label = component + 1 at the seeds.
+__global__ void k_expand_labels(SeedList sl, int* __restrict__ labels, unsigned* st) {
+  const int n = sl.heads[2];
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x)
+    labels[sl.list[e]] = component_of(sl, e, st) + 1;
 }
 
 // Per-component accumulators (index label-1).
@@ -184,17 +349,18 @@ struct CompStats {
   int* first;  // minimum linear index (the root)
 };
 
-__global__ void k_comp_reduce(int w, int h, const int* __restrict__ labels, const float* __restrict__ score,
-                              const uint8_t* __restrict__ mask, CompStats cs) {
-  const int64_t n = static_cast<int64_t>(w) * h;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int lbl = labels[i];
-    if (lbl <= 0) continue;
-    const int c = lbl - 1;
-    const int x = static_cast<int>(i % w), y = static_cast<int>(i / w);
-    const double v = static_cast<double>(score[i]);
-    const double wt = fabs(v);
+// Reductions of every seed into its component. A seed's 8-neighbours of the same
+// polarity are in its own component, so the mask ring takes the neighbours that
+// are not seeds; a neighbour (or the pixel itself) carrying the other polarity
+// marks the component (flag_dipole_positives, src/catalog.cpp:431-458).
+__global__ void k_comp_reduce(int w, int h, SeedList sl, const float* __restrict__ score,
+                              const uint8_t* __restrict__ mask, CompStats cs, unsigned* st) {
+  const int n = sl.heads[2];
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
+    const int c = component_of(sl, e, st);
+    if (c < 0) continue;
+    const int i = sl.list[e], x = i % w, y = i / w;
+    const double wt = fabs(static_cast<double>(score[i]));
     atomicAdd(&cs.count[c], 1);
     atomicAdd(&cs.sum[c], wt);
     atomicAdd(&cs.sx[c], wt * x);
@@ -203,44 +369,20 @@ __global__ void k_comp_reduce(int w, int h, const int* __restrict__ labels, cons
         (static_cast<unsigned long long>(__float_as_uint(fabsf(score[i]))) << 32) |
         static_cast<unsigned long long>(0xffffffffu - static_cast<unsigned>(i));
     atomicMax(&cs.peak[c], key);
-    atomicMin(&cs.first[c], static_cast<int>(i));
-    if (mask) {
-      unsigned m = mask[i];
-      for (int dy = -1; dy <= 1; ++dy) {
-        const int yy = y + dy;
-        if (yy < 0 || yy >= h) continue;
-        for (int dx = -1; dx <= 1; ++dx) {
-          if (dx == 0 && dy == 0) continue;
-          const int xx = x + dx;
-          if (xx < 0 || xx >= w) continue;
-          const int64_t j = static_cast<int64_t>(yy) * w + xx;
-          if (labels[j] != lbl) m |= mask[j];
-        }
-      }
-      if (m) atomicOr(&cs.mask_or[c], m);
-    }
-  }
-}
-
-// Opposite-polarity seeds touching a label's 3x3 neighbourhood
-// (flag_dipole_positives, src/catalog.cpp:431-458).
-__global__ void k_dipole_touch(int w, int h, const uint8_t* __restrict__ seeds, uint8_t other_bit,
-                               const int* __restrict__ labels, unsigned* touched) {
-  const int64_t n = static_cast<int64_t>(w) * h;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    if (!(seeds[i] & other_bit)) continue;
-    const int x = static_cast<int>(i % w), y = static_cast<int>(i / w);
-    for (int dy = -1; dy <= 1; ++dy) {
-      const int yy = y + dy;
-      if (yy < 0 || yy >= h) continue;
+    atomicMin(&cs.first[c], i);
+    unsigned m = mask ? mask[i] : 0u;
+    bool touched = false;
+#pragma unroll
+    for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
       for (int dx = -1; dx <= 1; ++dx) {
-        const int xx = x + dx;
-        if (xx < 0 || xx >= w) continue;
-        const int l = labels[static_cast<int64_t>(yy) * w + xx];
-        if (l > 0) touched[l - 1] = 1u;
+        if (y + dy < 0 || y + dy >= h || x + dx < 0 || x + dx >= w) continue;
+        const int j = i + dy * w + dx;
+        touched = touched || has_bit(sl.other, j);
+        if (mask && !has_bit(sl.bits, j)) m |= mask[j];
       }
-    }
+    if (m) atomicOr(&cs.mask_or[c], m);
+    if (touched) cs.touched[c] = 1u;
   }
 }
 
@@ -279,13 +421,14 @@ struct FinishParams {
 __device__ long lround_away(double v) { return static_cast<long>(v >= 0 ? floor(v + 0.5) : -floor(-v + 0.5)); }
 
 // summarize_component (src/catalog.cpp:337-418) finishing + dipole flag +
-// enrich_entries (src/catalog.cpp:476-596).
-__global__ void k_comp_finish(int ncomp, int w, int h, const float* __restrict__ score,
+// enrich_entries (src/catalog.cpp:476-596). A warp per component: its lanes load
+// the aperture's pixels together and every lane adds them in raster order.
+__global__ void __launch_bounds__(128) k_comp_finish(int ncomp, int w, int h, const float* __restrict__ score,
                               const float* __restrict__ diff, const uint8_t* __restrict__ mask,
                               const float* __restrict__ variance, const float* __restrict__ psf,
                               const double* __restrict__ bx, const double* __restrict__ by, int nb,
                               CompStats cs, FinishParams fp, CompOut o) {
-  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (c >= ncomp) return;
   const double kFwhmPerSigma = 2.354820045030949;
   const double kPi = 3.14159265358979323846;
@@ -319,20 +462,22 @@ __global__ void k_comp_finish(int ncomp, int w, int h, const float* __restrict__
   {
     const int x0 = static_cast<int>(lround_away(x)), y0 = static_cast<int>(lround_away(y));
     const double r2 = static_cast<double>(radius) * radius;
+    const int64_t side = 2 * static_cast<int64_t>(radius) + 1, area = side * side;
     double fsum = 0.0;
-    for (int dy = -radius; dy <= radius; ++dy) {
-      const int yy = y0 + dy;
-      if (yy < 0 || yy >= h) continue;
-      for (int dx = -radius; dx <= radius; ++dx) {
-        if (dx * dx + dy * dy > r2) continue;
-        const int xx = x0 + dx;
-        if (xx < 0 || xx >= w) continue;
-        const float v = diff[static_cast<int64_t>(yy) * w + xx];
-        if (isfinite(v)) fsum += static_cast<double>(v);
-      }
+    for (int64_t e0 = 0; e0 < area; e0 += 32) {
+      const int64_t e = e0 + lane;
+      const int dy = static_cast<int>(e / side) - radius, dx = static_cast<int>(e % side) - radius;
+      const int yy = y0 + dy, xx = x0 + dx;
+      float v = 0.0f;
+      if (e < area && yy >= 0 && yy < h && xx >= 0 && xx < w && !(dx * dx + dy * dy > r2))
+        v = diff[static_cast<int64_t>(yy) * w + xx];
+      const unsigned in = __ballot_sync(0xffffffffu, v != 0.0f && isfinite(v));  // adding a zero changes nothing
+      for (unsigned left = in; left; left &= left - 1)
+        fsum += static_cast<double>(__shfl_sync(0xffffffffu, v, __ffs(left) - 1));
     }
     o.flux[c] = fsum;
   }
+  if (lane != 0) return;
   uint8_t q = 0;
   if (!consistent) q |= 1u;
   if (mflags != 0) q |= 4u;
@@ -409,36 +554,14 @@ __global__ void k_comp_finish(int ncomp, int w, int h, const float* __restrict__
 // Host driver
 // ---------------------------------------------------------------------------
 
-static int grid_for(int64_t n, int threads = 256) {
-  return static_cast<int>(std::min<int64_t>((n + threads - 1) / threads, 148 * 16));
-}
+// Blocks of the kernels that walk the seed list (its length is on the device).
+constexpr int kListBlocks = 148 * 2;
 
-// Label the seeds carrying `bit`; labels written to `labels`, returns count.
-static int label_polarity(Context& c, int w, int h, const uint8_t* seeds, uint8_t bit, int* labels) {
-  cudaStream_t s = c.stream;
-  const int64_t n = static_cast<int64_t>(w) * h;
-  int* L = static_cast<int*>(c.slot(kSlotScratch0, sizeof(int) * n));
-  int* rank_at = static_cast<int*>(c.slot(kSlotRootRank, sizeof(int) * n));
-  const int nb = static_cast<int>((n + kRankBlock - 1) / kRankBlock);
-  int* counts = static_cast<int*>(c.slot(kSlotBlockCounts, sizeof(int) * (nb + 2)));
-  k_label_init<<<grid_for(n), 256, 0, s>>>(n, seeds, bit, L);
-  DGPU_LAUNCH("k_label_init");
-  k_label_merge<<<grid_for(n), 256, 0, s>>>(w, h, seeds, bit, L, c.d_status, c.label_loop_cap);
-  DGPU_LAUNCH("k_label_merge");
-  k_label_flatten<<<grid_for(n), 256, 0, s>>>(n, L, c.d_status, c.label_loop_cap);
-  DGPU_LAUNCH("k_label_flatten");
-  k_root_count<<<nb, kRankBlock, 0, s>>>(n, L, counts);
-  DGPU_LAUNCH("k_root_count");
-  k_scan_counts<<<1, 1024, 0, s>>>(nb, counts, counts + nb);
-  DGPU_LAUNCH("k_scan_counts");
-  k_root_rank<<<nb, kRankBlock, 0, s>>>(n, L, counts, rank_at);
-  DGPU_LAUNCH("k_root_rank");
-  k_label_final<<<grid_for(n), 256, 0, s>>>(n, L, rank_at, labels, c.d_status);
-  DGPU_LAUNCH("k_label_final");
-  int total = 0;
-  read_back(c, &total, counts + nb, sizeof(int));
-  sync_reads(c);
-  return total;
+void expand_labels(Context& c, int64_t n, int* labels) {
+  const SeedList sl = SeedList::at(static_cast<int*>(c.slot_ptr[kSlotLabels]), n);
+  DGPU_CUDA(cudaMemsetAsync(labels, 0, sizeof(int) * n, c.stream));
+  k_expand_labels<<<kListBlocks, 256, 0, c.stream>>>(sl, labels, c.d_status);
+  DGPU_LAUNCH("k_expand_labels");
 }
 
 int run_catalog(Context& c, int w, int h, const float* score, const float* diff, const uint8_t* mask,
@@ -446,21 +569,32 @@ int run_catalog(Context& c, int w, int h, const float* score, const float* diff,
                 const double* bright_x, const double* bright_y, int n_bright) {
   cudaStream_t s = c.stream;
   const int64_t n = static_cast<int64_t>(w) * h;
-  uint8_t* seeds = static_cast<uint8_t*>(c.slot(kSlotSeedPos, n));
-  int* labels = static_cast<int*>(c.slot(kSlotLabels, sizeof(int) * n));
+  const SeedList sl = SeedList::at(static_cast<int*>(c.slot(kSlotLabels, sizeof(int) * SeedList::ints(n))), n);
+  const bool neg = p.return_negative != 0;
+  const int nb = static_cast<int>(SeedList::blocks(n));
   {
     StageTimer t(c, "catalog: seed");
-    k_seed<<<grid_for(n), 256, 0, s>>>(n, score, mask, p.exclude_bad_pixels ? 1 : 0,
-                                       static_cast<float>(p.threshold_sigma),
-                                       static_cast<float>(p.threshold_sigma_dipole), seeds);
-    DGPU_LAUNCH("k_seed");
+    DGPU_CUDA(cudaMemsetAsync(sl.heads, 0, sizeof(int) * 4, s));
+    const uint8_t* excluded = p.exclude_bad_pixels ? mask : nullptr;
+    const bool vec = reinterpret_cast<uintptr_t>(score) % 16 == 0 && reinterpret_cast<uintptr_t>(excluded) % 4 == 0;
+    k_seed_bits<<<nb, 256, 0, s>>>(n, nb, score, excluded, vec,
+                                   static_cast<float>(p.threshold_sigma),
+                                   static_cast<float>(p.threshold_sigma_dipole), neg, sl);
+    DGPU_LAUNCH("k_seed_bits");
   }
-  const bool neg = p.return_negative != 0;
-  const uint8_t bit = neg ? 2 : 1, other = neg ? 1 : 2;
-  int ncomp;
+  int ncomp = 0;
   {
     StageTimer t(c, neg ? "catalog: label negative" : "catalog: label positive");
-    ncomp = label_polarity(c, w, h, seeds, bit, labels);
+    k_seed_list<<<nb, kSeedBlock / 32, 0, s>>>(n, nb, sl);
+    DGPU_LAUNCH("k_seed_list");
+    k_label_merge<<<kListBlocks, 256, 0, s>>>(w, sl, c.d_status, c.label_loop_cap);
+    DGPU_LAUNCH("k_label_merge");
+    k_label_flatten<<<kListBlocks, 256, 0, s>>>(sl, c.d_status, c.label_loop_cap);
+    DGPU_LAUNCH("k_label_flatten");
+    k_root_rank<<<kListBlocks, 256, 0, s>>>(sl);
+    DGPU_LAUNCH("k_root_rank");
+    read_back(c, &ncomp, sl.heads + 3, sizeof(int));
+    sync_reads(c);
   }
   c.cat_npix = n;
   c.cat_count = ncomp;
@@ -493,10 +627,8 @@ int run_catalog(Context& c, int w, int h, const float* score, const float* diff,
   (void)stats_bytes;
   DGPU_CUDA(cudaMemsetAsync(sb, 0, zero_bytes, s));
   DGPU_CUDA(cudaMemsetAsync(cs.first, 0x7f, 4 * nc, s));
-  k_comp_reduce<<<grid_for(n), 256, 0, s>>>(w, h, labels, score, mask, cs);
+  k_comp_reduce<<<kListBlocks, 256, 0, s>>>(w, h, sl, score, mask, cs, c.d_status);
   DGPU_LAUNCH("k_comp_reduce");
-  k_dipole_touch<<<grid_for(n), 256, 0, s>>>(w, h, seeds, other, labels, cs.touched);
-  DGPU_LAUNCH("k_dipole_touch");
 
   // Output columns: 12 doubles, 4 int32 (peak_x, peak_y, n_pix, psf_chi2_dof), 8 u8.
   const size_t out_bytes = nc * (12 * 8 + 4 * 4 + 8) + 512;
@@ -538,7 +670,7 @@ int run_catalog(Context& c, int w, int h, const float* score, const float* diff,
   fp.shape_tol = p.shape_chi2_tolerance;
   fp.bright_radius = p.bright_star_radius > 0.0 ? p.bright_star_radius : 3.0 * p.expected_fwhm;
   fp.psf_size = psf_size;
-  k_comp_finish<<<(ncomp + 127) / 128, 128, 0, s>>>(ncomp, w, h, score, diff, mask, variance, psf,
+  k_comp_finish<<<(ncomp + 3) / 4, 128, 0, s>>>(ncomp, w, h, score, diff, mask, variance, psf,
                                                      bright_x, bright_y, n_bright, cs, fp, o);
   DGPU_LAUNCH("k_comp_finish");
   // Bring the columns back into the context (host).
