@@ -72,7 +72,7 @@ int dgpu_detect_stamps(dgpu_context* ctx, int mem, int64_t width, int64_t height
     const auto* d = static_cast<const float*>(stage_in(c, mem, data, 4 * n, kSlotInSci));
     const auto* m = static_cast<const uint8_t*>(stage_in(c, mem, mask, n, kSlotInMaskS));
     DetectHost r;
-    const int k = run_detect(c, w, h, d, m, resolve(params), 0, r);
+    const int k = run_detect(c, w, h, d, m, resolve(params), r);
     *count = k;
     for (int i = 0; i < k && i < capacity; ++i) {
       x[i] = r.x[i];

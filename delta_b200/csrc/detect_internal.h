@@ -22,9 +22,10 @@ struct DetectHost {
   std::vector<double> flux, snr, fwhm;
 };
 
-int run_detect(Context& c, int w, int h, const float* img, const uint8_t* mask, const DetectParamsDev& p, int which,
+// Full detect pipeline of one image; returns the kept count.
+int run_detect(Context& c, int w, int h, const float* img, const uint8_t* mask, const DetectParamsDev& p,
                DetectHost& res);
-// run_detect of two images (workspace slots 0 and 1) sharing each synchronisation.
+// run_detect of two images in the same launches, sharing the synchronisation.
 void run_detect_pair(Context& c, int w, int h, const float* img0, const uint8_t* mask0, const float* img1,
                      const uint8_t* mask1, const DetectParamsDev& p, DetectHost& res0, DetectHost& res1);
 void run_background(Context& c, int64_t n, const float* img, const uint8_t* mask, double* median, double* sigma);

@@ -7,7 +7,9 @@
 //    with a fully on-frame, finite, unmasked, unsaturated stamp footprint;
 //  * per-candidate flux-weighted second-moment FWHM (FP64);
 //  * candidates sorted by flux descending (raster index ascending on ties),
-//    then brightest-first greedy isolation in one CTA, chunk by chunk.
+//    then brightest-first greedy isolation, both in one CTA.
+// Both images of a pair go through each launch together, and nothing is read
+// back until the kept stamps are measured.
 #include <cuda_runtime.h>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -21,38 +23,18 @@
 
 namespace dgpu {
 
-// ---------------------------------------------------------------------------
-// Sample medians: the radix select of k_select.cu on a flat-index-strided
-// sample, and the absolute-deviation transform for the MAD.
-// ---------------------------------------------------------------------------
-// keys <- key(|value - med|) in place (src/detect.cpp:110).
-__global__ void k_abs_dev(const RadixSelect* st, const float* __restrict__ med, uint32_t* __restrict__ keys) {
-  const unsigned count = st->count;
-  const float m = *med;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x)
-    keys[i] = float_key(fabsf(key_float(keys[i]) - m));
-}
-
-static void select_median(cudaStream_t s, RadixSelect* st, const uint32_t* keys, int64_t cap, float* out) {
-  launch_select_upper_median(s, st, keys, cap, out);
-}
-
-// bgout[0] = median (float), bgout[1] = MAD (float)
-void launch_background(Context& c, int64_t n, const float* img, const uint8_t* mask, float* bgout, Slot sel_slot,
-                       Slot key_slot) {
-  cudaStream_t s = c.stream;
+// The background sample of an image: about 2^18 pixels at a fixed flat step;
+// out[0] = median, out[1] = MAD (src/detect.cpp:100-112).
+static MedianJob background_job(int64_t n, const float* img, const uint8_t* mask, float* out) {
   constexpr int64_t kTarget = 1 << 18;
-  const int64_t step = n > kTarget ? n / kTarget : 1;
-  const int64_t ns = (n + step - 1) / step;
-  RadixSelect* st = static_cast<RadixSelect*>(c.slot(sel_slot, sizeof(RadixSelect)));
-  uint32_t* keys = static_cast<uint32_t*>(c.slot(key_slot, sizeof(uint32_t) * std::max<int64_t>(ns, 1)));
-  DGPU_CUDA(cudaMemsetAsync(st, 0, sizeof(RadixSelect), s));
-  const int blocks = static_cast<int>(std::min<int64_t>((ns + 255) / 256, 148 * 8));
-  launch_sample_keys(s, n, step, img, mask, keys, st);
-  select_median(s, st, keys, ns, bgout);
-  k_abs_dev<<<std::max(blocks, 1), 256, 0, s>>>(st, bgout, keys);
-  DGPU_LAUNCH("k_abs_dev");
-  select_median(s, st, keys, ns, bgout + 1);
+  MedianJob j;
+  j.v = img;
+  j.mask = mask;
+  j.n = n;
+  j.step = n > kTarget ? n / kTarget : 1;
+  j.out = out;
+  j.mad = 1;
+  return j;
 }
 
 // ---------------------------------------------------------------------------
@@ -108,161 +90,368 @@ __device__ double fwhm_dev(const float* img, int w, int h, int x, int y, int r, 
   return 2.354820045030949 * sqrt(var);
 }
 
-__global__ void k_peaks(int w, int h, const float* __restrict__ img, const float* __restrict__ bg,
-                        DetectParamsDev p, unsigned* count, int cap, int* __restrict__ cand) {
-  const double med = static_cast<double>(bg[0]);
-  const double sigma = 1.4826 * static_cast<double>(bg[1]);
+// One image of a launch over up to two.
+struct DetectDev {
+  const float* img;
+  const uint8_t* mask;
+  const float* bg;    // median, MAD
+  unsigned* count;    // [0] candidates, [1] 3x3 peaks, [2] kept, [3] 1: too many candidates for the fast path
+  int* peaks;         // raster indices
+  int* cand;          // peaks whose stamp footprint is usable
+  int* kept;          // max_stamps
+  double* props;      // 3 x max_stamps: flux, S/N, FWHM
+};
+struct DetectPair {
+  DetectDev d[kMedianJobs];
+};
+
+// 3x3 maxima above the threshold, 256 adjacent pixels of a row per warp. The
+// comparisons are those of the FP64 values: v > t for a float v and a double t
+// is v > (the largest float <= t). Bound by reading the image (4 bytes a pixel).
+constexpr int kPeakSpan = 256;
+
+__global__ void __launch_bounds__(256) k_peaks(int w, int h, DetectPair jobs, DetectParamsDev p, int cap) {
+  const DetectDev j = jobs.d[blockIdx.y];
+  const double med = static_cast<double>(j.bg[0]);
+  const double sigma = 1.4826 * static_cast<double>(j.bg[1]);
   const double thr = med + p.threshold_sigma * (sigma > 0.0 ? sigma : 1.0);
-  const int b = p.border;
-  const int64_t n = static_cast<int64_t>(w) * h;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int x = static_cast<int>(i % w), y = static_cast<int>(i / w);
-    if (y < b || y >= h - b || x < b || x >= w - b) continue;
-    if (x < 1 || y < 1 || x >= w - 1 || y >= h - 1) continue;  // 3x3 window on frame
-    const double v = static_cast<double>(img[i]);
-    if (!(v > thr)) continue;
-    bool peak = true;
-    for (int dy = -1; dy <= 1 && peak; ++dy)
-      for (int dx = -1; dx <= 1; ++dx) {
-        if (dx == 0 && dy == 0) continue;
-        if (static_cast<double>(img[i + static_cast<int64_t>(dy) * w + dx]) > v) {
-          peak = false;
-          break;
-        }
-      }
-    if (!peak) continue;
-    const unsigned slot = atomicAdd(count, 1u);
-    if (static_cast<int>(slot) < cap) cand[slot] = static_cast<int>(i);
+  float t = static_cast<float>(thr);
+  if (static_cast<double>(t) > thr) t = nextafterf(t, -INFINITY);
+  const int b = max(p.border, 1);  // and the 3x3 window on the frame
+  const int lane = threadIdx.x & 31, spans = (w + kPeakSpan - 1) / kPeakSpan;
+  const int warps = static_cast<int>((gridDim.x * blockDim.x) >> 5);
+  for (int64_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < static_cast<int64_t>(spans) * h; s += warps) {
+    const int y = static_cast<int>(s / spans), x0 = static_cast<int>(s - static_cast<int64_t>(y) * spans) * kPeakSpan + lane;
+    if (y < b || y >= h - b) continue;
+    const float* row = j.img + static_cast<size_t>(y) * w;
+    float v[kPeakSpan / 32];
+#pragma unroll
+    for (int u = 0; u < kPeakSpan / 32; ++u) v[u] = x0 + 32 * u < w ? __ldg(row + x0 + 32 * u) : 0.0f;
+#pragma unroll
+    for (int u = 0; u < kPeakSpan / 32; ++u) {
+      const int x = x0 + 32 * u;
+      if (x < b || x >= w - b || !(v[u] > t)) continue;
+      bool peak = true;
+#pragma unroll
+      for (int dy = -1; dy <= 1; ++dy)
+#pragma unroll
+        for (int dx = -1; dx <= 1; ++dx)
+          if ((dx != 0 || dy != 0) && __ldg(row + static_cast<int64_t>(dy) * w + x + dx) > v[u]) peak = false;
+      if (!peak) continue;
+      const unsigned slot = atomicAdd(j.count + 1, 1u);
+      if (static_cast<int>(slot) < cap) j.peaks[slot] = y * w + x;
+    }
   }
 }
 
 // Stamp footprint of every 3x3 peak, one warp per peak: fully on the frame,
-// finite, unmasked and below saturation (src/detect.cpp:190-214).
-__global__ void k_footprint(int w, int h, const float* __restrict__ img, const uint8_t* __restrict__ mask,
-                            DetectParamsDev p, const unsigned* __restrict__ n_peaks, int cap,
-                            const int* __restrict__ peaks, unsigned* count, int* __restrict__ cand) {
+// finite, unmasked and below saturation (src/detect.cpp:190-214). Eight rows are
+// in flight at a time.
+__global__ void __launch_bounds__(256) k_footprint(int w, int h, DetectPair jobs, DetectParamsDev p, int cap) {
+  const DetectDev j = jobs.d[blockIdx.y];
   const int lane = threadIdx.x & 31;
   const int nwarp = static_cast<int>((gridDim.x * blockDim.x) >> 5);
-  const int np = min(static_cast<int>(*n_peaks), cap);
+  const int np = min(static_cast<int>(j.count[1]), cap);
   const int r = p.stamp_radius;
   for (int c = static_cast<int>((blockIdx.x * blockDim.x + threadIdx.x) >> 5); c < np; c += nwarp) {
-    const int i = peaks[c];
+    const int i = j.peaks[c];
     const int x = i % w, y = i / w;
     if (x - r < 0 || x + r >= w || y - r < 0 || y + r >= h) continue;
     bool ok = true;
-    for (int dy = -r; dy <= r && ok; ++dy) {
+    for (int dy = -r; dy <= r && ok; dy += 8) {
       for (int dx = lane - r; dx <= r; dx += 32) {
-        const size_t j = static_cast<size_t>(y + dy) * w + (x + dx);
-        const float v = img[j];
-        if (!isfinite(v) || (mask && mask[j] != 0) || (p.saturation > 0.0 && static_cast<double>(v) >= p.saturation))
-          ok = false;
+        float v[8];
+        uint8_t m[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+          const size_t at = static_cast<size_t>(y + min(dy + u, r)) * w + (x + dx);
+          v[u] = __ldg(j.img + at);
+          m[u] = j.mask ? __ldg(j.mask + at) : 0;
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+          if (!isfinite(v[u]) || m[u] != 0 || (p.saturation > 0.0 && static_cast<double>(v[u]) >= p.saturation)) ok = false;
       }
       ok = __all_sync(0xffffffffu, ok);
     }
     if (ok && lane == 0) {
-      const unsigned slot = atomicAdd(count, 1u);
-      if (static_cast<int>(slot) < cap) cand[slot] = i;
+      const unsigned slot = atomicAdd(j.count, 1u);
+      if (static_cast<int>(slot) < cap) j.cand[slot] = i;
     }
   }
 }
 
-// Sort keys: (flux descending, index ascending) -> ascending uint64.
+// (flux descending, index ascending) as an ascending uint64.
+__device__ __forceinline__ unsigned long long cand_key(float v, int idx) {
+  return (static_cast<unsigned long long>(~float_key(v)) << 32) | static_cast<unsigned>(idx);
+}
+
 __global__ void k_cand_keys(const unsigned* count, int cap, const int* __restrict__ cand, const float* __restrict__ img,
                             unsigned long long* __restrict__ keys, int* __restrict__ vals) {
   const int nc = min(static_cast<int>(*count), cap);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < nc; i += gridDim.x * blockDim.x) {
     const int idx = cand[i];
-    const uint32_t fk = ~float_key(img[idx]);  // descending value
-    keys[i] = (static_cast<unsigned long long>(fk) << 32) | static_cast<unsigned>(idx);
+    keys[i] = cand_key(img[idx], idx);
     vals[i] = idx;
   }
 }
 
-// Brightest-first greedy isolation (src/detect.cpp:223-240) in one CTA.
-// Output: kept raster indices in order; *n_kept.
-__global__ void __launch_bounds__(1024)
-k_isolate(int w, const unsigned* count, int cap, const int* __restrict__ sorted_idx, long long iso2, int max_stamps,
-          int* __restrict__ kept, int* n_kept, unsigned* status) {
-  extern __shared__ int ks[];  // kept x, y interleaved (2 * max_stamps)
-  __shared__ int s_nk;
-  __shared__ unsigned char pass[1024];
-  __shared__ int cx[1024], cy[1024];
-  const int nc = min(static_cast<int>(*count), cap);
-  if (threadIdx.x == 0) s_nk = 0;
+// Brightest-first greedy isolation (src/detect.cpp:223-240) by one CTA of 1024
+// threads, chunk by chunk of at most 1024 candidates in order, a thread to each.
+// The kept stamps, and the chunk's candidates that none of those excludes, hang
+// on lists hashed by cells of the isolation radius, so that a candidate looks at
+// nine cells only. In each round a candidate looks for a brighter neighbour that
+// is kept (it is out) or undecided (it waits there, and goes on from there when
+// that one is out); if none is left it is kept. The rounds follow the longest
+// chain of waiting candidates, 3 to 5 on star fields; the brightest undecided
+// candidate always decides, so 1024 bound them.
+constexpr int kIsoHeads = 1024;
+struct Isolation {
+  int4 node[1024];  // x, y, next
+  int head[kIsoHeads], khead[kIsoHeads];
+  unsigned char state[1024];
+  int wsum[32];
+};
+__device__ __forceinline__ int iso_bucket(int cx, int cy) {
+  return static_cast<int>((static_cast<unsigned>(cx) * 0x9E3779B1u ^ static_cast<unsigned>(cy) * 0x85EBCA6Bu) >> 22);
+}
+// Dynamic shared memory of the kept stamps: x, y and the next of each.
+__host__ __device__ constexpr size_t iso_smem(int max_stamps) {
+  return (2 * sizeof(int) + sizeof(uint16_t)) * static_cast<size_t>(max_stamps > 1 ? max_stamps : 1);
+}
+__device__ __forceinline__ bool iso_near(int dx, int dy, int r, long long r2) {
+  dx = abs(dx);
+  dy = abs(dy);
+  if (dx >= r || dy >= r) return false;
+  const long long lx = dx, ly = dy;
+  return lx * lx + ly * ly < r2;
+}
+
+// One chunk: thread t < n holds raster index idx. Returns the number kept so far.
+__device__ int isolate_chunk(Isolation& sh, int w, int n, int idx, int iso, int max_stamps, int nk, int* ks,
+                             int* __restrict__ kept) {
+  enum : unsigned char { kOut, kKept, kOpen };
+  volatile unsigned char* state = sh.state;
+  uint16_t* knext = reinterpret_cast<uint16_t*>(ks + 2 * (max_stamps > 1 ? max_stamps : 1));
+  constexpr int kEnd = 0xffff;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int r = abs(iso), cell = max(1, r);
+  const long long r2 = static_cast<long long>(r) * r;
+  const int x = idx % w, y = idx / w, cx = x / cell, cy = y / cell;
+  for (int i = tid; i < kIsoHeads; i += 1024) {
+    sh.head[i] = kEnd;
+    if (nk == 0) sh.khead[i] = kEnd;
+  }
   __syncthreads();
-  for (int base = 0; base < nc; base += blockDim.x) {
-    if (s_nk >= max_stamps) break;
-    const int i = base + threadIdx.x;
-    bool ok = false;
-    if (i < nc) {
-      const int idx = sorted_idx[i];
-      const int x = idx % w, y = idx / w;
-      cx[threadIdx.x] = x;
-      cy[threadIdx.x] = y;
-      ok = true;
-      const int nk = s_nk;
-      for (int k = 0; k < nk; ++k) {
-        const long long dx = x - ks[2 * k], dy = y - ks[2 * k + 1];
-        if (dx * dx + dy * dy < iso2) {
-          ok = false;
+  bool open = tid < n;
+  if (nk > 0)
+    for (int q = 0; q < 9 && open; ++q)
+      for (int k = sh.khead[iso_bucket(cx - 1 + q % 3, cy - 1 + q / 3)]; k != kEnd && open; k = knext[k])
+        open = !iso_near(x - ks[2 * k], y - ks[2 * k + 1], r, r2);
+  state[tid] = open ? kOpen : kOut;
+  if (open) sh.node[tid] = make_int4(x, y, atomicExch(&sh.head[iso_bucket(cx, cy)], tid), 0);
+  __syncthreads();
+  bool mine = false;
+  int q = 0, k = open ? sh.head[iso_bucket(cx - 1, cy - 1)] : kEnd;
+  do {
+    while (open) {
+      if (k == kEnd) {
+        if (++q == 9) {
+          mine = true;
+          open = false;
+          state[tid] = kKept;
+          break;
+        }
+        const int row = q >= 6 ? 2 : q >= 3 ? 1 : 0;
+        k = sh.head[iso_bucket(cx - 1 + q - 3 * row, cy - 1 + row)];
+        continue;
+      }
+      const int4 c = sh.node[k];
+      if (k < tid && iso_near(x - c.x, y - c.y, r, r2)) {
+        const unsigned char st = state[k];
+        if (st == kOpen) break;
+        if (st == kKept) {
+          open = false;
+          state[tid] = kOut;
           break;
         }
       }
+      k = c.z;
     }
-    pass[threadIdx.x] = ok ? 1 : 0;
-    __syncthreads();
-    // Sequential resolution within the chunk by warp 0.
-    if (threadIdx.x < 32) {
-      const int lim = min(static_cast<int>(blockDim.x), nc - base);
-      int nk = s_nk;
-      const int chunk_start = nk;
-      // The candidates that passed, in order, 32 flags per ballot.
-      for (int t0 = 0; t0 < lim && nk < max_stamps; t0 += 32) {
-        unsigned todo = __ballot_sync(0xffffffffu, t0 + static_cast<int>(threadIdx.x) < lim && pass[t0 + threadIdx.x]);
-        while (todo && nk < max_stamps) {
-          const int t = t0 + __ffs(todo) - 1;
-          todo &= todo - 1;
-          bool iso = true;
-          for (int k = chunk_start + threadIdx.x; k < nk; k += 32) {
-            const long long dx = cx[t] - ks[2 * k], dy = cy[t] - ks[2 * k + 1];
-            if (dx * dx + dy * dy < iso2) iso = false;
-          }
-          iso = __all_sync(0xffffffffu, iso);
-          if (iso) {
-            if (threadIdx.x == 0) {
-              ks[2 * nk] = cx[t];
-              ks[2 * nk + 1] = cy[t];
-              kept[nk] = cy[t] * w + cx[t];
-            }
-            __syncwarp();
-            ++nk;
-          }
-        }
-      }
-      if (threadIdx.x == 0) s_nk = nk;
-    }
-    __syncthreads();
+  } while (__syncthreads_or(open));
+  const unsigned vote = __ballot_sync(0xffffffffu, mine);
+  if (lane == 0) sh.wsum[warp] = __popc(vote);
+  __syncthreads();
+  const int c = sh.wsum[lane];
+  int at = nk + __popc(vote & ((1u << lane) - 1u)) + __reduce_add_sync(0xffffffffu, lane < warp ? c : 0);
+  if (mine && at < max_stamps) {
+    ks[2 * at] = x;
+    ks[2 * at + 1] = y;
+    kept[at] = idx;
+    knext[at] = static_cast<uint16_t>(atomicExch(&sh.khead[iso_bucket(cx, cy)], at));
   }
-  if (threadIdx.x == 0) *n_kept = s_nk;
-  (void)status;
+  nk = min(nk + __reduce_add_sync(0xffffffffu, c), max_stamps);
+  __syncthreads();
+  return nk;
+}
+
+// Ascending bitonic sort of 1024 keys, one per thread: exchanges within a warp by
+// shuffles, only the longer ones through shared memory. Returns the thread's key.
+__device__ unsigned long long sort_1024(unsigned long long k, unsigned long long* sk) {
+  const int tid = threadIdx.x;
+  for (int size = 2; size <= 1024; size <<= 1)
+    for (int half = size >> 1; half > 0; half >>= 1) {
+      unsigned long long other;
+      if (half >= 32) {
+        __syncthreads();
+        sk[tid] = k;
+        __syncthreads();
+        other = sk[tid ^ half];
+      } else {
+        other = __shfl_xor_sync(0xffffffffu, k, half);
+      }
+      const bool least = ((tid & size) == 0) == ((tid & half) == 0);
+      if (least == (other < k)) k = other;
+    }
+  return k;
+}
+
+// Sort and isolation of one image's candidates in one CTA, which holds up to
+// kSortMost keys. Only the chunks that isolation asks for are sorted: each time
+// the brightest keys left, 512 to 1024 of them, are found on a histogram of the
+// range that is left (and of the bin where it passes 1024, if there are fewer
+// than 512 below that), gathered and sorted. With max_stamps of a few hundred one
+// or two chunks do, however many candidates there are. More candidates set
+// count[3] (the host then takes the general path). Keys to global memory, a radix
+// sort and an isolation by single warps took 4 to 20 launches and 110 to 190 us
+// per image (2000 to 8400 candidates); this launch takes 40 us for both images
+// (770 and 1650 candidates at 1003x1531, 8400 at 4096x4096; 52 and 212 us when it
+// sorted all keys).
+constexpr int kSortMost = 16384;
+constexpr int kSortStamps = 4096;  // the most stamps whose places fit beside the keys
+
+__global__ void __launch_bounds__(1024) k_sort_isolate(int w, DetectPair jobs, int iso, int max_stamps) {
+  using u64 = unsigned long long;
+  extern __shared__ __align__(16) u64 keys[];
+  __shared__ Isolation sh;
+  __shared__ u64 chunk[1024];
+  __shared__ int hist[1024];
+  __shared__ u64 s_lo, s_hi;
+  __shared__ int s_sum[32], s_n, s_bin, s_below;
+  const DetectDev j = jobs.d[blockIdx.x];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nc = static_cast<int>(min(j.count[0], static_cast<unsigned>(kSortMost) + 1u));
+  if (nc > kSortMost) {
+    if (tid == 0) j.count[3] = 1u;
+    return;
+  }
+  if (tid == 0) {
+    s_lo = ~0ull;
+    s_hi = 0;
+  }
+  __syncthreads();
+  u64 lo = ~0ull, hi = 0;
+  for (int i = tid; i < nc; i += 1024) {
+    const int idx = j.cand[i];
+    const u64 k = cand_key(__ldg(j.img + idx), idx);
+    keys[i] = k;
+    lo = min(lo, k);
+    hi = max(hi, k);
+  }
+  for (int d = 16; d > 0; d >>= 1) {
+    lo = min(lo, __shfl_xor_sync(0xffffffffu, lo, d));
+    hi = max(hi, __shfl_xor_sync(0xffffffffu, hi, d));
+  }
+  if (lane == 0) {
+    atomicMin(&s_lo, lo);
+    atomicMax(&s_hi, hi);
+  }
+  __syncthreads();
+  lo = s_lo;
+  const u64 last = s_hi;  // keys in [lo, last] are left
+  int* ks = reinterpret_cast<int*>(keys + kSortMost);
+  int nk = 0;
+  for (int left = nc; left > 0 && nk < max_stamps;) {
+    // end: one past the chunk's greatest key. [lo, from) is in the chunk, n keys.
+    u64 end = last, from = lo, to = last;
+    int n = 0;
+    if (left > 1024) {
+      while (true) {
+        const int shift = max(0, 64 - __clzll(static_cast<long long>(to - from)) - 10);  // (to - from) >> shift < 1024
+        hist[tid] = 0;
+        __syncthreads();
+        for (int i = tid; i < nc; i += 1024) {
+          const u64 k = keys[i];
+          if (k >= from && k <= to) atomicAdd(&hist[(k - from) >> shift], 1);
+        }
+        __syncthreads();
+        int sum = hist[tid];
+        for (int d = 1; d < 32; d <<= 1) {
+          const int o = __shfl_up_sync(0xffffffffu, sum, d);
+          if (lane >= d) sum += o;
+        }
+        if (lane == 31) s_sum[warp] = sum;
+        __syncthreads();
+        sum += __reduce_add_sync(0xffffffffu, lane < warp ? s_sum[lane] : 0);
+        const int before = sum - hist[tid];
+        if (n + before <= 1024 && n + sum > 1024) {  // one bin: more than 1024 keys are left
+          s_bin = tid;
+          s_below = before;
+        }
+        __syncthreads();
+        n += s_below;
+        from += static_cast<u64>(s_bin) << shift;
+        to = min(to, from + (((1ull << shift) - 1)));
+        end = from - 1;
+        if (n >= 512) break;
+      }
+    } else {
+      n = left;
+    }
+    if (tid == 0) s_n = 0;
+    __syncthreads();
+    for (int i = tid; i < nc; i += 1024) {
+      const u64 k = keys[i];
+      if (k >= lo && k <= end) chunk[atomicAdd(&s_n, 1)] = k;
+    }
+    __syncthreads();
+    const u64 k = sort_1024(tid < n ? chunk[tid] : ~0ull, chunk);
+    nk = isolate_chunk(sh, w, n, tid < n ? static_cast<int>(k & 0xffffffffull) : 0, iso, max_stamps, nk, ks, j.kept);
+    lo = end + 1;
+    left -= n;
+  }
+  if (tid == 0) j.count[2] = static_cast<unsigned>(nk);
+}
+
+// Isolation of candidates sorted in global memory.
+__global__ void __launch_bounds__(1024)
+k_isolate(int w, DetectDev j, int cap, const int* __restrict__ sorted_idx, int iso, int max_stamps) {
+  extern __shared__ int ks[];
+  __shared__ Isolation sh;
+  const int nc = min(static_cast<int>(j.count[0]), cap);
+  int nk = 0;
+  for (int base = 0; base < nc && nk < max_stamps; base += 1024) {
+    const int n = min(nc - base, 1024);
+    const int idx = static_cast<int>(threadIdx.x) < n ? sorted_idx[base + threadIdx.x] : 0;
+    nk = isolate_chunk(sh, w, n, idx, iso, max_stamps, nk, ks, j.kept);
+  }
+  if (threadIdx.x == 0) j.count[2] = static_cast<unsigned>(nk);
 }
 
 // One CTA per kept stamp: the threads stage the clipped weights
 // max(f - bg, 0) of the FWHM window in shared memory (0 off the frame, which
 // adds an exact zero where the reference skips the pixel), then thread 0 runs
 // the two FP64 moment passes of fwhm_dev in the same (dy, dx) order.
-__global__ void __launch_bounds__(256) k_stamp_props(int w, int h, const float* __restrict__ img,
-                                                      const float* __restrict__ bg, const int* __restrict__ kept,
-                                                      const int* __restrict__ n_kept, int fwhm_radius,
-                                                      double* __restrict__ flux, double* __restrict__ snr,
-                                                      double* __restrict__ fwhm) {
+__global__ void __launch_bounds__(256) k_stamp_props(int w, int h, DetectPair jobs, int fwhm_radius, int max_stamps) {
   extern __shared__ double wt[];  // (2r+1)^2
+  const DetectDev j = jobs.d[blockIdx.y];
   const int i = blockIdx.x;
-  if (i >= *n_kept) return;
-  const double med = static_cast<double>(bg[0]);
-  const double sigma = 1.4826 * static_cast<double>(bg[1]);
-  const int idx = kept[i];
+  if (i >= static_cast<int>(j.count[2])) return;
+  const float* img = j.img;
+  double *flux = j.props, *snr = flux + max_stamps, *fwhm = snr + max_stamps;
+  const double med = static_cast<double>(j.bg[0]);
+  const double sigma = 1.4826 * static_cast<double>(j.bg[1]);
+  const int idx = j.kept[i];
   const int x = idx % w, y = idx / w;
   const int r = fwhm_radius, side = 2 * r + 1;
   for (int e = threadIdx.x; e < side * side; e += blockDim.x) {
@@ -487,161 +676,168 @@ void launch_weighted_mean(Context& c, int64_t n, const float* d, const float* v,
   out2[1] = b;
 }
 
-// The detect pipeline of one image in three phases, each ending in read-backs
-// that the caller's sync_reads completes: (1) background, 3x3 peaks and the
-// footprint test -> candidate counts; (2) brightest-first sort and greedy
-// isolation -> kept count; (3) the kept stamps' flux, S/N and FWHM. Two
-// images (their own workspace slots, `which` 0 and 1) can run phase by phase
-// so that they share each synchronisation.
+// The detect pipeline of up to two images of one size.
 struct DetectJob {
   const float* img;
   const uint8_t* mask;
-  int which;
   DetectHost* res;
-  float* bg;
-  unsigned* count;
-  int *cand, *sorted, *kept, *vals, *nk;
-  unsigned long long *keys, *keys2;
-  unsigned hc[2] = {0, 0};
+  unsigned hc[4] = {0, 0, 0, 0};
   float hbg[2] = {0.0f, 0.0f};
-  int nkept = 0;
   std::vector<int> hk;
+  std::vector<double> props;
 };
 constexpr int kDetectCap = 1 << 20;
 
-static void detect_phase1(Context& c, int w, int h, const DetectParamsDev& p, DetectJob& j) {
-  cudaStream_t s = c.stream;
-  const int64_t n = static_cast<int64_t>(w) * h;
-  const Slot ss = j.which ? kSlotFit12 : kSlotFit10, ks = j.which ? kSlotFit13 : kSlotFit11;
-  j.bg = static_cast<float*>(c.slot(j.which ? kSlotFit15 : kSlotFit14, 64));
-  launch_background(c, n, j.img, j.mask, j.bg, ss, ks);
-  const int cap = kDetectCap;
-  char* buf = static_cast<char*>(
-      c.slot(j.which ? kSlotFft1 : kSlotFft0, (sizeof(int) * 3 + 2 * sizeof(unsigned long long)) * cap + 256));
-  j.count = reinterpret_cast<unsigned*>(buf);
-  j.cand = reinterpret_cast<int*>(buf + 64);
-  j.sorted = j.cand + cap;
-  j.kept = j.sorted + cap;
-  j.keys = reinterpret_cast<unsigned long long*>(j.kept + cap);
-  j.keys2 = j.keys + cap;
-  j.vals = static_cast<int*>(c.slot(j.which ? kSlotFft3 : kSlotFft2, sizeof(int) * cap + 64));
-  j.nk = j.vals + cap;
-  unsigned* n_peaks = j.count + 1;  // 3x3 peaks before the footprint test; `sorted` holds them until the sort
-  DGPU_CUDA(cudaMemsetAsync(j.count, 0, 2 * sizeof(unsigned), s));
-  const int blocks = static_cast<int>(std::min<int64_t>((n + 255) / 256, 148 * 16));
-  k_peaks<<<blocks, 256, 0, s>>>(w, h, j.img, j.bg, p, n_peaks, cap, j.sorted);
-  DGPU_LAUNCH("k_peaks");
-  k_footprint<<<148 * 8, 256, 0, s>>>(w, h, j.img, j.mask, p, n_peaks, cap, j.sorted, j.count, j.cand);
-  DGPU_LAUNCH("k_footprint");
-  read_back(c, j.hc, j.count, 2 * sizeof(unsigned));
-  read_back(c, j.hbg, j.bg, sizeof(j.hbg));
-}
-
-// After phase 1's sync. Returns whether a read-back was queued.
-static bool detect_phase2(Context& c, int w, const DetectParamsDev& p, DetectJob& j) {
-  cudaStream_t s = c.stream;
-  const int cap = kDetectCap;
-  if (j.hc[1] > static_cast<unsigned>(cap)) fail(DGPU_ERR_RUNTIME, "detect_stamps: more than 2^20 peak candidates");
-  const int nc = static_cast<int>(j.hc[0]);
-  j.nkept = 0;
-  if (nc <= 0) return false;
-  k_cand_keys<<<(nc + 255) / 256, 256, 0, s>>>(j.count, cap, j.cand, j.img, j.keys, j.vals);
-  DGPU_LAUNCH("k_cand_keys");
-  size_t tmp_bytes = 0;
-  DGPU_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, j.keys, j.keys2, j.vals, j.sorted, nc, 0, 64, s));
-  void* tmp = c.slot(j.which ? kSlotFft5 : kSlotFft4, tmp_bytes + 16);
-  DGPU_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, j.keys, j.keys2, j.vals, j.sorted, nc, 0, 64, s));
-  const long long iso = p.isolation_radius;
-  const size_t smem = sizeof(int) * 2 * std::max(p.max_stamps, 1);
-  if (smem > 160 * 1024) fail(DGPU_ERR_INVALID, "detect_stamps: max_stamps above 20480 is not supported");
-  ensure_dynamic_smem(reinterpret_cast<const void*>(k_isolate), smem);
-  k_isolate<<<1, 1024, smem, s>>>(w, j.count, cap, j.sorted, iso * iso, p.max_stamps, j.kept, j.nk, c.d_status);
-  DGPU_LAUNCH("k_isolate");
-  read_back(c, &j.nkept, j.nk, sizeof(int));
-  return true;
-}
-
-// After phase 2's sync. Returns whether a read-back was queued.
-static bool detect_phase3(Context& c, int w, int h, const DetectParamsDev& p, DetectJob& j) {
-  cudaStream_t s = c.stream;
-  DetectHost& res = *j.res;
-  res.median = static_cast<double>(j.hbg[0]);
-  res.sigma = 1.4826 * static_cast<double>(j.hbg[1]);
-  const int nkept = j.nkept;
-  res.x.assign(nkept, 0);
-  res.y.assign(nkept, 0);
-  res.flux.assign(nkept, 0);
-  res.snr.assign(nkept, 0);
-  res.fwhm.assign(nkept, 0);
-  if (nkept <= 0) return false;
-  double* props =
-      static_cast<double*>(c.slot(j.which ? kSlotCompOut : kSlotCompStats, sizeof(double) * 3 * nkept));
+static void launch_stamp_props(cudaStream_t s, int w, int h, const DetectParamsDev& p, const DetectPair& jobs, int njobs,
+                               int nstamps, int stride) {
   const size_t psmem = sizeof(double) * static_cast<size_t>(2 * p.fwhm_radius + 1) * (2 * p.fwhm_radius + 1);
   if (psmem > 200 * 1024) fail(DGPU_ERR_INVALID, "detect_stamps: fwhm_radius too large");
   ensure_dynamic_smem(reinterpret_cast<const void*>(k_stamp_props), psmem);
-  k_stamp_props<<<nkept, 256, psmem, s>>>(w, h, j.img, j.bg, j.kept, j.nk, p.fwhm_radius, props, props + nkept,
-                                          props + 2 * nkept);
+  k_stamp_props<<<dim3(nstamps, njobs), 256, psmem, s>>>(w, h, jobs, p.fwhm_radius, stride);
   DGPU_LAUNCH("k_stamp_props");
-  j.hk.assign(nkept, 0);
-  read_back(c, j.hk.data(), j.kept, sizeof(int) * nkept);
-  read_back(c, res.flux.data(), props, sizeof(double) * nkept);
-  read_back(c, res.snr.data(), props + nkept, sizeof(double) * nkept);
-  read_back(c, res.fwhm.data(), props + 2 * nkept, sizeof(double) * nkept);
-  return true;
 }
 
-static void detect_finish(int w, DetectJob& j) {
-  for (int i = 0; i < j.nkept; ++i) {
-    j.res->x[i] = j.hk[i] % w;
-    j.res->y[i] = j.hk[i] / w;
+// The general path of one image, for more candidates than one CTA sorts or more
+// stamps than it keeps in shared memory beside them: radix sort, isolation and
+// measurement, reading the kept count back in between. On entry j.hc[0] > 0.
+static void detect_general(Context& c, int w, int h, const DetectParamsDev& p, DetectJob& j, const DetectDev& d) {
+  cudaStream_t s = c.stream;
+  const int cap = kDetectCap, nc = static_cast<int>(j.hc[0]);
+  char* buf = static_cast<char*>(c.slot(kSlotFft2, (sizeof(int) * 2 + 2 * sizeof(unsigned long long)) * cap));
+  auto* keys = reinterpret_cast<unsigned long long*>(buf);
+  auto* keys2 = keys + cap;
+  int* vals = reinterpret_cast<int*>(keys2 + cap);
+  int* sorted = vals + cap;
+  k_cand_keys<<<(nc + 255) / 256, 256, 0, s>>>(d.count, cap, d.cand, d.img, keys, vals);
+  DGPU_LAUNCH("k_cand_keys");
+  size_t tmp_bytes = 0;
+  DGPU_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys2, vals, sorted, nc, 0, 64, s));
+  void* tmp = c.slot(kSlotFft4, tmp_bytes + 16);
+  DGPU_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, keys2, vals, sorted, nc, 0, 64, s));
+  const size_t smem = iso_smem(p.max_stamps);
+  if (sizeof(int) * 2 * std::max(p.max_stamps, 1) > 160 * 1024) fail(DGPU_ERR_INVALID, "detect_stamps: max_stamps above 20480 is not supported");
+  ensure_dynamic_smem(reinterpret_cast<const void*>(k_isolate), smem);
+  k_isolate<<<1, 1024, smem, s>>>(w, d, cap, sorted, p.isolation_radius, p.max_stamps);
+  DGPU_LAUNCH("k_isolate");
+  read_back(c, j.hc, d.count, sizeof(j.hc));
+  sync_reads(c);
+  const int nk = static_cast<int>(j.hc[2]);
+  if (nk <= 0) return;
+  DetectPair one{};
+  one.d[0] = d;
+  one.d[0].props = static_cast<double*>(c.slot(kSlotCompOut, sizeof(double) * 3 * nk));
+  launch_stamp_props(s, w, h, p, one, 1, nk, nk);
+  j.hk.resize(nk);
+  j.props.resize(3 * static_cast<size_t>(nk));
+  read_back(c, j.hk.data(), d.kept, sizeof(int) * nk);
+  read_back(c, j.props.data(), one.d[0].props, sizeof(double) * 3 * nk);
+  sync_reads(c);
+}
+
+static void run_detect_jobs(Context& c, int w, int h, const DetectParamsDev& p, DetectJob* j, int njobs) {
+  cudaStream_t s = c.stream;
+  const int64_t n = static_cast<int64_t>(w) * h;
+  const int cap = kDetectCap, most = std::max(p.max_stamps, 0);
+  // In one CTA's shared memory: the sort keys and the kept stamps.
+  const size_t sort_smem = sizeof(unsigned long long) * kSortMost + iso_smem(most);
+  const size_t psmem = sizeof(double) * static_cast<size_t>(2 * p.fwhm_radius + 1) * (2 * p.fwhm_radius + 1);
+  const bool fast = most <= kSortStamps && psmem <= 200 * 1024;
+  const size_t kept_ints = (static_cast<size_t>(std::max(most, 1)) + 1) & ~size_t(1);
+  const size_t per = 64 + sizeof(int) * (2 * static_cast<size_t>(cap) + kept_ints) + sizeof(double) * 3 * std::max(most, 1);
+  char* buf = static_cast<char*>(c.slot(kSlotFft0, per * njobs));
+  DetectPair jobs{};
+  MedianJob med[kMedianJobs];
+  for (int i = 0; i < njobs; ++i) {
+    DetectDev& d = jobs.d[i];
+    char* b = buf + per * i;
+    d.img = j[i].img;
+    d.mask = j[i].mask;
+    d.count = reinterpret_cast<unsigned*>(b);
+    float* bg = reinterpret_cast<float*>(b + 32);
+    d.bg = bg;
+    d.peaks = reinterpret_cast<int*>(b + 64);
+    d.cand = d.peaks + cap;
+    d.kept = d.cand + cap;
+    d.props = reinterpret_cast<double*>(d.kept + kept_ints);
+    med[i] = background_job(n, d.img, d.mask, bg);
+    med[i].clear = d.count;
+    med[i].nclear = 4;
+  }
+  launch_medians(s, med, njobs, c.slot(kSlotSamples, medians_scratch(med, njobs)));
+  const int64_t spans = static_cast<int64_t>((w + kPeakSpan - 1) / kPeakSpan) * h;
+  k_peaks<<<dim3(static_cast<unsigned>(std::min<int64_t>((spans + 7) / 8, 148 * 8)), njobs), 256, 0, s>>>(w, h, jobs, p, cap);
+  DGPU_LAUNCH("k_peaks");
+  k_footprint<<<dim3(148 * 4, njobs), 256, 0, s>>>(w, h, jobs, p, cap);
+  DGPU_LAUNCH("k_footprint");
+  if (fast) {
+      ensure_dynamic_smem(reinterpret_cast<const void*>(k_sort_isolate), sort_smem);
+    k_sort_isolate<<<njobs, 1024, sort_smem, s>>>(w, jobs, p.isolation_radius, p.max_stamps);
+    DGPU_LAUNCH("k_sort_isolate");
+    if (most > 0) launch_stamp_props(s, w, h, p, jobs, njobs, most, most);
+  }
+  for (int i = 0; i < njobs; ++i) {
+    read_back(c, j[i].hc, jobs.d[i].count, sizeof(j[i].hc));
+    read_back(c, j[i].hbg, jobs.d[i].bg, sizeof(j[i].hbg));
+    if (fast && most > 0) {
+      j[i].hk.resize(most);
+      j[i].props.resize(3 * static_cast<size_t>(most));
+      read_back(c, j[i].hk.data(), jobs.d[i].kept, sizeof(int) * most);
+      read_back(c, j[i].props.data(), jobs.d[i].props, sizeof(double) * 3 * most);
+    }
+  }
+  sync_reads(c);
+  for (int i = 0; i < njobs; ++i) {
+    if (j[i].hc[1] > static_cast<unsigned>(cap)) fail(DGPU_ERR_RUNTIME, "detect_stamps: more than 2^20 peak candidates");
+    int stride = most;
+    if (j[i].hc[0] > 0 && (!fast || j[i].hc[3] != 0)) {
+      detect_general(c, w, h, p, j[i], jobs.d[i]);
+      stride = static_cast<int>(j[i].hc[2]);
+    }
+    DetectHost& res = *j[i].res;
+    res.median = static_cast<double>(j[i].hbg[0]);
+    res.sigma = 1.4826 * static_cast<double>(j[i].hbg[1]);
+    const int nk = static_cast<int>(j[i].hc[2]);
+    res.x.resize(nk);
+    res.y.resize(nk);
+    res.flux.resize(nk);
+    res.snr.resize(nk);
+    res.fwhm.resize(nk);
+    for (int q = 0; q < nk; ++q) {
+      res.x[q] = j[i].hk[q] % w;
+      res.y[q] = j[i].hk[q] / w;
+      res.flux[q] = j[i].props[q];
+      res.snr[q] = j[i].props[static_cast<size_t>(stride) + q];
+      res.fwhm[q] = j[i].props[2 * static_cast<size_t>(stride) + q];
+    }
   }
 }
 
-// Full detect pipeline for one image. Returns the kept count; host copies of
-// x, y, flux, snr, fwhm in `res`.
-int run_detect(Context& c, int w, int h, const float* img, const uint8_t* mask, const DetectParamsDev& p, int which,
+int run_detect(Context& c, int w, int h, const float* img, const uint8_t* mask, const DetectParamsDev& p,
                DetectHost& res) {
   DetectJob j;
   j.img = img;
   j.mask = mask;
-  j.which = which;
   j.res = &res;
-  detect_phase1(c, w, h, p, j);
-  sync_reads(c);
-  if (detect_phase2(c, w, p, j)) sync_reads(c);
-  if (detect_phase3(c, w, h, p, j)) sync_reads(c);
-  detect_finish(w, j);
-  return j.nkept;
+  run_detect_jobs(c, w, h, p, &j, 1);
+  return static_cast<int>(res.x.size());
 }
 
-// Both images of a pair, phase by phase: three synchronisations, not six.
 void run_detect_pair(Context& c, int w, int h, const float* img0, const uint8_t* mask0, const float* img1,
                      const uint8_t* mask1, const DetectParamsDev& p, DetectHost& res0, DetectHost& res1) {
   DetectJob j[2];
   j[0].img = img0;
   j[0].mask = mask0;
-  j[0].which = 0;
   j[0].res = &res0;
   j[1].img = img1;
   j[1].mask = mask1;
-  j[1].which = 1;
   j[1].res = &res1;
-  detect_phase1(c, w, h, p, j[0]);
-  detect_phase1(c, w, h, p, j[1]);
-  sync_reads(c);
-  bool q = detect_phase2(c, w, p, j[0]);
-  q = detect_phase2(c, w, p, j[1]) || q;
-  if (q) sync_reads(c);
-  q = detect_phase3(c, w, h, p, j[0]);
-  q = detect_phase3(c, w, h, p, j[1]) || q;
-  if (q) sync_reads(c);
-  detect_finish(w, j[0]);
-  detect_finish(w, j[1]);
+  run_detect_jobs(c, w, h, p, j, 2);
 }
 
 void run_background(Context& c, int64_t n, const float* img, const uint8_t* mask, double* median, double* sigma) {
   float* bg = static_cast<float*>(c.slot(kSlotFit14, 64));
-  launch_background(c, n, img, mask, bg, kSlotFit10, kSlotFit11);
+  const MedianJob job = background_job(n, img, mask, bg);
+  launch_medians(c.stream, &job, 1, c.slot(kSlotSamples, medians_scratch(&job, 1)));
   float hbg[2];
   read_back(c, hbg, bg, sizeof(hbg));
   sync_reads(c);
@@ -656,9 +852,9 @@ void run_catalog_stamps(Context& c, int w, int h, const float* sci, const uint8_
   cudaStream_t s = c.stream;
   const int64_t npx = static_cast<int64_t>(w) * h;
   float* bgs = static_cast<float*>(c.slot(kSlotFit14, 64));
-  float* bgr = static_cast<float*>(c.slot(kSlotFit15, 64));
-  launch_background(c, npx, sci, sm, bgs, kSlotFit10, kSlotFit11);
-  launch_background(c, npx, ref, rm, bgr, kSlotFit12, kSlotFit13);
+  float* bgr = bgs + 2;
+  const MedianJob jobs[2] = {background_job(npx, sci, sm, bgs), background_job(npx, ref, rm, bgr)};
+  launch_medians(s, jobs, 2, c.slot(kSlotSamples, medians_scratch(jobs, 2)));
   int* dxy = static_cast<int*>(c.slot(kSlotBright, sizeof(int) * 2 * std::max(n, 1)));
   DGPU_CUDA(h2d_async(dxy, xs_host, sizeof(int) * n, s));
   DGPU_CUDA(h2d_async(dxy + n, ys_host, sizeof(int) * n, s));
@@ -689,59 +885,31 @@ void run_catalog_stamps(Context& c, int w, int h, const float* sci, const uint8_
 }
 
 // ---------------------------------------------------------------------------
-// Allocation-free background estimate (dgpu_estimate_background_noalloc).
-//
-// Same algorithm and kernels as launch_background, with the sample keys and
-// the radix-select state in one fixed, file-scope device array instead of the
-// context's workspace. The sample has at most 2^19 entries for any frame below
-// 2^31 pixels (step = n / 2^18 gives ceil(n / step) < 2^19), so the array is
-// 2 MiB + 1 KiB per device. Each call clears the select state (its counter
-// must start at zero) on the caller's stream before use. The array is shared
-// by every call on a device: calls that overlap in time (other streams or
-// threads) race on it and must be serialised by the caller.
+// Allocation-free background estimate (dgpu_estimate_background_noalloc): the
+// launches of run_background, with the sample keys (at most 2^19 for any frame
+// below 2^31 pixels: step = n / 2^18) and the two results in one fixed, file-scope
+// device array instead of the context's workspace. The array is shared by every
+// call on a device: calls that overlap in time (other streams or threads) race
+// on it and must be serialised by the caller.
 // ---------------------------------------------------------------------------
-namespace {
-
-constexpr int64_t kNoAllocMaxSamples = int64_t(1) << 19;
-
 struct NoAllocBackground {
-  RadixSelect sel;          // count / rank / prefix / histogram: cleared by every call
   float result[4];  // [0] median, [1] MAD
-  uint32_t keys[kNoAllocMaxSamples];
+  uint32_t keys[kMedianMax];
 };
-
 static __device__ __align__(256) NoAllocBackground g_noalloc_background;
 
-// Device address of the array on the current device. Resolved on every call
-// (a cheap lookup, no allocation) rather than cached: after a device reset the
-// runtime reloads the module and the array may sit at a new address.
-NoAllocBackground* noalloc_background_scratch() {
+void background_noalloc(int64_t n, const float* img, const uint8_t* mask, cudaStream_t s, float* out2) {
+  // Resolved on every call (a cheap lookup, no allocation) rather than cached:
+  // after a device reset the runtime reloads the module and the array may sit at
+  // a new address.
   void* p = nullptr;
   const cudaError_t e = cudaGetSymbolAddress(&p, g_noalloc_background);
   if (e != cudaSuccess)
     fail(DGPU_ERR_CUDA, std::string("estimate_background_noalloc: cudaGetSymbolAddress: ") + cudaGetErrorString(e));
-  return static_cast<NoAllocBackground*>(p);
-}
-
-}  // namespace
-
-void background_noalloc(int64_t n, const float* img, const uint8_t* mask, cudaStream_t s, float* out2) {
-  constexpr int64_t kTarget = 1 << 18;
-  const int64_t step = n > kTarget ? n / kTarget : 1;
-  const int64_t ns = (n + step - 1) / step;
-  if (ns > kNoAllocMaxSamples)
-    fail(DGPU_ERR_INVALID, "estimate_background_noalloc: sample exceeds the fixed 2^19-entry scratch");
-  NoAllocBackground* sc = noalloc_background_scratch();
-  RadixSelect* st = &sc->sel;
-  uint32_t* keys = sc->keys;
-  float* res = sc->result;
-  DGPU_CUDA(cudaMemsetAsync(st, 0, sizeof(RadixSelect), s));
-  const int blocks = static_cast<int>(std::min<int64_t>((ns + 255) / 256, 148 * 8));
-  launch_sample_keys(s, n, step, img, mask, keys, st);
-  select_median(s, st, keys, ns, res);
-  k_abs_dev<<<std::max(blocks, 1), 256, 0, s>>>(st, res, keys);
-  DGPU_LAUNCH("k_abs_dev");
-  select_median(s, st, keys, ns, res + 1);
+  auto* sc = static_cast<NoAllocBackground*>(p);
+  const float* res = sc->result;
+  const MedianJob job = background_job(n, img, mask, sc->result);
+  launch_medians(s, &job, 1, sc->keys);
   DGPU_CUDA(cudaMemcpyAsync(out2, res, 2 * sizeof(float), cudaMemcpyDeviceToHost, s));
   DGPU_CUDA(cudaStreamSynchronize(s));
 }

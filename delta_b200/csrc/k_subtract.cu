@@ -730,25 +730,13 @@ void launch_mask_fill(cudaStream_t s, int64_t n, const uint8_t* mask, const uint
   DGPU_LAUNCH("k_mask_fill");
 }
 
-// ---------------------------------------------------------------------------
-// Upper median of a stride-7 sample by exact radix select (8 bits per pass over
-// the monotone uint32 key). Matches std::nth_element(size/2) on the sample
-// (src/subtract.cpp:20-51 for the reference fill, 915-945 for the difference
-// fill). An empty sample yields 0.
-// ---------------------------------------------------------------------------
-
+// Upper median of a stride-7 sample (std::nth_element(size / 2); an empty sample
+// yields 0): the good finite reference pixels (src/subtract.cpp:20-51), or the
+// unmasked finite difference pixels under the grown mask (915-945).
 void launch_strided_median(Context& c, int kind, int64_t n, const float* values, const uint8_t* mask,
                            float* d_result) {
-  // kind 0 (reference): good finite reference pixels; kind 1 (difference):
-  // unmasked finite difference pixels (mask is the grown output mask).
   (void)kind;
-  cudaStream_t s = c.stream;
-  const int64_t nsamp = (n + 6) / 7;
-  auto* st = static_cast<RadixSelect*>(c.slot(kSlotSelect, sizeof(RadixSelect)));
-  auto* keys = static_cast<uint32_t*>(c.slot(kSlotSamples, sizeof(uint32_t) * std::max<int64_t>(nsamp, 1)));
-  DGPU_CUDA(cudaMemsetAsync(st, 0, sizeof(RadixSelect), s));
-  launch_sample_keys(s, n, 7, values, mask, keys, st);
-  launch_select_upper_median(s, st, keys, nsamp, d_result);
+  launch_upper_median(c, n, 7, values, mask, d_result);
 }
 
 // photometric_scale (src/fit.cpp:513-530): out = sum_c float(S_c) * a_c in

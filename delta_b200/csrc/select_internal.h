@@ -1,7 +1,6 @@
-// Exact sample medians on the device by radix select: the sample is compacted
-// into monotone uint32 keys (float_key), then four 8-bit histogram passes find
-// the element of rank count / 2 -- the value std::nth_element(count / 2)
-// returns. Shared by the subtraction's fill values (src/subtract.cpp:20-51,
+// Exact sample medians on the device by radix select over monotone uint32 keys
+// (float_key): the element of rank count / 2, the value std::nth_element(count
+// / 2) returns. Shared by the subtraction's fill values (src/subtract.cpp:20-51,
 // 915-945) and stamp selection's background and MAD (src/detect.cpp:100-112).
 #pragma once
 
@@ -9,24 +8,32 @@
 
 #include <cstdint>
 
+#include "internal.h"
+
 namespace dgpu {
 
-struct RadixSelect {
-  unsigned count;   // keys in the sample
-  unsigned rank;    // remaining rank within the current prefix bucket
-  unsigned prefix;  // key bits fixed so far
-  unsigned arrived;  // blocks done with the current histogram pass
-  unsigned hist[256];
+// One sample: the finite values v[j * step] whose mask byte is 0 (any value when
+// mask is null).
+struct MedianJob {
+  const float* v = nullptr;
+  const uint8_t* mask = nullptr;
+  int64_t n = 0, step = 1;
+  float* out = nullptr;       // [0] the upper median (0 for an empty sample)
+  int mad = 0;                // 1: out[1] = the upper median of |value - out[0]|
+  unsigned* clear = nullptr;  // counters to zero on the way (see nclear)
+  int nclear = 0;
 };
 
-// Appends the keys of the finite values v[j * step] whose mask byte is 0 (any
-// value when mask is null) to keys, counting them in st->count, which the
-// caller has zeroed. keys must hold ceil(n / step) entries.
-void launch_sample_keys(cudaStream_t s, int64_t n, int64_t step, const float* v, const uint8_t* mask, uint32_t* keys,
-                        RadixSelect* st);
+// Samples of one launch: up to two (the two images of a pair).
+constexpr int kMedianJobs = 2;
+// Largest sample launch_medians takes.
+constexpr int64_t kMedianMax = int64_t(1) << 19;
 
-// *out = the key of rank st->count / 2 among keys[0 .. st->count) as a float
-// (0 for an empty sample); cap bounds st->count. Leaves st->count as it was.
-void launch_select_upper_median(cudaStream_t s, RadixSelect* st, const uint32_t* keys, int64_t cap, float* out);
+// scratch: medians_scratch bytes of device memory.
+size_t medians_scratch(const MedianJob* jobs, int njobs);
+void launch_medians(cudaStream_t s, const MedianJob* jobs, int njobs, void* scratch);
+
+// *out = the upper median of a sample of any size.
+void launch_upper_median(Context& c, int64_t n, int64_t step, const float* v, const uint8_t* mask, float* out);
 
 }  // namespace dgpu

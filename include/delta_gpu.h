@@ -355,9 +355,8 @@ typedef struct {
  * context: it runs on the calling thread's current device, on `stream`
  * (NULL = legacy default stream), with `data` (float32, width x height) and the
  * optional `mask` (uint8) in device memory, and returns after synchronising
- * `stream`. Its scratch is one fixed array of 2 MiB + 1 KiB per device inside
- * the library (it holds the at most 2^19 sample keys of any frame below 2^31
- * pixels); the select state in it is cleared at the start of every call.
+ * `stream`. Its scratch is one fixed array of 2 MiB + 256 bytes per device inside
+ * the library (the at most 2^19 sample keys of any frame below 2^31 pixels).
  * Limits: frames up to 2^31 - 1 pixels (larger -> DGPU_ERR_INVALID). Every
  * call looks up that array's address on the current device
  * (cudaGetSymbolAddress, which allocates nothing); the first call on a device
