@@ -161,9 +161,15 @@ int dgpu_decorrelate(dgpu_context* ctx, int mem, int64_t width, int64_t height, 
     double* vbuf = static_cast<double*>(c.slot(kSlotFft1, sizeof(double) * (ncell + 2 * static_cast<size_t>(nblk) + 4)));
     double* cell_sumk2 = vbuf;
     double* vsr = vbuf + ncell;
-    float2* spec = static_cast<float2*>(
-        c.slot(kSlotFft0, sizeof(float2) * static_cast<size_t>(std::max(nblk, ncell)) * n * nb));
-    {
+    const bool power_fused = cell_power_fused(g, b.ks, t.k, nc);
+    float2* spec = nullptr;  // of the unfused passes
+    if (!power_fused || !block_filter_fused(g))
+      spec = static_cast<float2*>(
+          c.slot(kSlotFft0, sizeof(float2) * static_cast<size_t>(std::max(nblk, ncell)) * n * nb));
+    if (power_fused) {
+      StageTimer tm(c, "decorrelate: kernel-power cache");
+      launch_cell_power(s, g, ncell, t, d_theta, nc, d_phi, b.ks, d_cen, cell_sumk2, cell_power);
+    } else {
       StageTimer tm(c, "decorrelate: kernel-power cache");
       float* dense = static_cast<float*>(c.slot(kSlotFft3, sizeof(float) * static_cast<size_t>(ncell) * n * n));
       DGPU_CUDA(cudaMemsetAsync(dense, 0, sizeof(float) * static_cast<size_t>(ncell) * n * n, s));

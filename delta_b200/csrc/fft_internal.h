@@ -30,6 +30,11 @@ void launch_rows_inv(cudaStream_t s, const FftGeom& g, int mode, int nitems, con
 // The three passes of mode 0 (r2c rows, filtered columns, raw c2r rows into
 // dense_out) fused per block in one cluster launch; needs n = 256 and tw_tab.
 bool block_filter_fused(const FftGeom& g);
+// |Khat|^2 of every cell in one launch (else launch_local_kernels, launch_rows_fwd and
+// launch_cols): 128 and 256 point blocks with a twiddle table.
+bool cell_power_fused(const FftGeom& g, int ks, int knots, int nc);
+void launch_cell_power(cudaStream_t s, const FftGeom& g, int ncell, const TpsDev& t, const double* theta, int nc,
+                       const float* phi, int ks, const double* centres, double* sumk2, double* power);
 void launch_block_filter(cudaStream_t s, const FftGeom& g, int nitems, const float* src, int w, int h,
                          const int* oxs, const int* oys, int nox, const double* cell_power, const double* cell_sumk2,
                          const int* block_cell, const double* vsr, double* bnum, float* dense_out);

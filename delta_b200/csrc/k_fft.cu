@@ -116,7 +116,9 @@ __device__ void smem_fft(float2* x, int L, int m, int logm, const float2* tw, in
 // multiplies by W_N^(n2 k1) and writes a padded k1-major layout; pass B does the
 // N2-point DFT in registers and writes natural order. Two shared-memory round
 // trips per line instead of log2(N) + 1. tw[k] = W_N^k for k < N/2 (the sign
-// of W selects forward or inverse); lines need ls >= N + 17; 256 threads.
+// of W selects forward or inverse); lines need ls >= N + 17. A line stays with one
+// warp throughout (2 lines of 256 or 4 of 128 at a time), so the passes need no
+// barrier of the CTA.
 // ---------------------------------------------------------------------------
 __host__ __device__ constexpr int bitrev_c(int i, int bits) {
   int r = 0;
@@ -172,17 +174,22 @@ __device__ __forceinline__ void reg_fft(float2 (&v)[M]) {
   }
 }
 
+// Lines of one warp at a time, and their transform: lines x .. x + (L - 1) ls, L <=
+// kWarpLines<N>.
+template <int N>
+constexpr int kWarpLines = N == 256 ? 2 : 4;
+
 template <int N, int SIGN>
-__device__ void fft_lines_4step_d(float2* x, int L, int ls, const float2* tw) {
+__device__ __forceinline__ void fft_warp(float2* x, int L, int ls, const float2* tw) {
   constexpr int N1 = 16, N2 = N / 16;
   constexpr int LOGN2 = N == 256 ? 4 : 3;
-  constexpr int kLinesA = 256 / N2, kLinesB = 256 / N1;
-  for (int l0 = 0; l0 < L; l0 += kLinesA) {
-    const int line = l0 + threadIdx.x / N2, n2 = threadIdx.x % N2;
+  const int lane = threadIdx.x & 31;
+  {
+    const int line = lane / N2, n2 = lane % N2;
     const bool act = line < L;
+    float2* xl = x + line * ls;
     float2 v[N1];
     if (act) {
-      float2* xl = x + line * ls;
 #pragma unroll
       for (int n1 = 0; n1 < N1; ++n1) v[n1] = xl[N2 * n1 + n2];
       reg_fft<N1, 4, SIGN>(v);
@@ -194,32 +201,39 @@ __device__ void fft_lines_4step_d(float2* x, int L, int ls, const float2* tw) {
         v[k1] = cmul(v[k1], w);
       }
     }
-    __syncthreads();
+    __syncwarp();
     if (act) {
-      float2* xl = x + line * ls;
 #pragma unroll
       for (int k1 = 0; k1 < N1; ++k1) xl[k1 * (N2 + 1) + n2] = v[k1];
     }
-    __syncthreads();
+    __syncwarp();
   }
-  for (int l0 = 0; l0 < L; l0 += kLinesB) {
-    const int line = l0 + threadIdx.x / N1, k1 = threadIdx.x % N1;
+#pragma unroll
+  for (int l0 = 0; l0 < kWarpLines<N>; l0 += 2) {
+    const int line = l0 + lane / N1, k1 = lane % N1;
     const bool act = line < L;
+    float2* xl = x + line * ls;
     float2 u[N2];
     if (act) {
-      const float2* xl = x + line * ls;
 #pragma unroll
       for (int n2 = 0; n2 < N2; ++n2) u[n2] = xl[k1 * (N2 + 1) + n2];
       reg_fft<N2, LOGN2, SIGN>(u);
     }
-    __syncthreads();
+    __syncwarp();
     if (act) {
-      float2* xl = x + line * ls;
 #pragma unroll
       for (int k2 = 0; k2 < N2; ++k2) xl[k1 + N1 * k2] = u[k2];
     }
-    __syncthreads();
   }
+  __syncwarp();
+}
+
+template <int N, int SIGN>
+__device__ void fft_lines_4step_d(float2* x, int L, int ls, const float2* tw) {
+  constexpr int W = kWarpLines<N>;
+  for (int l0 = (threadIdx.x >> 5) * W; l0 < L; l0 += (blockDim.x >> 5) * W)
+    fft_warp<N, SIGN>(x + l0 * ls, min(W, L - l0), ls, tw);
+  __syncthreads();
 }
 
 // Line stride for an FFT of length m: room for the four-step layout where it
@@ -474,12 +488,17 @@ k_rows_inv(FftGeom G, int mode, const float2* __restrict__ spec, const int* __re
 // (item x n x n) for the overlap-add gather. The row and column arithmetic is
 // that of k_rows_fwd / k_cols / k_rows_inv except for the packed DC / Nyquist
 // pair (the same transforms to FP32 rounding); the spectrum never leaves the
-// chip.
+// chip. It is bound by latency (shared memory, remote and own), at 16 warps an SM:
+// a warp takes four rows or four column lines through a pass by itself, so that the
+// CTA's barriers stand only around the filter, and moves its four rows' bins as 32
+// contiguous bytes a column: 355 us at 465 blocks, where batches of 16 rows with
+// barriers between their steps and eight bytes a column took 582 us.
 // ---------------------------------------------------------------------------
 constexpr int kBfRanks = 4;
 constexpr int kBfN = 256;
-constexpr int kBfBatch = 16;  // rows per row-pass batch
+constexpr int kBfRows = 4;    // rows a warp takes at a time
 constexpr int kBfCols = 32;   // column lines per rank
+constexpr int kBfZl = 152;    // row line stride: 8 mod 16, two lines on distinct banks
 
 // Bins 1..127 of every row live in line k % 32 of rank k / 32. The DC (k = 0)
 // and Nyquist (k = 128) bins of a real row are real, so their two columns share
@@ -495,13 +514,14 @@ k_block_filter(FftGeom G, const float* __restrict__ src, int w, int h, const int
                const double* __restrict__ vsr, double* __restrict__ bnum, float* __restrict__ dense_out) {
   extern __shared__ __align__(16) float2 fsm2[];
   constexpr int n = kBfN, hn = n / 2, nb = hn + 1;
-  const int ls = fft_ls(n, true), zl = fft_ls(hn, false);
+  constexpr int ls = kBfN + 17, zl = kBfZl;
   cg::cluster_group cl = cg::this_cluster();
   const int rank = static_cast<int>(cl.block_rank());
   const int item = blockIdx.x / kBfRanks;
-  float2* x = fsm2;                      // kBfCols x ls column lines
-  float2* z = x + kBfCols * ls;          // kBfBatch x zl row lines
-  float2* tw = z + kBfBatch * zl;        // the whole twiddle table
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  float2* x = fsm2;                                           // kBfCols x ls column lines
+  float2* z = x + kBfCols * ls + warp * (kBfRows * zl);       // this warp's kBfRows x zl row lines
+  float2* tw = x + kBfCols * ls + (256 / 32) * kBfRows * zl;  // the whole twiddle table
   copy_tw(tw, G.tw_tab, n + n / 2 + 2 * nb);
   const float2* tw_fwd_n = tw;
   const float2* tw_inv_n = tw + n / 2;
@@ -515,42 +535,36 @@ k_block_filter(FftGeom G, const float* __restrict__ src, int w, int h, const int
     return cl.map_shared_rank(x + (k - bf_cb(q)) * ls + row, q);
   };
   const int bx = oxs[item % nox], by = oys[item / nox];
-  const int ncol = kBfCols;
-  const int rbeg = rank * (n / kBfRanks), rend = rbeg + n / kBfRanks;
+  const int rbeg = rank * (n / kBfRanks) + warp * kBfRows, rend = (rank + 1) * (n / kBfRanks);
+  constexpr int kRowStep = (256 / 32) * kBfRows;
   cl.sync();  // every rank has started before its shared memory is written
 
-  // Row pass (r2c), scattered to the column owners. 256 threads: each loop
-  // below has a fixed trip count, so its loads are all in flight together.
-  const int tid = threadIdx.x;
-  // The next batch's samples are loaded while this batch transforms.
-  constexpr int kPer = kBfBatch * hn / 256;
+  // Row pass (r2c), scattered to the column owners, a warp's four rows at a time.
+  // The next four rows' samples are loaded while these transform.
+  constexpr int kPer = kBfRows * hn / 32;
+  const int rr = lane & 3, kl = lane >> 2;  // bins: 4 rows x 8 columns a warp
   float2 v[kPer];
-  auto load_batch = [&](int b) {
+  auto load_rows = [&](int b) {
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-      const int e = tid + 256 * i, rr = e / hn, j = e - rr * hn;
-      const int sy = reflect_clamp(by + b + rr, h);
-      const float* srow = src + static_cast<size_t>(sy) * w;
+      const int j = lane + 32 * (i & 3);
+      const float* srow = src + static_cast<size_t>(reflect_clamp(by + b + (i >> 2), h)) * w;
       v[i] = make_float2(__ldg(srow + reflect_clamp(bx + 2 * j, w)), __ldg(srow + reflect_clamp(bx + 2 * j + 1, w)));
     }
   };
-  load_batch(rbeg);
-  for (int b0 = rbeg; b0 < rend; b0 += kBfBatch) {
+  load_rows(rbeg);
+  for (int b0 = rbeg; b0 < rend; b0 += kRowStep) {
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-      const int e = tid + 256 * i, rr = e / hn, j = e - rr * hn;
-      z[rr * zl + j] = v[i];
-    }
-    if (b0 + kBfBatch < rend) load_batch(b0 + kBfBatch);
-    __syncthreads();
-    fft_lines<-1>(z, kBfBatch, hn, G.logn - 1, tw_fwd_hn, zl);
-#pragma unroll
-    for (int i = 0; i < (kBfBatch * nb + 255) / 256; ++i) {
-      const int e = tid + 256 * i;
-      if (e >= kBfBatch * nb) break;
-      const int rr = e / nb, k = e - rr * nb;
-      const float2 zk = z[rr * zl + (k % hn)];
-      const float2 zc = cconj(z[rr * zl + ((hn - k) % hn)]);
+    for (int i = 0; i < kPer; ++i) z[(i >> 2) * zl + lane + 32 * (i & 3)] = v[i];
+    __syncwarp();
+    if (b0 + kRowStep < rend) load_rows(b0 + kRowStep);
+    fft_warp<hn, -1>(z, kBfRows, zl, tw_fwd_hn);
+#pragma unroll 4
+    for (int k0 = 0; k0 <= hn; k0 += 8) {
+      const int k = k0 + kl;
+      if (k > hn) break;
+      const float2 zk = z[rr * zl + (k & (hn - 1))];
+      const float2 zc = cconj(z[rr * zl + ((hn - k) & (hn - 1))]);
       const float2 ev = make_float2(0.5f * (zk.x + zc.x), 0.5f * (zk.y + zc.y));
       const float2 d = csub(zk, zc);
       const float2 od = make_float2(0.5f * d.y, -0.5f * d.x);
@@ -560,7 +574,7 @@ k_block_filter(FftGeom G, const float* __restrict__ src, int w, int h, const int
       else
         *bin(k, b0 + rr) = X;
     }
-    __syncthreads();
+    __syncwarp();
   }
   cl.sync();
 
@@ -570,7 +584,7 @@ k_block_filter(FftGeom G, const float* __restrict__ src, int w, int h, const int
   // DC + i Nyquist splits into A = (Z_k + conj Z_-k) / 2 (the DC column's) and
   // B = (Z_k - conj Z_-k) / 2i (the Nyquist column's), each is filtered with
   // its own column's factor, and A + iB is put back.
-  fft_lines<-1>(x, ncol, n, G.logn, tw_fwd_n, ls);
+  fft_lines_4step_d<n, -1>(x, kBfCols, ls, tw_fwd_n);
   {
     const int cell = block_cell[item];
     const double vs = vsr[2 * item], vr = vsr[2 * item + 1];
@@ -612,31 +626,28 @@ k_block_filter(FftGeom G, const float* __restrict__ src, int w, int h, const int
     }
   }
   __syncthreads();
-  fft_lines<1>(x, ncol, n, G.logn, tw_inv_n, ls);
+  fft_lines_4step_d<n, 1>(x, kBfCols, ls, tw_inv_n);
   cl.sync();
 
-  // Row inverse (c2r): gather each row's bins from the owners; the next
-  // batch's bins are requested while this batch transforms.
-  float2 xk[kPer], xc[kPer];
-  auto gather_batch = [&](int b) {
+  // Row inverse (c2r): a warp gathers its four rows' bins from the owners.
+  for (int b0 = rbeg; b0 < rend; b0 += kRowStep) {
+    const int row = b0 + rr;
+    float2 xk[kPer], xc[kPer];
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-      const int e = tid + 256 * i, rr = e / hn, k = e - rr * hn;
+      const int k = 8 * i + kl;
       if (k == 0) {  // the packed line: DC in the real part, Nyquist in the imaginary part
-        const float2 p = *cl.map_shared_rank(x + b + rr, 0);
+        const float2 p = *cl.map_shared_rank(x + row, 0);
         xk[i] = make_float2(p.x, 0.0f);
         xc[i] = make_float2(p.y, 0.0f);
       } else {
-        xk[i] = *bin(k, b + rr);
-        xc[i] = cconj(*bin(hn - k, b + rr));
+        xk[i] = *bin(k, row);
+        xc[i] = cconj(*bin(hn - k, row));
       }
     }
-  };
-  gather_batch(rbeg);
-  for (int b0 = rbeg; b0 < rend; b0 += kBfBatch) {
 #pragma unroll
     for (int i = 0; i < kPer; ++i) {
-      const int e = tid + 256 * i, rr = e / hn, k = e - rr * hn;
+      const int k = 8 * i + kl;
       float2 a = xk[i], c = xc[i];
       if (k == 0) {  // c2r ignores the imaginary parts of the DC and Nyquist bins
         a.y = 0.0f;
@@ -646,16 +657,14 @@ k_block_filter(FftGeom G, const float* __restrict__ src, int w, int h, const int
       const float2 o2 = cmul(csub(a, c), split_inv[k]);
       z[rr * zl + k] = make_float2(e2.x - o2.y, e2.y + o2.x);  // 2E + i 2O
     }
-    if (b0 + kBfBatch < rend) gather_batch(b0 + kBfBatch);
-    __syncthreads();
-    fft_lines<1>(z, kBfBatch, hn, G.logn - 1, tw_inv_hn, zl);
-#pragma unroll 4
-    for (int i = 0; i < kBfBatch * n / 256; ++i) {
-      const int e = tid + 256 * i, rr = e / n, m = e - rr * n;
-      const float2 v = z[rr * zl + (m >> 1)];
-      dense_out[(static_cast<size_t>(item) * n + b0 + rr) * n + m] = (m & 1) ? v.y : v.x;
+    __syncwarp();
+    fft_warp<hn, 1>(z, kBfRows, zl, tw_inv_hn);
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      const int j = lane + 32 * (i & 3);
+      reinterpret_cast<float2*>(dense_out + (static_cast<size_t>(item) * n + b0 + (i >> 2)) * n)[j] = z[(i >> 2) * zl + j];
     }
-    __syncthreads();
+    __syncwarp();
   }
   cl.sync();  // this CTA's lines stay alive until every rank has gathered
 }
@@ -668,7 +677,9 @@ k_block_filter(FftGeom G, const float* __restrict__ src, int w, int h, const int
 // One CTA per tile of kOlaTW columns x kOlaTH rows, one thread per column: a
 // thread finds its column's covering blocks (in colour order) and their Hann
 // weights once, the CTA finds each row's once (shared memory), and every pixel
-// then reads only its block outputs.
+// then reads only its block outputs. Bound by the FP64 conversions of that float
+// rounding; the weight sums' reciprocals are one division per row and column (two
+// FP64 divisions per pixel: 132 us at 2048 x 4096, now 101).
 constexpr int kOlaTW = 128;
 constexpr int kOlaTH = 16;
 
@@ -697,9 +708,11 @@ k_ola_gather(int w, int h, int n, const int* __restrict__ oxs, int nox, const in
              const double* __restrict__ wx_total, const double* __restrict__ wy_total, float* __restrict__ acc,
              float* __restrict__ var_acc) {
   __shared__ int r_iy[kOlaTH][3], r_ly[kOlaTH][3];
-  __shared__ double r_wyt[kOlaTH];
+  __shared__ double r_hw[kOlaTH][3], r_sig[kOlaTH][3];
+  __shared__ double r_wyt[kOlaTH], r_ryt[kOlaTH];
   const int x = blockIdx.x * kOlaTW + threadIdx.x;
   const int y0 = blockIdx.y * kOlaTH;
+  const double inv_n2 = static_cast<double>(1.0f / static_cast<float>(static_cast<size_t>(n) * n));
   if (threadIdx.x < kOlaTH && y0 + static_cast<int>(threadIdx.x) < h) {
     const int y = y0 + threadIdx.x;
     int iy[3], ly[3];
@@ -708,8 +721,11 @@ k_ola_gather(int w, int h, int n, const int* __restrict__ oxs, int nox, const in
     for (int r = 0; r < 3; ++r) {
       r_iy[threadIdx.x][r] = iy[r];
       r_ly[threadIdx.x][r] = ly[r];
+      r_hw[threadIdx.x][r] = hwin[ly[r]];
+      r_sig[threadIdx.x][r] = hwin[ly[r]] * inv_n2;
     }
     r_wyt[threadIdx.x] = wy_total[y];
+    r_ryt[threadIdx.x] = 1.0 / wy_total[y];
   }
   __syncthreads();
   if (x >= w) return;
@@ -718,8 +734,7 @@ k_ola_gather(int w, int h, int n, const int* __restrict__ oxs, int nox, const in
   double wxv[3];
 #pragma unroll
   for (int r = 0; r < 3; ++r) wxv[r] = ix[r] >= 0 ? hwin[lx[r]] : 0.0;
-  const double wxt = wx_total[x];
-  const double inv_n2 = static_cast<double>(1.0f / static_cast<float>(static_cast<size_t>(n) * n));
+  const double wxt = wx_total[x], rxt = 1.0 / wxt;
   const int rows = min(kOlaTH, h - y0);
   for (int t = 0; t < rows; ++t) {
     const int y = y0 + t;
@@ -735,8 +750,8 @@ k_ola_gather(int w, int h, int n, const int* __restrict__ oxs, int nox, const in
         const int ly = r_ly[t][cb];
         const float f = bout[(static_cast<size_t>(item) * n + ly) * n + lx[ca]];
         const double num = bnum[item];
-        const double wy_sig = hwin[ly] * inv_n2;
-        const double wy_var = hwin[ly];
+        const double wy_sig = r_sig[t][cb];
+        const double wy_var = r_hw[t][cb];
         a = static_cast<float>(static_cast<double>(a) + wy_sig * wxv[ca] * static_cast<double>(f));
         v = static_cast<float>(static_cast<double>(v) + wy_var * wxv[ca] * num);
       }
@@ -744,8 +759,9 @@ k_ola_gather(int w, int h, int n, const int* __restrict__ oxs, int nox, const in
     const double ws = r_wyt[t] * wxt;
     const size_t o = static_cast<size_t>(y) * w + x;
     if (ws > 0.0) {
-      acc[o] = static_cast<float>(static_cast<double>(a) / ws);
-      var_acc[o] = static_cast<float>(static_cast<double>(v) / ws);
+      const double rs = r_ryt[t] * rxt;
+      acc[o] = static_cast<float>(static_cast<double>(a) * rs);
+      var_acc[o] = static_cast<float>(static_cast<double>(v) * rs);
     } else {
       acc[o] = 0.0f;
       var_acc[o] = 0.0f;
@@ -846,59 +862,145 @@ k_block_var(FftGeom G, const float* __restrict__ vs, const float* __restrict__ v
   if (threadIdx.x == 0) vsr[2 * item + layer] = static_cast<double>(__uint_as_float(s_prefix));
 }
 
-// Local kernel per cell: K = sum_n float(a_n(cx,cy)) phi_n (exact thin-plate
-// fields at the cell's representative block centre), sum K^2 in FP64, and its
-// zero-phase embedding into an n x n real image (src/noise.cpp:65-84, 167-189,
-// 329-343). `dense` must be zeroed beforehand.
+constexpr int kCpCols = 16;  // column lines of k_cell_power at a time
+
+// Local kernel of a cell: K = sum_n float(a_n(cx,cy)) phi_n (exact thin-plate
+// fields at the cell's representative block centre) into kk (shared), and sum K^2 in
+// FP64 (returned by thread 0). A thread per knot, per coefficient of the point and
+// per field (one thread doing all of them took 54 us at 465 cells); blockDim 256.
+constexpr int kCellKnots = 1024, kCellFields = 256;
+struct CellShared {
+  double s[kCellKnots];  // thin-plate values at the knots
+  double d[kCellKnots];  // the point's design row
+  double red[256];
+  float an[kCellFields];
+};
+__device__ double cell_kernel(CellShared& S, const TpsDev& t, const double* __restrict__ theta, int nc,
+                              const float* __restrict__ phi, int ks, double cx, double cy, float* kk) {
+  const int k = t.k, nr = k - 3, tid = threadIdx.x;
+  const double ux = (cx - t.cx) / t.scale, uy = (cy - t.cy) / t.scale;
+  for (int j = tid; j < k; j += blockDim.x) {
+    const double dx = ux - t.kn[2 * j], dy = uy - t.kn[2 * j + 1];
+    const double r2 = dx * dx + dy * dy;
+    S.s[j] = r2 <= 0.0 ? 0.0 : 0.5 * r2 * log(r2);
+  }
+  __syncthreads();
+  for (int m = tid; m < k; m += blockDim.x) {
+    double v = m == nr ? 1.0 : m == nr + 1 ? ux : uy;
+    if (m < nr) {
+      v = 0.0;
+      for (int j = 0; j < k; ++j) v = fma(S.s[j], t.z[j * nr + m], v);
+    }
+    S.d[m] = v;
+  }
+  __syncthreads();
+  for (int q = tid; q < nc; q += blockDim.x) {
+    double f = 0.0;
+    for (int m = 0; m < k; ++m) f = fma(S.d[m], theta[q * k + m], f);
+    S.an[q] = static_cast<float>(f);
+  }
+  __syncthreads();
+  double part = 0.0;
+  for (int i = tid; i < ks * ks; i += blockDim.x) {
+    float v = 0.0f;
+    for (int q = 0; q < nc; ++q) v = __fmaf_rn(S.an[q], phi[static_cast<size_t>(q) * ks * ks + i], v);
+    kk[i] = v;
+    part = fma(static_cast<double>(v), static_cast<double>(v), part);
+  }
+  S.red[tid] = part;
+  __syncthreads();
+  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+    if (tid < o) S.red[tid] += S.red[tid + o];
+    __syncthreads();
+  }
+  return S.red[0];
+}
+
+// The kernel of each cell and its zero-phase embedding into an n x n real image
+// (src/noise.cpp:65-84, 167-189, 329-343). `dense` must be zeroed beforehand.
 __global__ void __launch_bounds__(256)
 k_local_kernels(FftGeom G, TpsDev t, const double* __restrict__ theta, int nc, const float* __restrict__ phi,
                 int ks, const double* __restrict__ centres, double* __restrict__ sumk2, float* __restrict__ dense,
                 float* __restrict__ kern_out) {
   extern __shared__ float kk[];
-  __shared__ float an[64];
-  __shared__ double red[256];
-  const int cell = blockIdx.x, n = G.n;
-  if (threadIdx.x == 0) {
-    double d[64];
-    const double cx = centres[2 * cell], cy = centres[2 * cell + 1];
-    const int k = t.k, nr = k - 3;
-    const double ux = (cx - t.cx) / t.scale, uy = (cy - t.cy) / t.scale;
-    for (int m = 0; m < nr; ++m) d[m] = 0.0;
-    for (int j = 0; j < k; ++j) {
-      const double dx = ux - t.kn[2 * j], dy = uy - t.kn[2 * j + 1];
-      const double r2 = dx * dx + dy * dy;
-      const double s = r2 <= 0.0 ? 0.0 : 0.5 * r2 * log(r2);
-      for (int m = 0; m < nr; ++m) d[m] = fma(s, t.z[j * nr + m], d[m]);
-    }
-    d[nr] = 1.0;
-    d[nr + 1] = ux;
-    d[nr + 2] = uy;
-    for (int q = 0; q < nc; ++q) {
-      double f = 0.0;
-      for (int m = 0; m < k; ++m) f = fma(d[m], theta[q * k + m], f);
-      an[q] = static_cast<float>(f);
-    }
-  }
-  __syncthreads();
-  const int r = ks / 2;
-  double part = 0.0;
+  __shared__ CellShared S;
+  const int cell = blockIdx.x, n = G.n, r = ks / 2;
+  const double s2 = cell_kernel(S, t, theta, nc, phi, ks, centres[2 * cell], centres[2 * cell + 1], kk);
   for (int i = threadIdx.x; i < ks * ks; i += blockDim.x) {
-    float v = 0.0f;
-    for (int q = 0; q < nc; ++q) v = __fmaf_rn(an[q], phi[static_cast<size_t>(q) * ks * ks + i], v);
-    kk[i] = v;
-    part = fma(static_cast<double>(v), static_cast<double>(v), part);
     const int ky = i / ks, kx = i - ky * ks;
     const int gy = ((ky - r) % n + n) % n, gx = ((kx - r) % n + n) % n;
-    if (dense) dense[(static_cast<size_t>(cell) * n + gy) * n + gx] = v;
-    if (kern_out) kern_out[static_cast<size_t>(cell) * ks * ks + i] = v;
+    if (dense) dense[(static_cast<size_t>(cell) * n + gy) * n + gx] = kk[i];
+    if (kern_out) kern_out[static_cast<size_t>(cell) * ks * ks + i] = kk[i];
   }
-  red[threadIdx.x] = part;
+  if (threadIdx.x == 0 && sumk2) sumk2[cell] = s2;
+}
+
+__host__ __device__ constexpr int cp_lines(int n) {  // float2 of the column lines
+  const int lines = kCpCols * (n + 17), scratch = static_cast<int>((sizeof(CellShared) + 7) / 8);
+  return lines > scratch ? lines : scratch;
+}
+
+// |Khat|^2 of each cell's kernel in one launch, for 128 and 256 point blocks: the
+// kernel, the row transforms of its ks rows (all other rows of the embedding are
+// zero) and the column transforms, C columns at a time, none of it through global
+// memory; CTA y of a cell takes every gridDim.y-th group of columns. The arithmetic
+// is that of the passes it replaces (k_local_kernels, k_rows_fwd, k_cols), which
+// wrote and read the dense image and the whole spectrum: 141 us at 465 cells of 256 x
+// 256, where they took 426 us. Bound as k_block_filter is, by the line transforms.
+__global__ void __launch_bounds__(256, 3)
+k_cell_power(FftGeom G, TpsDev t, const double* __restrict__ theta, int nc, const float* __restrict__ phi, int ks,
+             const double* __restrict__ centres, double* __restrict__ sumk2, double* __restrict__ power) {
+  extern __shared__ __align__(16) float2 fsm2[];
+  const int n = G.n, hn = n / 2, nb = hn + 1, r = ks / 2;
+  constexpr int C = kCpCols;
+  const int zl = fft_ls(hn, false), ls = fft_ls(n, true);
+  float2* x = fsm2;              // C x ls column lines; before them cell_kernel's scratch
+  float2* z = x + cp_lines(n);   // ks x zl row lines
+  CellShared& S = *reinterpret_cast<CellShared*>(x);
+  float2* tw = z + ks * zl;      // n/2
+  float2* twh = tw + n / 2;      // hn/2
+  float2* split = twh + hn / 2;  // nb
+  float* kk = reinterpret_cast<float*>(split + nb);
+  copy_tw(tw, G.tw_tab, n / 2);
+  copy_tw(twh, G.tw_tab + tw_off_fwd_hn(n), hn / 2);
+  copy_tw(split, G.tw_tab + tw_off_split_fwd(n), nb);
+  const int cell = blockIdx.x;
+  const double s2 = cell_kernel(S, t, theta, nc, phi, ks, centres[2 * cell], centres[2 * cell + 1], kk);
+  if (threadIdx.x == 0 && blockIdx.y == 0) sumk2[cell] = s2;
+  for (int e = threadIdx.x; e < ks * hn; e += blockDim.x) {
+    const int ky = e / hn, j = e - ky * hn;
+    const int k0 = (2 * j + r) & (n - 1), k1 = (2 * j + 1 + r) & (n - 1);
+    z[ky * zl + j] = make_float2(k0 < ks ? kk[ky * ks + k0] : 0.0f, k1 < ks ? kk[ky * ks + k1] : 0.0f);
+  }
   __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (threadIdx.x < static_cast<unsigned>(o)) red[threadIdx.x] += red[threadIdx.x + o];
+  fft_lines<-1>(z, ks, hn, G.logn - 1, twh, zl);
+  for (int c0 = blockIdx.y * C; c0 < nb; c0 += gridDim.y * C) {
+    const int ncol = min(C, nb - c0);
+    for (int e = threadIdx.x; e < C * n; e += blockDim.x) {
+      const int row = e / C, cc = e - row * C, ky = (row + r) & (n - 1), k = c0 + cc;
+      float2 X = make_float2(0.0f, 0.0f);
+      if (cc >= ncol) continue;
+      if (ky < ks) {
+        const float2 zk = z[ky * zl + (k & (hn - 1))];
+        const float2 zc = cconj(z[ky * zl + ((hn - k) & (hn - 1))]);
+        const float2 ev = make_float2(0.5f * (zk.x + zc.x), 0.5f * (zk.y + zc.y));
+        const float2 d = csub(zk, zc);                           // 2i O
+        const float2 od = make_float2(0.5f * d.y, -0.5f * d.x);  // O = d / (2i)
+        X = cadd(ev, cmul(split[k], od));
+      }
+      x[cc * ls + row] = X;
+    }
+    __syncthreads();
+    fft_lines<-1>(x, ncol, n, G.logn, tw, ls);
+    for (int e = threadIdx.x; e < C * n; e += blockDim.x) {
+      const int row = e / C, cc = e - row * C;
+      if (cc >= ncol) continue;
+      const float2 v = x[cc * ls + row];
+      const double re = v.x, im = v.y;
+      power[(static_cast<size_t>(cell) * n + row) * nb + c0 + cc] = re * re + im * im;
+    }
     __syncthreads();
   }
-  if (threadIdx.x == 0 && sumk2) sumk2[cell] = red[0];
 }
 
 // Normalise by the separable Hann weight sum (src/noise.cpp:458-479).
@@ -992,6 +1094,7 @@ void launch_block_var(cudaStream_t s, const FftGeom& g, int nitems, int nextra, 
 void launch_local_kernels(cudaStream_t s, const FftGeom& g, int ncell, const TpsDev& t, const double* theta, int nc,
                           const float* phi, int ks, const double* centres, double* sumk2, float* dense,
                           float* kern_out) {
+  if (t.k > kCellKnots || nc > kCellFields) fail(DGPU_ERR_INVALID, "decorrelate: too many knots or components");
   const size_t smem = sizeof(float) * static_cast<size_t>(ks) * ks;
   ensure_dynamic_smem(reinterpret_cast<const void*>(k_local_kernels), smem);
   k_local_kernels<<<ncell, 256, smem, s>>>(g, t, theta, nc, phi, ks, centres, sumk2, dense, kern_out);
@@ -1000,13 +1103,37 @@ void launch_local_kernels(cudaStream_t s, const FftGeom& g, int ncell, const Tps
 
 bool block_filter_fused(const FftGeom& g) { return g.n == kBfN && g.tw_tab != nullptr; }
 
+static size_t cell_power_smem(const FftGeom& g, int ks) {
+  const int n = g.n, hn = n / 2;
+  return sizeof(float2) * (static_cast<size_t>(cp_lines(n)) + static_cast<size_t>(ks) * fft_ls(hn, false) +
+                           n / 2 + hn / 2 + hn + 1) +
+         sizeof(float) * ks * ks;
+}
+bool cell_power_fused(const FftGeom& g, int ks, int knots, int nc) {
+  return (g.n == 128 || g.n == 256) && g.tw_tab != nullptr && ks <= g.n / 2 && knots <= kCellKnots &&
+         nc <= kCellFields &&
+         cell_power_smem(g, ks) <= 160 * 1024;
+}
+void launch_cell_power(cudaStream_t s, const FftGeom& g, int ncell, const TpsDev& t, const double* theta, int nc,
+                       const float* phi, int ks, const double* centres, double* sumk2, double* power) {
+  // Column groups over several CTAs per cell while there are fewer than four per SM;
+  // with more cells each CTA would repeat the kernel and its rows for nothing (465
+  // cells: 1, 2, 3, 5 and 9 CTAs each take 141, 153, 149, 146 and 172 us).
+  const int groups = (g.n / 2 + 1 + kCpCols - 1) / kCpCols;
+  const int split = std::min(groups, std::max(1, 148 * 4 / std::max(ncell, 1)));
+  const size_t smem = cell_power_smem(g, ks);
+  ensure_dynamic_smem(reinterpret_cast<const void*>(k_cell_power), smem);
+  k_cell_power<<<dim3(ncell, split), 256, smem, s>>>(g, t, theta, nc, phi, ks, centres, sumk2, power);
+  DGPU_LAUNCH("k_cell_power");
+}
+
 void launch_block_filter(cudaStream_t s, const FftGeom& g, int nitems, const float* src, int w, int h,
                          const int* oxs, const int* oys, int nox, const double* cell_power, const double* cell_sumk2,
                          const int* block_cell, const double* vsr, double* bnum, float* dense_out) {
   if (!block_filter_fused(g)) fail(DGPU_ERR_INVALID, "decorrelate: fused block filter needs n = 256 and a twiddle table");
   if (nitems == 0) return;
   const size_t smem = sizeof(float2) * (static_cast<size_t>(kBfCols) * fft_ls(kBfN, true) +
-                                        static_cast<size_t>(kBfBatch) * fft_ls(kBfN / 2, false) + twiddle_table_len(kBfN));
+                                        static_cast<size_t>(256 / 32) * kBfRows * kBfZl + twiddle_table_len(kBfN));
   ensure_dynamic_smem(reinterpret_cast<const void*>(k_block_filter), smem);
   k_block_filter<<<nitems * kBfRanks, 256, smem, s>>>(g, src, w, h, oxs, oys, nox, cell_power, cell_sumk2, block_cell,
                                                        vsr, bnum, dense_out);

@@ -228,7 +228,7 @@ template <class Group>
 __device__ void ldlt_blocked(double* B, int P, double* Wt, double* Lt, double (*rows)[kLb + 1], const Group& grp) {
   __shared__ double blk[kLb][kLb + 1];  // L of the diagonal block (d on the diagonal)
   __shared__ double wk[kLb][kLb + 1];   // wk[j][k] = d_j l_kj
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = blockDim.x;
+  const int tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), nt = blockDim.x;
   const int rank = grp.rank(), nr = grp.count();
   for (int p0 = 0; p0 < P; p0 += kLb) {
     const int nb = min(kLb, P - p0);
@@ -370,7 +370,7 @@ struct LdltWork {
 __global__ void __launch_bounds__(kLdltThreads) k_ldlt_factor(SolveBatch b, int s0, LdltWork wk) {
   extern __shared__ double lrows[][kLb + 1];
   __shared__ LdltShared S;
-  const int P = b.P, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int P = b.P, tid = threadIdx.x, lane = tid & 31, warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const size_t PP = static_cast<size_t>(P) * P;
   const int s = s0 + static_cast<int>(blockIdx.x);
   double* A = wk.d + blockIdx.x * ldlt_sys_doubles(P);
