@@ -8,6 +8,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <cstdlib>
 #include <cmath>
 
@@ -23,66 +24,83 @@ namespace dgpu {
 __device__ __forceinline__ double tps_green_d(double r2) { return r2 <= 0.0 ? 0.0 : 0.5 * r2 * log(r2); }
 
 // fields(p, f) = design(p) . theta[f*k:(f+1)*k], design = [sigma Z | 1 | u | v]
-// (src/spatial.cpp:67-97, src/subtract.cpp:58-63).
-__device__ void eval_fields_at(const TpsDev t, const double* __restrict__ theta, int nf, double x,
-                               double y, double* out /* nf */) {
-  constexpr int kMaxK = 64;
-  double d[kMaxK];
+// (src/spatial.cpp:67-97, src/subtract.cpp:58-63), of 32 points by a CTA: lane =
+// point, the warps share the knots, then the design's columns, then the fields (each
+// sum whole and in order in one thread). put(f, value) takes this lane's point. A
+// thread per point doing all of it, its design row in local memory, took 17 us for
+// the lattice of a 256 x 320 frame and 37 us at 4096 x 4096, now 6 and 12.
+constexpr int kFieldPoints = 32;
+size_t fields_smem(int k) { return sizeof(double) * 2 * kFieldPoints * static_cast<size_t>(k); }
+template <class Put>
+__device__ __forceinline__ void eval_fields(const TpsDev& t, const double* __restrict__ theta, int nf, double x, double y,
+                                            Put put) {
+  extern __shared__ __align__(16) double fsm[];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
   const int k = t.k, nr = k - 3;
+  double* s = fsm + lane;                     // k x 32
+  double* d = s + kFieldPoints * k;           // k x 32
   const double ux = (x - t.cx) / t.scale, uy = (y - t.cy) / t.scale;
-  for (int m = 0; m < nr; ++m) d[m] = 0.0;
-  for (int j = 0; j < k; ++j) {
-    const double dx = ux - t.kn[2 * j], dy = uy - t.kn[2 * j + 1];
-    const double s = tps_green_d(dx * dx + dy * dy);
-    for (int m = 0; m < nr; ++m) d[m] = fma(s, t.z[j * nr + m], d[m]);
+  for (int j = warp; j < k; j += warps) {
+    const double dx = ux - __ldg(t.kn + 2 * j), dy = uy - __ldg(t.kn + 2 * j + 1);
+    s[j * kFieldPoints] = tps_green_d(dx * dx + dy * dy);
   }
-  d[nr] = 1.0;
-  d[nr + 1] = ux;
-  d[nr + 2] = uy;
-  for (int f = 0; f < nf; ++f) {
-    double acc = 0.0;
+  __syncthreads();
+  for (int m = warp; m < k; m += warps) {
+    double v = m == nr ? 1.0 : m == nr + 1 ? ux : uy;
+    if (m < nr) {
+      v = 0.0;
+#pragma unroll 5
+      for (int j = 0; j < k; ++j) v = fma(s[j * kFieldPoints], __ldg(t.z + j * nr + m), v);
+    }
+    d[m * kFieldPoints] = v;
+  }
+  __syncthreads();
+  for (int f = warp; f < nf; f += warps) {
     const double* th = theta + static_cast<size_t>(f) * k;
-    for (int m = 0; m < k; ++m) acc = fma(d[m], th[m], acc);
-    out[f] = acc;
+    double acc = 0.0;
+#pragma unroll 5
+    for (int m = 0; m < k; ++m) acc = fma(d[m * kFieldPoints], __ldg(th + m), acc);
+    put(f, acc);
   }
 }
 
-__global__ void k_lattice(TpsDev t, const double* __restrict__ theta, int nf,
-                          const int* __restrict__ gx, const int* __restrict__ gy, int ncx, int ncy,
-                          double* __restrict__ lat, float* __restrict__ latf) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= ncx * ncy) return;
-  const int ix = i % ncx, iy = i / ncx;
-  double f[64];
-  eval_fields_at(t, theta, nf, static_cast<double>(gx[ix]), static_cast<double>(gy[iy]), f);
-  for (int q = 0; q < nf; ++q) {
-    const size_t o = (static_cast<size_t>(q) * ncy + iy) * ncx + ix;
-    lat[o] = f[q];
-    latf[o] = static_cast<float>(f[q]);
-  }
+__global__ void __launch_bounds__(256) k_lattice(TpsDev t, const double* __restrict__ theta, int nf,
+                                                 const int* __restrict__ gx, const int* __restrict__ gy, int ncx,
+                                                 int ncy, double* __restrict__ lat, float* __restrict__ latf) {
+  const int i = blockIdx.x * kFieldPoints + (threadIdx.x & 31), n = ncx * ncy;
+  const int at = min(i, n - 1), ix = at % ncx, iy = at / ncx;
+  eval_fields(t, theta, nf, static_cast<double>(gx[ix]), static_cast<double>(gy[iy]), [&](int f, double v) {
+    if (i >= n) return;
+    const size_t o = (static_cast<size_t>(f) * ncy + iy) * ncx + ix;
+    lat[o] = v;
+    latf[o] = static_cast<float>(v);
+  });
 }
 
-__global__ void k_exact_fields(TpsDev t, const double* __restrict__ theta, int nf, int w, int h,
-                               float* __restrict__ full) {
-  const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= static_cast<int64_t>(w) * h) return;
-  const int x = static_cast<int>(i % w), y = static_cast<int>(i / w);
-  double f[64];
-  eval_fields_at(t, theta, nf, static_cast<double>(x), static_cast<double>(y), f);
-  for (int q = 0; q < nf; ++q) full[static_cast<size_t>(q) * w * h + i] = static_cast<float>(f[q]);
+__global__ void __launch_bounds__(256) k_exact_fields(TpsDev t, const double* __restrict__ theta, int nf, int w, int h,
+                                                      float* __restrict__ full) {
+  const int64_t i = static_cast<int64_t>(blockIdx.x) * kFieldPoints + (threadIdx.x & 31), n = static_cast<int64_t>(w) * h;
+  const int64_t at = min(i, n - 1);
+  eval_fields(t, theta, nf, static_cast<double>(at % w), static_cast<double>(at / w), [&](int f, double v) {
+    if (i < n) full[static_cast<size_t>(f) * n + i] = static_cast<float>(v);
+  });
 }
 
 void launch_lattice(cudaStream_t s, const TpsDev& t, const double* theta, int nf, const int* gx,
                     const int* gy, int ncx, int ncy, double* lat, float* latf) {
   const int n = ncx * ncy;
-  k_lattice<<<ceil_div(n, 128), 128, 0, s>>>(t, theta, nf, gx, gy, ncx, ncy, lat, latf);
+  const size_t smem = fields_smem(t.k);
+  ensure_dynamic_smem(reinterpret_cast<const void*>(k_lattice), smem);
+  k_lattice<<<ceil_div(n, kFieldPoints), 256, smem, s>>>(t, theta, nf, gx, gy, ncx, ncy, lat, latf);
   DGPU_LAUNCH("k_lattice");
 }
 
 void launch_exact_fields(cudaStream_t s, const TpsDev& t, const double* theta, int nf, int w, int h,
                          float* full) {
   const int64_t n = static_cast<int64_t>(w) * h;
-  k_exact_fields<<<ceil_div(n, 128), 128, 0, s>>>(t, theta, nf, w, h, full);
+  const size_t smem = fields_smem(t.k);
+  ensure_dynamic_smem(reinterpret_cast<const void*>(k_exact_fields), smem);
+  k_exact_fields<<<ceil_div(n, kFieldPoints), 256, smem, s>>>(t, theta, nf, w, h, full);
   DGPU_LAUNCH("k_exact_fields");
 }
 
@@ -448,8 +466,20 @@ void launch_model_convolve_orders(cudaStream_t s, const SubtractArgs& a, const i
 // (ly, lx) tap order; then + Var(S).
 // ---------------------------------------------------------------------------
 
+// 4 x 4 adjacent outputs per thread. A window row is kept as four planes of every
+// fourth column, so that the 16 threads of a row read consecutive words and each
+// step along the taps takes one new window value; four taps of a row come with one
+// 16-byte load. That is 8 loads for 64 multiply-adds, which leaves the FP32 pipe the
+// bound of the taps; the squares' ordered FP64 sums and the window come on top.
+// 4096 x 4096: 166 us at radius 8, where columns 16 apart and taps one by one (8 loads
+// for 16) took 211.
+
 constexpr int kVarB = 64;
 constexpr int kVarMaxRk = 64;
+__host__ __device__ constexpr int var_tap_stride(int rk) { return (2 * rk + 1 + 3) & ~3; }
+// Floats of a plane: room for the columns the padded taps reach, and odd, so that the
+// two rows of outputs in a warp lie 16 banks apart.
+__host__ __device__ constexpr int var_plane(int rk) { return ((kVarB + 2 * rk + 1 + 6) / 4) | 1; }
 
 __global__ void __launch_bounds__(256)
 k_variance(int w, int h, DevFields F, const float* __restrict__ phi, int rk, int nc,
@@ -458,11 +488,12 @@ k_variance(int w, int h, DevFields F, const float* __restrict__ phi, int rk, int
   extern __shared__ __align__(16) unsigned char smraw[];
   const int ks = 2 * rk + 1;
   const int kk = ks * ks;
-  const int iw = kVarB + 2 * rk;
-  float* kf = reinterpret_cast<float*>(smraw);        // kk, mirrored K^2
-  float* k1 = kf + kk;                                // kk, K (unsquared)
-  float* win = k1 + kk;                               // iw * iw
-  float* an = win + iw * iw;                          // nc
+  // Window column c of a row lies at (c % 4) pw + c / 4.
+  const int pw = var_plane(rk), rs = 4 * pw;
+  float* k1 = reinterpret_cast<float*>(smraw);        // K (unsquared); then the taps, rows padded to whole fours
+  float* win = k1 + ks * var_tap_stride(rk);          // (kVarB + 2 rk) rows
+  float* kf = win + (kVarB + 2 * rk) * rs;            // kk, mirrored K^2
+  float* an = kf + kk;                                // nc
   __shared__ double s_qsum;
   __shared__ double s_box[kVarMaxRk];
   __shared__ float s_min[8], s_max[8];
@@ -489,6 +520,7 @@ k_variance(int w, int h, DevFields F, const float* __restrict__ phi, int rk, int
     // the barrier below.
     if (tid == 32) {
       double q = 0.0;
+#pragma unroll 8
       for (int i = 0; i < kk; ++i) q = fma(static_cast<double>(k1[i]), static_cast<double>(k1[i]), q);
       s_qsum = q;
     } else if (tid < 32) {
@@ -496,6 +528,7 @@ k_variance(int w, int h, DevFields F, const float* __restrict__ phi, int rk, int
         double box = 0.0;
         const int lo = rk - hw, hi = rk + hw;
         for (int yy = lo; yy <= hi; ++yy)
+#pragma unroll 4
           for (int xx = lo; xx <= hi; ++xx) box += static_cast<double>(kf[yy * ks + xx]);
         s_box[hw] = box;
       }
@@ -504,15 +537,29 @@ k_variance(int w, int h, DevFields F, const float* __restrict__ phi, int rk, int
     float lmin = INFINITY, lmax = -INFINITY;
     int finite = 1;
     const int iwh = bh + 2 * rk, iww = bw + 2 * rk;
-    for (int i = tid; i < iwh * iww; i += blockDim.x) {
-      const int r = i / iww, c = i - r * iww;
-      const int gy = by - rk + r, gx = bx - rk + c;
-      const float v = (gy < 0 || gy >= h || gx < 0 || gx >= w) ? 0.0f : __ldg(var_r + static_cast<size_t>(gy) * w + gx);
-      win[r * iw + c] = v;
-      lmin = fminf(lmin, v);
-      lmax = fmaxf(lmax, v);
-      finite &= isfinite(v) ? 1 : 0;
-    }
+    constexpr int kRows = 5;  // rows of a warp in flight together
+    for (int r0 = tid >> 5; r0 < iwh; r0 += 8 * kRows)
+      for (int c = tid & 31; c < rs; c += 32) {
+        const int gx = bx - rk + c;
+        const bool in = c < iww, xin = in && gx >= 0 && gx < w;
+        float v[kRows];
+#pragma unroll
+        for (int u = 0; u < kRows; ++u) {
+          const int r = r0 + 8 * u, gy = by - rk + r;
+          v[u] = (xin && r < iwh && gy >= 0 && gy < h) ? __ldg(var_r + static_cast<size_t>(gy) * w + gx) : 0.0f;
+        }
+#pragma unroll
+        for (int u = 0; u < kRows; ++u) {
+          const int r = r0 + 8 * u;
+          if (r >= iwh) break;
+          win[r * rs + (c & 3) * pw + (c >> 2)] = v[u];
+          if (in) {
+            lmin = fminf(lmin, v[u]);
+            lmax = fmaxf(lmax, v[u]);
+            finite &= isfinite(v[u]) ? 1 : 0;
+          }
+        }
+      }
     for (int o = 16; o > 0; o >>= 1) {
       lmin = fminf(lmin, __shfl_xor_sync(0xffffffffu, lmin, o));
       lmax = fmaxf(lmax, __shfl_xor_sync(0xffffffffu, lmax, o));
@@ -541,61 +588,103 @@ k_variance(int w, int h, DevFields F, const float* __restrict__ phi, int rk, int
     const bool flat = wmax > 0.0f && (wmax - wmin) <= 1e-3f * wmax;
     const float q = static_cast<float>(s_qsum);
     const int lo = rk - hw, hi = rk + hw;
-    // 4 x 4 outputs per thread: rows oy0 .. oy0+3, columns tx + 16 j (strided,
-    // so a warp's window loads hit distinct banks). Per output the taps are
-    // still accumulated in (ly, lx) order.
+    // The taps of the box, rows padded with zeros (k1 is done with).
+    const int nt = 2 * hw + 1, ts = (nt + 3) & ~3;
+    for (int i = tid; i < nt * ts; i += blockDim.x) {
+      const int r = i / ts, c = i - r * ts;
+      k1[i] = c < nt ? kf[(lo + r) * ks + lo + c] : 0.0f;
+    }
+    __syncthreads();
+    // Outputs: rows oy0 .. oy0 + 3, columns 4 tx .. 4 tx + 3. Per output the taps are
+    // accumulated in (ly, lx) order.
     const int tx = tid & 15, oy0 = (tid >> 4) * 4;
-    // acc[i][p] holds columns 2p and 2p + 1 of row i as a pair: one packed FMA
-    // (__ffma2_rn, an IEEE fma per lane) per tap for two columns.
-    float2 acc[4][2];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-      for (int p = 0; p < 2; ++p) acc[i][p] = make_float2(0.0f, 0.0f);
+    float acc[4][4] = {};
     if (flat) {
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int p = 0; p < 2; ++p) {
-          const float* wp = win + (oy0 + i + rk) * iw + tx + 32 * p + rk;
-          acc[i][p] = make_float2(q * wp[0], q * wp[16]);
-        }
-    } else {
-      for (int r = 0; r <= 3 + 2 * hw; ++r) {
-        const float* wrp = win + (oy0 + lo + r) * iw + tx;
-        for (int lx = lo; lx <= hi; ++lx) {
-          float2 v[2];
+        for (int j = 0; j < 4; ++j) acc[i][j] = q * win[(oy0 + i + rk) * rs + ((rk + j) & 3) * pw + tx + ((rk + j) >> 2)];
+    } else if (all_finite) {
+      auto row = [&](int r, auto whole) {
+        const float* wr = win + (oy0 + lo + r) * rs + tx;
+        auto at = [&](int c) { return wr[(c & 3) * pw + (c >> 2)]; };  // window column 4 tx + c
+        float v[7];
 #pragma unroll
-          for (int p = 0; p < 2; ++p) v[p] = make_float2(wrp[32 * p + lx], wrp[32 * p + 16 + lx]);
+        for (int k = 0; k < 3; ++k) v[k] = at(lo + k);
+        auto taps = [&](int l, auto count) {
+          constexpr int K = decltype(count)::value;
+#pragma unroll
+          for (int k = 3; k < 3 + K; ++k) v[k] = at(lo + l + k);
 #pragma unroll
           for (int i = 0; i < 4; ++i) {
-            const int ly = lo + r - i;
-            if (ly < lo || ly > hi) continue;
-            const float c = kf[ly * ks + lx];
-            if (!all_finite && c == 0.0f) continue;
-            const float2 cc = make_float2(c, c);
+            const int ly = r - i;  // tap row
+            if (!decltype(whole)::value && (ly < 0 || ly >= nt)) continue;
+            const float4 c = *reinterpret_cast<const float4*>(k1 + ly * ts + l);
+            const float cv[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
-            for (int p = 0; p < 2; ++p) acc[i][p] = __ffma2_rn(cc, v[p], acc[i][p]);
+            for (int k = 0; k < K; ++k)
+#pragma unroll
+              for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(cv[k], v[k + j], acc[i][j]);
           }
+        };
+        int l = 0;
+        for (; l + 4 <= nt; l += 4) {
+          taps(l, std::integral_constant<int, 4>{});
+#pragma unroll
+          for (int k = 0; k < 3; ++k) v[k] = v[k + 4];
         }
+        if (nt & 2)  // nt is odd
+          taps(l, std::integral_constant<int, 3>{});
+        else
+          taps(l, std::integral_constant<int, 1>{});
+      };
+      for (int r = 0; r <= 2 * hw + 3; ++r) {
+        if (r >= 3 && r < nt)
+          row(r, std::true_type{});
+        else
+          row(r, std::false_type{});
       }
+    } else {  // zero taps are skipped
+      for (int r = 0; r <= 2 * hw + 3; ++r)
+        for (int l = 0; l < nt; ++l)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int ly = r - i;
+            if (ly < 0 || ly >= nt) continue;
+            const float c = k1[ly * ts + l];
+            if (c == 0.0f) continue;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              acc[i][j] = fmaf(c, win[(oy0 + lo + r) * rs + ((lo + l + j) & 3) * pw + tx + ((lo + l + j) >> 2)], acc[i][j]);
+          }
+    }
+    if (!flat)
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
-        for (int p = 0; p < 2; ++p) acc[i][p] = make_float2(0.0f + acc[i][p].x, 0.0f + acc[i][p].y);
-    }
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f + acc[i][j];
+    // Whole rows of four where every row starts on a 16-byte boundary.
+    const bool vec = (w & 3) == 0 && ((reinterpret_cast<uintptr_t>(var_out) | reinterpret_cast<uintptr_t>(var_s)) & 15) == 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int oy = oy0 + i;
       if (oy >= bh) continue;
+      const size_t o = static_cast<size_t>(by + oy) * w + bx + 4 * tx;
+      if (vec && 4 * tx + 3 < bw) {
+        float4 v = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        if (var_s) {
+          const float4 sv = __ldg(reinterpret_cast<const float4*>(var_s + o));
+          v = make_float4(v.x + sv.x, v.y + sv.y, v.z + sv.z, v.w + sv.w);
+        }
+        *reinterpret_cast<float4*>(var_out + o) = v;
+        continue;
+      }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const int ox = tx + 16 * j;
-        if (ox >= bw) continue;
-        const size_t o = static_cast<size_t>(by + oy) * w + bx + ox;
-        float v = (j & 1) ? acc[i][j >> 1].y : acc[i][j >> 1].x;
-        if (var_s) v = v + __ldg(var_s + o);
-        var_out[o] = v;
+        if (4 * tx + j >= bw) continue;
+        float v = acc[i][j];
+        if (var_s) v = v + __ldg(var_s + o + j);
+        var_out[o + j] = v;
       }
     }
   } else {
@@ -611,9 +700,12 @@ void launch_variance(cudaStream_t s, int w, int h, const DevFields& F, const flo
                      int nc, const float* var_s, const float* var_r, float* var_out) {
   const int ks = 2 * rk + 1;
   const int iw = kVarB + 2 * rk;
-  const size_t smem = sizeof(float) * (2 * static_cast<size_t>(ks) * ks + static_cast<size_t>(iw) * iw + nc + 4);
-  if (smem > 200 * 1024 || rk > kVarMaxRk)
+  // What is refused: more than 200 KB without the padding.
+  if (sizeof(float) * (2 * static_cast<size_t>(ks) * ks + static_cast<size_t>(iw) * iw + nc + 4) > 200 * 1024 ||
+      rk > kVarMaxRk)
     fail(DGPU_ERR_INVALID, "subtract: kernel radius too large for the variance engine");
+  const size_t smem = sizeof(float) * (static_cast<size_t>(ks) * var_tap_stride(rk) + static_cast<size_t>(iw) * 4 * var_plane(rk) +
+                                       static_cast<size_t>(ks) * ks + nc + 4);
   ensure_dynamic_smem(reinterpret_cast<const void*>(k_variance), smem);
   dim3 grid(ceil_div(w, kVarB), ceil_div(h, kVarB));
   k_variance<<<grid, 256, smem, s>>>(w, h, F, phi, rk, nc, var_s, var_r, var_out);
@@ -623,91 +715,186 @@ void launch_variance(cudaStream_t s, int w, int h, const DevFields& F, const flo
 // ---------------------------------------------------------------------------
 // Mask growth (src/subtract.cpp:826-914): science-side flags 1:1, reference
 // flags and saturated reference pixels OR-dilated by r (box), edge border r,
-// non-finite difference. One CTA per 32x32 tile with the (32+2r)^2 grow window
-// built on the fly in shared memory (x-dilate, then y-dilate).
-// exact_bad records the undilated garbage pixels for the fill pass.
+// non-finite difference. exact_bad records the undilated garbage pixels for the fill
+// pass. One CTA per T x T tile, four pixels to a 32-bit word: the grow window's words
+// are ORed along x from byte-shifted pairs (most are zero and skipped), then along y,
+// where a thread's four rows share the rows common to them. A byte per pixel, 2 r + 1
+// of them per output and direction, took 213 us at 4096 x 4096, radius 8, now 87.
 // ---------------------------------------------------------------------------
 
-constexpr int kMkT = 32;
-
-__global__ void __launch_bounds__(256)
+template <int T>
+__global__ void __launch_bounds__(T * T / 16)
 k_mask(int w, int h, const float* __restrict__ sci, const float* __restrict__ ref,
        const uint8_t* __restrict__ sm, const uint8_t* __restrict__ rm, int has_sat, float sat, int r,
-       const float* __restrict__ diff, uint8_t* __restrict__ mask_out, uint8_t* __restrict__ exact_bad) {
-  extern __shared__ uint8_t msm[];
-  const int gw = kMkT + 2 * r;
-  uint8_t* g = msm;              // gw x gw grow sources
-  uint8_t* gxr = g + gw * gw;    // gw rows x 32 cols after the x dilation
-  const int bx = blockIdx.x * kMkT, by = blockIdx.y * kMkT;
+       const float* __restrict__ diff, uint8_t* __restrict__ mask_out, uint8_t* __restrict__ exact_bad, int vec) {
+  extern __shared__ uint32_t msm32[];
+  constexpr int TW = T / 4;                    // words of a tile row
+  const int r4 = (r + 3) & ~3, gh = T + 2 * r, gw = (T + 2 * r4) / 4;
+  uint32_t* g = msm32;          // gh x gw words: columns from bx - r4
+  uint32_t* gxr = g + gh * gw;  // gh x TW after the x dilation
+  const int bx = blockIdx.x * T, by = blockIdx.y * T;
   const int tid = threadIdx.x;
+  // Flags that grow, of the four pixels from (x, y) on.
+  auto grow_word = [&](int x, int y) {
+    uint32_t v = 0;
+    if (y < 0 || y >= h || x + 3 < 0 || x >= w) return v;
+    const int64_t idx = static_cast<int64_t>(y) * w + x;
+    if (vec && x >= 0 && x + 3 < w) {
+      if (rm) v = __ldg(reinterpret_cast<const uint32_t*>(rm + idx));
+      if (has_sat) {
+        const float4 f = __ldg(reinterpret_cast<const float4*>(ref + idx));
+        v |= (f.x >= sat ? 0x2u : 0u) | (f.y >= sat ? 0x200u : 0u) | (f.z >= sat ? 0x20000u : 0u) |
+             (f.w >= sat ? 0x2000000u : 0u);
+      }
+      return v;
+    }
+    for (int k = 0; k < 4; ++k) {
+      if (x + k < 0 || x + k >= w) continue;
+      uint32_t m = rm ? rm[idx + k] : 0u;
+      if (has_sat && ref[idx + k] >= sat) m |= 2u;
+      v |= m << (8 * k);
+    }
+    return v;
+  };
   const bool need_grow = (rm != nullptr) || has_sat;
   if (need_grow) {
-    for (int i = tid; i < gw * gw; i += blockDim.x) {
+    for (int i = tid; i < gh * gw; i += blockDim.x) {
       const int yy = i / gw, xx = i - yy * gw;
-      const int gy = by - r + yy, gx = bx - r + xx;
-      uint8_t v = 0;
-      if (gy >= 0 && gy < h && gx >= 0 && gx < w) {
-        const size_t idx = static_cast<size_t>(gy) * w + gx;
-        if (rm) v |= rm[idx];
-        if (has_sat && ref[idx] >= sat) v |= 2;
-      }
-      g[i] = v;
+      g[i] = grow_word(bx - r4 + 4 * xx, by - r + yy);
     }
     __syncthreads();
-    for (int i = tid; i < gw * kMkT; i += blockDim.x) {
-      const int yy = i / kMkT, xx = i - yy * kMkT;
-      uint8_t acc = 0;
-      for (int d = 0; d <= 2 * r; ++d) acc |= g[yy * gw + xx + d];
+    for (int i = tid; i < gh * TW; i += blockDim.x) {
+      const int yy = i / TW, o = i - yy * TW;
+      const uint32_t* row = g + yy * gw + o;
+      const int b0 = r4 - r, last = (b0 + 2 * r + 3) >> 2;  // first byte; last word of the window
+      uint32_t any = 0;
+      for (int k = 0; k <= last; ++k) any |= row[k];
+      uint32_t acc = 0;
+      if (any) {
+        for (int d = b0; d <= b0 + 2 * r; ++d) {
+          const int k = d >> 2;
+          acc |= __funnelshift_r(row[k], k < last ? row[k + 1] : 0u, 8 * (d & 3));
+        }
+      }
       gxr[i] = acc;
     }
     __syncthreads();
   }
-  for (int i = tid; i < kMkT * kMkT; i += blockDim.x) {
-    const int ly = i / kMkT, lx = i - ly * kMkT;
-    const int x = bx + lx, y = by + ly;
-    if (x >= w || y >= h) continue;
-    const size_t idx = static_cast<size_t>(y) * w + x;
-    uint8_t m = 0;
-    uint8_t eb = 0;
-    if (sm && sm[idx]) {
-      m |= sm[idx];
-      eb = 1;
+  const int o = tid % TW, ly0 = tid / TW * 4, x0 = bx + 4 * o;
+  if (x0 >= w) return;
+  uint32_t grown[4] = {0, 0, 0, 0};
+  if (need_grow) {
+    // Rows ly0 + i .. ly0 + i + 2 r; those from 3 to 2 r belong to all four.
+    const uint32_t* col = gxr + ly0 * TW + o;
+    if (2 * r >= 3) {
+      uint32_t mid = 0;
+      for (int d = 3; d <= 2 * r; ++d) mid |= col[d * TW];
+      const uint32_t c0 = col[0], c1 = col[TW], c2 = col[2 * TW];
+      const uint32_t e1 = col[(2 * r + 1) * TW], e2 = col[(2 * r + 2) * TW], e3 = col[(2 * r + 3) * TW];
+      grown[0] = mid | c0 | c1 | c2;
+      grown[1] = mid | c1 | c2 | e1;
+      grown[2] = mid | c2 | e1 | e2;
+      grown[3] = mid | e1 | e2 | e3;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        for (int d = 0; d <= 2 * r; ++d) grown[i] |= col[(i + d) * TW];
     }
-    if (rm && rm[idx]) eb = 1;
-    if (has_sat) {
-      if (ref[idx] >= sat) eb = 1;
-      if (sci[idx] >= sat) {
-        m |= 2;
-        eb = 1;
+  }
+  const bool whole = vec && x0 + 3 < w;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int y = by + ly0 + i;
+    if (y >= h) break;
+    const size_t idx = static_cast<size_t>(y) * w + x0;
+    uint32_t sw = 0, rw = 0;
+    float rv[4] = {}, sv[4] = {}, dv[4] = {};
+    const int n = min(4, w - x0);
+    if (whole) {
+      if (sm) sw = __ldg(reinterpret_cast<const uint32_t*>(sm + idx));
+      if (rm) rw = __ldg(reinterpret_cast<const uint32_t*>(rm + idx));
+      const float4 d = __ldg(reinterpret_cast<const float4*>(diff + idx));
+      dv[0] = d.x, dv[1] = d.y, dv[2] = d.z, dv[3] = d.w;
+      if (has_sat) {
+        const float4 a = __ldg(reinterpret_cast<const float4*>(ref + idx)), c = __ldg(reinterpret_cast<const float4*>(sci + idx));
+        rv[0] = a.x, rv[1] = a.y, rv[2] = a.z, rv[3] = a.w;
+        sv[0] = c.x, sv[1] = c.y, sv[2] = c.z, sv[3] = c.w;
+      }
+    } else {
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (k >= n) break;
+        if (sm) sw |= static_cast<uint32_t>(sm[idx + k]) << (8 * k);
+        if (rm) rw |= static_cast<uint32_t>(rm[idx + k]) << (8 * k);
+        dv[k] = diff[idx + k];
+        if (has_sat) {
+          rv[k] = ref[idx + k];
+          sv[k] = sci[idx + k];
+        }
       }
     }
-    if (need_grow) {
-      uint8_t acc = 0;
-      for (int d = 0; d <= 2 * r; ++d) acc |= gxr[(ly + d) * kMkT + lx];
-      m |= acc;
+    uint32_t m = sw | grown[i], eb = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const int x = x0 + k;
+      uint32_t f = 0;
+      bool bad = ((sw | rw) >> (8 * k) & 0xffu) != 0;
+      if (has_sat) {
+        if (rv[k] >= sat) bad = true;
+        if (sv[k] >= sat) {
+          f = 2;
+          bad = true;
+        }
+      }
+      if (x < r || x >= w - r || y < r || y >= h - r) f |= 16;
+      if (!isfinite(dv[k])) {
+        f |= 8;
+        bad = true;
+      }
+      m |= f << (8 * k);
+      eb |= (bad ? 1u : 0u) << (8 * k);
     }
-    if (x < r || x >= w - r || y < r || y >= h - r) m |= 16;
-    if (!isfinite(diff[idx])) {
-      m |= 8;
-      eb = 1;
+    if (whole) {
+      *reinterpret_cast<uint32_t*>(mask_out + idx) = m;
+      *reinterpret_cast<uint32_t*>(exact_bad + idx) = eb;
+    } else {
+      for (int k = 0; k < n; ++k) {
+        mask_out[idx + k] = static_cast<uint8_t>(m >> (8 * k));
+        exact_bad[idx + k] = static_cast<uint8_t>(eb >> (8 * k));
+      }
     }
-    mask_out[idx] = m;
-    exact_bad[idx] = eb;
   }
+}
+
+static size_t mask_smem(int t, int r) {
+  return static_cast<size_t>(t + 2 * r) * (t + 2 * ((r + 3) & ~3) + t);
 }
 
 void launch_mask(cudaStream_t s, int w, int h, const float* sci, const float* ref,
                  const uint8_t* sm, const uint8_t* rm, double saturation, int r, const float* diff,
                  uint8_t* mask_out, uint8_t* exact_bad) {
-  const int gw = kMkT + 2 * r;
-  const size_t smem = static_cast<size_t>(gw) * gw + static_cast<size_t>(gw) * kMkT;
-  if (smem > 200 * 1024) fail(DGPU_ERR_INVALID, "subtract: kernel radius too large for mask growth");
-  ensure_dynamic_smem(reinterpret_cast<const void*>(k_mask), smem);
-  dim3 grid(ceil_div(w, kMkT), ceil_div(h, kMkT));
+  if (static_cast<size_t>(32 + 2 * r) * (64 + 2 * r) > 200 * 1024)
+    fail(DGPU_ERR_INVALID, "subtract: kernel radius too large for mask growth");
   const int has_sat = saturation > 0.0 ? 1 : 0;
-  k_mask<<<grid, 256, smem, s>>>(w, h, sci, ref, sm, rm, has_sat, static_cast<float>(saturation), r,
-                                 diff, mask_out, exact_bad);
-  DGPU_LAUNCH("k_mask");
+  const float sat = static_cast<float>(saturation);
+  // Words of four pixels need rows that start on their boundaries.
+  const uintptr_t bits = reinterpret_cast<uintptr_t>(sci) | reinterpret_cast<uintptr_t>(ref) | reinterpret_cast<uintptr_t>(diff);
+  const uintptr_t bytes = reinterpret_cast<uintptr_t>(sm) | reinterpret_cast<uintptr_t>(rm) |
+                          reinterpret_cast<uintptr_t>(mask_out) | reinterpret_cast<uintptr_t>(exact_bad);
+  const int vec = (w & 3) == 0 && (bits & 15) == 0 && (bytes & 3) == 0;
+  // Tiles of 64, whose windows overlap less, once there are two for every SM (below
+  // that 32 x 32 ones fill more of them).
+  auto go = [&](auto kern, int t) {
+    const size_t smem = mask_smem(t, r);
+    ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
+    kern<<<dim3(ceil_div(w, t), ceil_div(h, t)), t * t / 16, smem, s>>>(w, h, sci, ref, sm, rm, has_sat, sat, r, diff,
+                                                                       mask_out, exact_bad, vec);
+    DGPU_LAUNCH("k_mask");
+  };
+  if (static_cast<int64_t>(ceil_div(w, 64)) * ceil_div(h, 64) >= 2 * 148 && mask_smem(64, r) <= 100 * 1024)
+    go(k_mask<64>, 64);
+  else
+    go(k_mask<32>, 32);
 }
 
 __global__ void k_mask_fill(int64_t n, const uint8_t* __restrict__ mask,
