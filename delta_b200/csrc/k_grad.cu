@@ -489,15 +489,19 @@ __global__ void __launch_bounds__(256, 2) k_adjoint_f(AdjRefArgs a, int n_max) {
       const float* g = gy + ny * KSP;
 #pragma unroll
       for (int j0 = 0; j0 < KSP; j0 += 8) {
+        const int nt = j0 + 8 < KSP ? 8 : a.ks - j0;  // taps of this block (the last: the rest are zeros)
         float2 v[15];
 #pragma unroll
-        for (int t = 0; t < 15; ++t) v[t] = *reinterpret_cast<const float2*>(col + (j0 + t) * kArCols);
+        for (int t = 0; t < 15; ++t)
+          if (t < 7 + nt) v[t] = *reinterpret_cast<const float2*>(col + (j0 + t) * kArCols);
         const float4 ka = *reinterpret_cast<const float4*>(g + j0), kb = *reinterpret_cast<const float4*>(g + j0 + 4);
         const float kv[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj)
+        for (int jj = 0; jj < 8; ++jj) {
+          if (jj >= nt) break;
 #pragma unroll
           for (int i = 0; i < 8; ++i) acc[i] = __ffma2_rn(make_float2(kv[jj], kv[jj]), v[i + jj], acc[i]);
+        }
       }
     }
     // (the x pass of the previous nx finished reading ys before this nx's first barrier)
@@ -520,10 +524,13 @@ __global__ void __launch_bounds__(256, 2) k_adjoint_f(AdjRefArgs a, int n_max) {
         const float4 ka = *reinterpret_cast<const float4*>(gx + nx * KSP + j0);
         const float4 kb = *reinterpret_cast<const float4*>(gx + nx * KSP + j0 + 4);
         const float kv[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
+        const int nt = j0 + 8 < KSP ? 8 : a.ks - j0;
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj)
+        for (int jj = 0; jj < 8; ++jj) {
+          if (jj >= nt) break;
 #pragma unroll
           for (int i = 0; i < 8; ++i) out[n][i] = __fmaf_rn(kv[jj], v[i + jj], out[n][i]);
+        }
       }
     }
   }

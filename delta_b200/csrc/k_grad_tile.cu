@@ -127,6 +127,7 @@ __global__ void __launch_bounds__(kThreads, GRAD ? 1 : 2) k_chi2_f(Chi2Args a, i
     float2 s0 = row[0], s1 = row[1];
 #pragma unroll
     for (int j0 = 0; j0 < KSP; j0 += 2) {
+      if (j0 > KSP - 8 && j0 >= ks) break;  // zero taps: the same for every thread
       float2 p0 = s0, p1 = s1;
       if (j0 > 0) {
         p1 = s0;
@@ -235,10 +236,12 @@ __global__ void __launch_bounds__(kThreads, GRAD ? 1 : 2) k_chi2_f(Chi2Args a, i
       }
 #pragma unroll
       for (int j0 = 0; j0 < KSP; j0 += 8) {
-        float2 v[R + 7];  // v[t] = x-sum row base - j0 - 7 + t
+        const int nt = j0 + 8 < KSP ? 8 : ks - j0;  // taps of this block (the last: the rest are zeros)
+        float2 v[R + 7];                            // v[t] = x-sum row base - j0 - 7 + t
         const float2* vb = col + (base - j0 - 7) * (kTW * V / 2);
 #pragma unroll
-        for (int t = 0; t < R + 7; ++t) v[t] = vb[t * (kTW * V / 2)];
+        for (int t = 0; t < R + 7; ++t)
+          if (t >= 8 - nt) v[t] = vb[t * (kTW * V / 2)];
         const float4 ka = *reinterpret_cast<const float4*>(g0 + j0), kb = *reinterpret_cast<const float4*>(g0 + j0 + 4);
         const float kv[8] = {ka.x, ka.y, ka.z, ka.w, kb.x, kb.y, kb.z, kb.w};
         float dv[8] = {};
@@ -249,12 +252,14 @@ __global__ void __launch_bounds__(kThreads, GRAD ? 1 : 2) k_chi2_f(Chi2Args a, i
           dv[4] = db.x, dv[5] = db.y, dv[6] = db.z, dv[7] = db.w;
         }
 #pragma unroll
-        for (int jj = 0; jj < 8; ++jj)
+        for (int jj = 0; jj < 8; ++jj) {
+          if (jj >= nt) break;
 #pragma unroll
           for (int i = 0; i < R; ++i) {
             cc[i] = __ffma2_rn(make_float2(kv[jj], kv[jj]), v[i - jj + 7], cc[i]);
             if (GRAD) cy[i] = __fmaf_rn(dv[jj], v[i - jj + 7].x, cy[i]);
           }
+        }
       }
       float f[R][COLS];
       fields_of(c, f);

@@ -25,11 +25,11 @@
 
 namespace dgpu {
 
-constexpr int kMfR = 8;                 // output rows per thread
+constexpr int kMfR = 4;                 // output rows per thread
 constexpr int kMfC = 8;                 // output columns per thread
-constexpr int kMfTX = 16, kMfTY = 16;   // threads per CTA along x, y
-constexpr int kMfBW = kMfTX * kMfC;     // tile width (128)
-constexpr int kMfBH = kMfTY * kMfR;     // tile height (128)
+constexpr int kMfTX = 8, kMfTY = 16;    // threads per CTA along x, y
+constexpr int kMfBW = kMfTX * kMfC;     // tile width (64)
+constexpr int kMfBH = kMfTY * kMfR;     // tile height (64)
 // Tile of the generic kernel (64 x 32, one column of 8 rows per thread).
 constexpr int kMfTW = 64;
 constexpr int kMfTH = 32;
@@ -41,88 +41,107 @@ struct MfGeom {
   static constexpr int SEG4 = (kMfC + PS - 1 + 3) / 4;      // 16-byte loads per window row per thread
   static constexpr int WW = kMfBW - kMfC + 4 * SEG4;        // staged window width (floats, multiple of 4)
   static constexpr int WH = kMfBH + PS - 1;                 // staged window height
-  static constexpr int TS = (PS + 3) & ~3;                  // tap row stride
-  static constexpr size_t smem = sizeof(float) * (static_cast<size_t>(WH) * WW + static_cast<size_t>(PS) * TS);
+  static constexpr int TS = (PS + 1) & ~1;                  // tap row stride (pairs)
+  static constexpr size_t smem = sizeof(float) * (static_cast<size_t>(WH) * WW + 2 * static_cast<size_t>(PS) * TS);
 };
 
 template <int PS>
-__global__ void __launch_bounds__(kMfTX * kMfTY, 2)
+__global__ void __launch_bounds__(kMfTX * kMfTY, 4)
 k_matched_filter_t(int w, int h, const float* __restrict__ img, const float* __restrict__ var,
                    const float* __restrict__ psf, float sumpsf2, float* __restrict__ out, int* __restrict__ nf_count,
                    int* __restrict__ nf_tiles) {
   using G = MfGeom<PS>;
   extern __shared__ __align__(16) float msm[];
   float* win = msm;                  // WH x WW
-  float* tap = win + G::WH * G::WW;  // PS x TS, zero padded
+  float2* tap = reinterpret_cast<float2*>(win + G::WH * G::WW);  // PS x TS taps as (k, k), zero padded
   const int bx = blockIdx.x * kMfBW, by = blockIdx.y * kMfBH;
   const int tid = threadIdx.x;
   for (int i = tid; i < PS * G::TS; i += blockDim.x) {
     const int r = i / G::TS, c = i - r * G::TS;
-    tap[i] = c < PS ? __ldg(psf + r * PS + c) : 0.0f;
+    const float k = c < PS ? __ldg(psf + r * PS + c) : 0.0f;
+    tap[i] = make_float2(k, k);
   }
   int finite = 1;
-  for (int i = tid; i < G::WH * G::WW; i += blockDim.x) {
-    const int r = i / G::WW, c = i - r * G::WW;
-    const int gy = by - G::R + r, gx = bx - G::R + c;
-    const float v = (gy < 0 || gy >= h || gx < 0 || gx >= w) ? 0.0f : __ldg(img + static_cast<size_t>(gy) * w + gx);
-    finite &= isfinite(v) ? 1 : 0;
-    win[i] = v;
-  }
+  constexpr int kRows = 8;  // rows of a warp in flight together
+  constexpr int kWarps = kMfTX * kMfTY / 32;
+  for (int r0 = tid >> 5; r0 < G::WH; r0 += kWarps * kRows)
+    for (int c = tid & 31; c < G::WW; c += 32) {
+      const int gx = bx - G::R + c;
+      const bool xin = gx >= 0 && gx < w;
+      float v[kRows];
+#pragma unroll
+      for (int u = 0; u < kRows; ++u) {
+        const int r = r0 + kWarps * u, gy = by - G::R + r;
+        v[u] = (xin && r < G::WH && gy >= 0 && gy < h) ? __ldg(img + static_cast<size_t>(gy) * w + gx) : 0.0f;
+      }
+#pragma unroll
+      for (int u = 0; u < kRows; ++u) {
+        const int r = r0 + kWarps * u;
+        if (r >= G::WH) break;
+        finite &= isfinite(v[u]) ? 1 : 0;
+        win[r * G::WW + c] = v[u];
+      }
+    }
   if (!__syncthreads_and(finite)) {
     if (tid == 0) nf_tiles[atomicAdd(nf_count, 1)] = blockIdx.y * gridDim.x + blockIdx.x;
     return;
   }
   const int c0 = (tid % kMfTX) * kMfC, r0 = (tid / kMfTX) * kMfR;
-  float acc[kMfR][kMfC];
+  float2 acc[kMfR][kMfC / 2];
 #pragma unroll
   for (int i = 0; i < kMfR; ++i)
 #pragma unroll
-    for (int c = 0; c < kMfC; ++c) acc[i][c] = 0.0f;
+    for (int c = 0; c < kMfC / 2; ++c) acc[i][c] = make_float2(0.0f, 0.0f);
 #pragma unroll 1
   for (int wr = 0; wr < kMfR + PS - 1; ++wr) {
-    float seg[4 * G::SEG4];
+    // The row's values as pairs from even and from odd columns on.
+    float2 even[2 * G::SEG4], odd[2 * G::SEG4];
     const float4* src = reinterpret_cast<const float4*>(win + (r0 + wr) * G::WW + c0);
 #pragma unroll
     for (int k = 0; k < G::SEG4; ++k) {
       const float4 q = src[k];
-      seg[4 * k] = q.x;
-      seg[4 * k + 1] = q.y;
-      seg[4 * k + 2] = q.z;
-      seg[4 * k + 3] = q.w;
+      even[2 * k] = make_float2(q.x, q.y);
+      even[2 * k + 1] = make_float2(q.z, q.w);
     }
+#pragma unroll
+    for (int k = 0; k + 1 < 2 * G::SEG4; ++k) odd[k] = make_float2(even[k].y, even[k + 1].x);
 #pragma unroll
     for (int i = 0; i < kMfR; ++i) {
       const int ly = wr - i;
       if (ly < 0 || ly >= PS) continue;  // the same for every thread
-      float t[G::TS];
-      const float4* tp = reinterpret_cast<const float4*>(tap + ly * G::TS);
+      const float2* tp = tap + ly * G::TS;
 #pragma unroll
-      for (int k = 0; k < G::TS / 4; ++k) {
-        const float4 q = tp[k];
-        t[4 * k] = q.x;
-        t[4 * k + 1] = q.y;
-        t[4 * k + 2] = q.z;
-        t[4 * k + 3] = q.w;
+      for (int lx = 0; lx < PS; lx += 2) {
+        const float4 q = *reinterpret_cast<const float4*>(tp + lx);
+#pragma unroll
+        for (int c = 0; c < kMfC / 2; ++c) acc[i][c] = __ffma2_rn(make_float2(q.x, q.y), even[c + lx / 2], acc[i][c]);
+        if (lx + 1 < PS)
+#pragma unroll
+          for (int c = 0; c < kMfC / 2; ++c) acc[i][c] = __ffma2_rn(make_float2(q.z, q.w), odd[c + lx / 2], acc[i][c]);
       }
-#pragma unroll
-      for (int lx = 0; lx < PS; ++lx)
-#pragma unroll
-        for (int c = 0; c < kMfC; ++c) acc[i][c] = __fmaf_rn(t[lx], seg[c + lx], acc[i][c]);
     }
   }
+  // Rows of eight outputs that start on a 16-byte boundary move four at a time.
+  const bool whole = (w & 3) == 0 && bx + c0 + kMfC <= w &&
+                     ((reinterpret_cast<uintptr_t>(var) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  auto score = [&](float a, float v) { return v > 0.0f ? __fdiv_rn(a, __fsqrt_rn(v * sumpsf2)) : 0.0f; };
 #pragma unroll
   for (int i = 0; i < kMfR; ++i) {
     const int y = by + r0 + i;
     if (y >= h) break;
+    const size_t o = static_cast<size_t>(y) * w + bx + c0;
+    if (whole) {
 #pragma unroll
-    for (int c = 0; c < kMfC; ++c) {
-      const int x = bx + c0 + c;
-      if (x < w) {
-        const size_t o = static_cast<size_t>(y) * w + x;
-        const float v = __ldg(var + o);
-        out[o] = v > 0.0f ? __fdiv_rn(acc[i][c], __fsqrt_rn(v * sumpsf2)) : 0.0f;
+      for (int c = 0; c < kMfC; c += 4) {
+        const float4 v = __ldg(reinterpret_cast<const float4*>(var + o + c));
+        const float2 a = acc[i][c / 2], b = acc[i][c / 2 + 1];
+        *reinterpret_cast<float4*>(out + o + c) = make_float4(score(a.x, v.x), score(a.y, v.y), score(b.x, v.z), score(b.y, v.w));
       }
+      continue;
     }
+#pragma unroll
+    for (int c = 0; c < kMfC; ++c)
+      if (bx + c0 + c < w) out[o + c] = score((c & 1) ? acc[i][c / 2].y : acc[i][c / 2].x, __ldg(var + o + c));
   }
 }
 
