@@ -147,7 +147,7 @@ struct Engine {
     w.ok = reinterpret_cast<int*>(w.lam + nsys);
     w.midx = w.ok + nsys;
     w.ridx = w.midx + nsys;
-    w.partial = static_cast<double*>(c.slot(kSlotFft2, sizeof(double) * 16 * std::max(nsys, 1)));
+    w.partial = static_cast<double*>(c.slot(kSlotFft2, sizeof(double) * 8 * std::max(nsys, 1)));
     return w;
   }
 

@@ -76,7 +76,7 @@ struct SolveBatch {
   double* edf = nullptr;            // nsys
   int* ok = nullptr;                // nsys: 1 Cholesky, 2 LDLT fallback, 0 failed
   unsigned* status = nullptr;
-  double* partial = nullptr;        // nsys x 16 per-rank trace partials
+  double* partial = nullptr;        // nsys x 8 per-rank trace partials
   // 0: no degrees of freedom wanted (edf stays unset): the rows F^T are not
   // appended, which halves the work. r is then 0 for the workspace too.
   int want_edf = 1;

@@ -116,8 +116,6 @@ struct Context {
   };
   std::vector<PendingStage> pending;
   bool timing_enabled = false;
-  // Do clusters of 16 CTAs of the solver fit on the device (-1: not asked yet)?
-  int solve_ranks16 = -1;
   // Catalog results of the last dgpu_build_catalog (host copies).
   std::vector<double> cat_d;    // 12 double columns x n
   std::vector<int32_t> cat_i;   // 3 int32 columns x n
