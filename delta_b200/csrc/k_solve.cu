@@ -20,8 +20,8 @@
 //             meanwhile updates and factors the next diagonal tile (one-tile
 //             look-ahead, LDL^T with the tile's rows in registers).
 // The workspace is tile-major (each tile one contiguous block with the
-// shared-memory row stride), so tile operands are staged by double-buffered
-// single bulk async copies completing on an mbarrier; products run on the
+// shared-memory row stride), so tile operands are staged by single bulk async
+// copies completing on an mbarrier, two jobs ahead; products run on the
 // FP64 tensor cores (mma.sync m8n8k4). A is never assembled: M, converted to
 // tiles once per distinct matrix, is read at a tile's first touch and the
 // penalty added there; E is generated at its first touch. theta = L^-T y by back
@@ -67,12 +67,16 @@ size_t solve_work_doubles(int P, int nf, int r, int nsys, int nm) {
 }
 __host__ __device__ __forceinline__ int tri_index(int ti, int tj) { return ti * (ti + 1) / 2 + tj; }
 
+// Job buffers: two jobs are in flight while a third computes, and two CTAs still fit
+// an SM (102 KB each).
+constexpr int kBufs = 3;
+
 struct SolveSmem {
-  double op[2][3][kTS];  // double-buffered job operands: C (updated), left, right
+  double op[kBufs][3][kTS];  // job operands: C (updated), left, right
   double d[kTS];         // Dinv_j in the panel phase; the diagonal tile in the trailing phase
   double v[1024];        // y / theta in the back substitution
   double red[kSolveThreads];
-  uint64_t bar[3];       // mbarriers: job buffers 0 and 1, the diagonal tile
+  uint64_t bar[kBufs + 1];  // mbarriers: the job buffers, the diagonal tile
 };
 
 constexpr long long kSolveSpin = 1ll << 22;  // bounded mbarrier wait (iterations)
@@ -156,10 +160,12 @@ __device__ __forceinline__ void cluster_step(const cg::cluster_group& cl) {
 }
 
 // Run this rank's jobs first, next(first), ... (< nt) with the operands of the
-// next job in flight while the current one computes. load(buf, t, bar, tx)
+// next two jobs in flight while the current one computes. load(buf, t, bar, tx)
 // stages job t into the three tiles of buf (bulk copies counted in tx,
 // generated values stored directly); compute(buf, t) uses them. par holds
-// the expected phase parity of each mbarrier.
+// the expected phase parity of each mbarrier. One CTA barrier per job: behind it the
+// previous job is done everywhere, so its buffer takes the job after next. The caller
+// passes a barrier before it uses the buffers again.
 template <class Next, class Load, class Compute>
 __device__ __forceinline__ void run_jobs(SolveSmem& S, unsigned& par, unsigned* status, int first, int nt, Next next,
                                          Load load, Compute compute) {
@@ -171,18 +177,19 @@ __device__ __forceinline__ void run_jobs(SolveSmem& S, unsigned& par, unsigned* 
     load(S.op[b], t, &S.bar[b], tx);
     if (w0) mbar_arrive_tx(&S.bar[b], tx);
   };
-  int cur = 0;
-  issue(0, first);
-  for (int t = first; t < nt;) {
-    const int tn = next(t);
-    if (tn < nt) issue(cur ^ 1, tn);
+  int cur = 0, t = first, t1 = next(first);
+  issue(0, t);
+  if (t1 < nt) issue(1, t1);
+  while (t < nt) {
     if (!mbar_wait(&S.bar[cur], (par >> cur) & 1u)) set_status(status, kStatusLoopLimit);
     par ^= 1u << cur;
     __syncthreads();
+    const int t2 = next(t1);
+    if (t2 < nt) issue(cur == 0 ? 2 : cur - 1, t2);  // the previous job's buffer
     compute(S.op[cur], t);
-    __syncthreads();
-    cur ^= 1;
-    t = tn;
+    cur = cur == 2 ? 0 : cur + 1;
+    t = t1;
+    t1 = t2;
   }
 }
 
@@ -199,28 +206,27 @@ __device__ __forceinline__ double rcp_newton(double d) {
 }
 
 // Right-looking LDL^T of N columns held in registers, lane = row: the pivot
-// of column q is on lane base + q; column q is broadcast through col (32
-// doubles of shared memory). Afterwards a[q] holds the unit factor l_rq
+// of column q is on lane base + q; column q is broadcast through col (2 x 32 doubles
+// of shared memory, used in turn, so one warp barrier a column). Rows above the pivot
+// are updated too: nothing reads them. Afterwards a[q] holds the unit factor l_rq
 // below the pivot, the pivot d_q on it and zero above.
 template <int N>
 __device__ __forceinline__ void ldl_cols(double (&a)[N], int lane, int base, int& bad, double* col) {
 #pragma unroll
   for (int q = 0; q < N; ++q) {
+    double* cq = col + (q & 1) * kT;
     double d = __shfl_sync(0xffffffffu, a[q], base + q);
-    if (!(d > 0.0)) {
-      bad = 1;
-      d = 1.0;
-    }
     const double u = a[q];
-    col[lane] = u;
-    const double l = u * rcp_newton(d);
+    cq[lane] = u;
+    double rd = rcp_newton(d);
+    if (!(d > 0.0)) {  // beside the reciprocal, not before it
+      bad = 1;
+      d = rd = 1.0;
+    }
+    const double l = u * rd;
     __syncwarp();
 #pragma unroll
-    for (int m = q + 1; m < N; ++m) {
-      const double um = col[base + m];
-      if (lane >= base + m) a[m] = fma(-l, um, a[m]);
-    }
-    __syncwarp();
+    for (int m = q + 1; m < N; ++m) a[m] = fma(-l, cq[base + m], a[m]);
     a[q] = lane > base + q ? l : (lane == base + q ? d : 0.0);
   }
 }
@@ -240,7 +246,9 @@ __device__ __noinline__ void factor_tile(SolveSmem& S, double* gL, double* gD, i
   double* sd = S.op[1][1];        // sqrt(D)
   double* isd = S.op[1][1] + kT;  // 1 / sqrt(D)
   double* col = S.op[1][1] + 2 * kT;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // The warp's index as a value the compiler knows to be uniform: behind a branch on
+  // threadIdx.x / 32 it must assume a diverged warp at each shuffle and warp barrier.
+  const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;
   int bad = 0;
   if (warp == 0) {
     const double* t = S.d + lane * kLd;
@@ -437,22 +445,22 @@ __global__ void __launch_bounds__(kSolveThreads, 2) k_solve_cluster(SolveBatch b
   __shared__ int s_estart[kMaxTiles];
   if (tid == 0) {
     s_ok = 1;
-    for (int q = 0; q < 3; ++q)
+    for (int q = 0; q <= kBufs; ++q)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 32;" ::"r"(saddr(&S.bar[q])) : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   for (int c = tid; c < ne; c += blockDim.x) s_estart[c] = e_start(c, y.r, y.k);
   __syncthreads();
-  unsigned par = 0;  // expected phase parity of S.bar[0..2]
+  unsigned par = 0;  // expected phase parity of each S.bar
   const bool w0 = tid < 32;
-  // Stage the diagonal tile job on S.bar[2]: stage(bar, tx) issues it.
+  // Stage the diagonal tile job on its mbarrier: stage(bar, tx) issues it.
   auto stage_diag = [&](auto stage) {
     if (w0) fence_proxy_async();
     uint32_t tx = 0;
-    stage(&S.bar[2], tx);
-    if (w0) mbar_arrive_tx(&S.bar[2], tx);
-    if (!mbar_wait(&S.bar[2], (par >> 2) & 1u)) set_status(b.status, kStatusLoopLimit);
-    par ^= 4u;
+    stage(&S.bar[kBufs], tx);
+    if (w0) mbar_arrive_tx(&S.bar[kBufs], tx);
+    if (!mbar_wait(&S.bar[kBufs], (par >> kBufs) & 1u)) set_status(b.status, kStatusLoopLimit);
+    par ^= 1u << kBufs;
     __syncthreads();
   };
 
