@@ -68,7 +68,10 @@ size_t solve_work_doubles(int P, int nf, int r, int nsys, int nm) {
 __host__ __device__ __forceinline__ int tri_index(int ti, int tj) { return ti * (ti + 1) / 2 + tj; }
 
 // Job buffers: two jobs are in flight while a third computes, and two CTAs still fit
-// an SM (102 KB each).
+// an SM (102 KB each). With two buffers and two CTA barriers a job, and pivot warps not
+// known to be converged: 25 systems of 150 unknowns 84 us, now 69; 10 or 5 of 725 501,
+// now 477; one of 725 with its penalty rows 783, now 740; 65 of 725 1346 and 1355 (bound
+// by the tiles' L2 traffic, four per product).
 constexpr int kBufs = 3;
 
 struct SolveSmem {
