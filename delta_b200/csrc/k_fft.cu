@@ -21,6 +21,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <type_traits>
 #include <cmath>
 
 #include "dev_common.cuh"
@@ -244,16 +245,29 @@ __host__ __device__ __forceinline__ int fft_ls(int m, bool transposed) {
   return transposed ? m + 1 : m;
 }
 
-// Dispatch: four-step for 128 / 256, radix-2 otherwise. SIGN is the
-// direction of `tw` (-1 forward, +1 inverse), known at every call site.
-template <int SIGN>
+// Lines of m points: four-step where M = m is 128 or 256, radix-2 where M is 0 (any
+// other m). SIGN is the direction of `tw` (-1 forward, +1 inverse). M is fixed for a
+// whole kernel (fft_kind): one kernel that held every transform took the registers
+// of the largest, which left k_cols one CTA per SM and k_rows_fwd, k_rows_inv two
+// (136, 98 and 99 registers, now 38, 30 and 38 for radix 2): decorrelation of 2048 x
+// 2048 took 1.86 ms in blocks of 32 and 1.02 ms in blocks of 128, now 0.99 and 0.62.
+template <int SIGN, int M>
 __device__ __forceinline__ void fft_lines(float2* x, int L, int m, int logm, const float2* tw, int ls) {
-  if (m == 256)
-    fft_lines_4step_d<256, SIGN>(x, L, ls, tw);
-  else if (m == 128)
-    fft_lines_4step_d<128, SIGN>(x, L, ls, tw);
+  if constexpr (M != 0)
+    fft_lines_4step_d<M, SIGN>(x, L, ls, tw);
   else
     smem_fft(x, L, m, logm, tw, ls);
+}
+
+// f(std::integral_constant<int, M>) for lines of m points.
+template <class F>
+static void fft_kind(int m, F&& f) {
+  if (m == 256)
+    f(std::integral_constant<int, 256>{});
+  else if (m == 128)
+    f(std::integral_constant<int, 128>{});
+  else
+    f(std::integral_constant<int, 0>{});
 }
 
 __device__ __forceinline__ int reflect_clamp(int s, int len) {
@@ -266,6 +280,7 @@ __device__ __forceinline__ int reflect_clamp(int s, int len) {
 // Row pass (r2c). mode 0: block rows of the frame, reflect padded
 // (src/noise.cpp:392-406); mode 1: rows of a dense n x n real image per item.
 // ---------------------------------------------------------------------------
+template <int M>
 __global__ void __launch_bounds__(256)
 k_rows_fwd(FftGeom G, int mode, const float* __restrict__ src, int w, int h, const int* __restrict__ oxs,
            const int* __restrict__ oys, int nox, float2* __restrict__ spec) {
@@ -310,7 +325,7 @@ k_rows_fwd(FftGeom G, int mode, const float* __restrict__ src, int w, int h, con
     z[rr * zl + j] = make_float2(a, b);
   }
   __syncthreads();
-  fft_lines<-1>(z, rows, hn, G.logn - 1, tw, zl);
+  fft_lines<-1, M>(z, rows, hn, G.logn - 1, tw, zl);
   for (int e = threadIdx.x; e < rows * nb; e += blockDim.x) {
     const int rr = e / nb, k = e - rr * nb;
     const float2 zk = z[rr * zl + (k % hn)];
@@ -326,6 +341,7 @@ k_rows_fwd(FftGeom G, int mode, const float* __restrict__ src, int w, int h, con
 // Column pass. mode 0: forward, multiply by the block filter, inverse (in
 // place); mode 1: forward and write |X|^2 in FP64 (kernel-power cache).
 // ---------------------------------------------------------------------------
+template <int M>
 __global__ void __launch_bounds__(256)
 k_cols(FftGeom G, int mode, float2* __restrict__ spec, const double* __restrict__ cell_power,
        const double* __restrict__ cell_sumk2, const int* __restrict__ block_cell, const double* __restrict__ vsr,
@@ -352,7 +368,7 @@ k_cols(FftGeom G, int mode, float2* __restrict__ spec, const double* __restrict_
       x[cc * ls + row] = cc < ncol ? sp[static_cast<size_t>(row) * nb + c0 + cc] : make_float2(0.f, 0.f);
     }
     __syncthreads();
-    fft_lines<-1>(x, C, n, G.logn, tw, ls);
+    fft_lines<-1, M>(x, C, n, G.logn, tw, ls);
   }
   if (mode == 1) {
     for (int e = threadIdx.x; e < C * n; e += blockDim.x) {
@@ -384,7 +400,7 @@ k_cols(FftGeom G, int mode, float2* __restrict__ spec, const double* __restrict_
   else
     make_twiddles(tw, n, +1);
   __syncthreads();
-  fft_lines<1>(x, C, n, G.logn, tw, ls);
+  fft_lines<1, M>(x, C, n, G.logn, tw, ls);
   for (int e = threadIdx.x; e < C * n; e += blockDim.x) {
     const int row = e / C, cc = e - row * C;
     if (cc < ncol) sp[static_cast<size_t>(row) * nb + c0 + cc] = x[cc * ls + row];
@@ -396,6 +412,7 @@ k_cols(FftGeom G, int mode, float2* __restrict__ spec, const double* __restrict_
 // acc / var_acc (src/noise.cpp:430-452); mode 1: plain store x 1/n^2 into a
 // dense n x n real output per item.
 // ---------------------------------------------------------------------------
+template <int M>
 __global__ void __launch_bounds__(256)
 k_rows_inv(FftGeom G, int mode, const float2* __restrict__ spec, const int* __restrict__ items, int w, int h,
            const int* __restrict__ oxs, const int* __restrict__ oys, int nox, const double* __restrict__ hwin,
@@ -437,7 +454,7 @@ k_rows_inv(FftGeom G, int mode, const float2* __restrict__ spec, const int* __re
     z[rr * zl + k] = make_float2(e2.x - o2.y, e2.y + o2.x);  // 2E + i 2O
   }
   __syncthreads();
-  fft_lines<1>(z, rows, hn, G.logn - 1, tw, zl);
+  fft_lines<1, M>(z, rows, hn, G.logn - 1, tw, zl);
   const float inv_n2 = 1.0f / static_cast<float>(static_cast<size_t>(n) * n);
   if (mode == 2) {  // raw real block output for the overlap-add gather (dense_out: item x n x n)
     for (int e = threadIdx.x; e < rows * n; e += blockDim.x) {
@@ -947,13 +964,13 @@ __host__ __device__ constexpr int cp_lines(int n) {  // float2 of the column lin
 // is that of the passes it replaces (k_local_kernels, k_rows_fwd, k_cols), which
 // wrote and read the dense image and the whole spectrum: 141 us at 465 cells of 256 x
 // 256, where they took 426 us. Bound as k_block_filter is, by the line transforms.
+template <int N>
 __global__ void __launch_bounds__(256, 3)
 k_cell_power(FftGeom G, TpsDev t, const double* __restrict__ theta, int nc, const float* __restrict__ phi, int ks,
              const double* __restrict__ centres, double* __restrict__ sumk2, double* __restrict__ power) {
   extern __shared__ __align__(16) float2 fsm2[];
-  const int n = G.n, hn = n / 2, nb = hn + 1, r = ks / 2;
-  constexpr int C = kCpCols;
-  const int zl = fft_ls(hn, false), ls = fft_ls(n, true);
+  constexpr int n = N, hn = n / 2, nb = hn + 1, C = kCpCols;
+  const int r = ks / 2, zl = fft_ls(hn, false), ls = fft_ls(n, true);
   float2* x = fsm2;              // C x ls column lines; before them cell_kernel's scratch
   float2* z = x + cp_lines(n);   // ks x zl row lines
   CellShared& S = *reinterpret_cast<CellShared*>(x);
@@ -973,7 +990,7 @@ k_cell_power(FftGeom G, TpsDev t, const double* __restrict__ theta, int nc, cons
     z[ky * zl + j] = make_float2(k0 < ks ? kk[ky * ks + k0] : 0.0f, k1 < ks ? kk[ky * ks + k1] : 0.0f);
   }
   __syncthreads();
-  fft_lines<-1>(z, ks, hn, G.logn - 1, twh, zl);
+  fft_lines<-1, hn == 128 ? 128 : 0>(z, ks, hn, G.logn - 1, twh, zl);
   for (int c0 = blockIdx.y * C; c0 < nb; c0 += gridDim.y * C) {
     const int ncol = min(C, nb - c0);
     for (int e = threadIdx.x; e < C * n; e += blockDim.x) {
@@ -991,7 +1008,7 @@ k_cell_power(FftGeom G, TpsDev t, const double* __restrict__ theta, int nc, cons
       x[cc * ls + row] = X;
     }
     __syncthreads();
-    fft_lines<-1>(x, ncol, n, G.logn, tw, ls);
+    fft_lines<-1, N>(x, ncol, n, G.logn, tw, ls);
     for (int e = threadIdx.x; e < C * n; e += blockDim.x) {
       const int row = e / C, cc = e - row * C;
       if (cc >= ncol) continue;
@@ -1053,18 +1070,24 @@ FftGeom make_fft_geom(int n) {
 void launch_rows_fwd(cudaStream_t s, const FftGeom& g, int mode, int nitems, const float* src, int w, int h,
                      const int* oxs, const int* oys, int nox, float2* spec) {
   const size_t smem = rows_smem(g);
-  ensure_dynamic_smem(reinterpret_cast<const void*>(k_rows_fwd), smem);
   dim3 grid(nitems, (g.n + g.rows_per_cta - 1) / g.rows_per_cta);
-  k_rows_fwd<<<grid, 256, smem, s>>>(g, mode, src, w, h, oxs, oys, nox, spec);
+  fft_kind(g.n / 2, [&](auto m) {
+    auto kern = k_rows_fwd<decltype(m)::value>;
+    ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
+    kern<<<grid, 256, smem, s>>>(g, mode, src, w, h, oxs, oys, nox, spec);
+  });
   DGPU_LAUNCH("k_rows_fwd");
 }
 
 void launch_cols(cudaStream_t s, const FftGeom& g, int mode, int nitems, float2* spec, const double* cell_power,
                  const double* cell_sumk2, const int* block_cell, const double* vsr, double* power_out) {
   const size_t smem = cols_smem(g);
-  ensure_dynamic_smem(reinterpret_cast<const void*>(k_cols), smem);
   dim3 grid(nitems, (g.n / 2 + 1 + g.cols_per_cta - 1) / g.cols_per_cta);
-  k_cols<<<grid, 256, smem, s>>>(g, mode, spec, cell_power, cell_sumk2, block_cell, vsr, power_out);
+  fft_kind(g.n, [&](auto m) {
+    auto kern = k_cols<decltype(m)::value>;
+    ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
+    kern<<<grid, 256, smem, s>>>(g, mode, spec, cell_power, cell_sumk2, block_cell, vsr, power_out);
+  });
   DGPU_LAUNCH("k_cols");
 }
 
@@ -1073,10 +1096,13 @@ void launch_rows_inv(cudaStream_t s, const FftGeom& g, int mode, int nitems, con
                      const double* cell_sumk2, const int* block_cell, float* acc, float* var_acc, float* dense_out) {
   if (nitems == 0) return;
   const size_t smem = rows_smem(g);
-  ensure_dynamic_smem(reinterpret_cast<const void*>(k_rows_inv), smem);
   dim3 grid(nitems, (g.n + g.rows_per_cta - 1) / g.rows_per_cta);
-  k_rows_inv<<<grid, 256, smem, s>>>(g, mode, spec, items, w, h, oxs, oys, nox, hwin, vsr, cell_sumk2, block_cell,
-                                     acc, var_acc, dense_out);
+  fft_kind(g.n / 2, [&](auto m) {
+    auto kern = k_rows_inv<decltype(m)::value>;
+    ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
+    kern<<<grid, 256, smem, s>>>(g, mode, spec, items, w, h, oxs, oys, nox, hwin, vsr, cell_sumk2, block_cell, acc,
+                                 var_acc, dense_out);
+  });
   DGPU_LAUNCH("k_rows_inv");
 }
 
@@ -1122,8 +1148,9 @@ void launch_cell_power(cudaStream_t s, const FftGeom& g, int ncell, const TpsDev
   const int groups = (g.n / 2 + 1 + kCpCols - 1) / kCpCols;
   const int split = std::min(groups, std::max(1, 148 * 4 / std::max(ncell, 1)));
   const size_t smem = cell_power_smem(g, ks);
-  ensure_dynamic_smem(reinterpret_cast<const void*>(k_cell_power), smem);
-  k_cell_power<<<dim3(ncell, split), 256, smem, s>>>(g, t, theta, nc, phi, ks, centres, sumk2, power);
+  auto kern = g.n == 256 ? k_cell_power<256> : k_cell_power<128>;
+  ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
+  kern<<<dim3(ncell, split), 256, smem, s>>>(g, t, theta, nc, phi, ks, centres, sumk2, power);
   DGPU_LAUNCH("k_cell_power");
 }
 
