@@ -885,52 +885,52 @@ constexpr int kCpCols = 16;  // column lines of k_cell_power at a time
 // fields at the cell's representative block centre) into kk (shared), and sum K^2 in
 // FP64 (returned by thread 0). A thread per knot, per coefficient of the point and
 // per field (one thread doing all of them took 54 us at 465 cells); blockDim 256.
+// scratch: cell_scratch(k, nc) doubles of shared memory.
 constexpr int kCellKnots = 1024, kCellFields = 256;
-struct CellShared {
-  double s[kCellKnots];  // thin-plate values at the knots
-  double d[kCellKnots];  // the point's design row
-  double red[256];
-  float an[kCellFields];
-};
-__device__ double cell_kernel(CellShared& S, const TpsDev& t, const double* __restrict__ theta, int nc,
+__host__ __device__ constexpr int cell_scratch(int k, int nc) { return 2 * k + 256 + (nc + 1) / 2; }
+__device__ double cell_kernel(double* scratch, const TpsDev& t, const double* __restrict__ theta, int nc,
                               const float* __restrict__ phi, int ks, double cx, double cy, float* kk) {
   const int k = t.k, nr = k - 3, tid = threadIdx.x;
+  double* s = scratch;     // thin-plate values at the knots
+  double* d = s + k;       // the point's design row
+  double* red = d + k;     // 256
+  float* an = reinterpret_cast<float*>(red + 256);
   const double ux = (cx - t.cx) / t.scale, uy = (cy - t.cy) / t.scale;
   for (int j = tid; j < k; j += blockDim.x) {
     const double dx = ux - t.kn[2 * j], dy = uy - t.kn[2 * j + 1];
     const double r2 = dx * dx + dy * dy;
-    S.s[j] = r2 <= 0.0 ? 0.0 : 0.5 * r2 * log(r2);
+    s[j] = r2 <= 0.0 ? 0.0 : 0.5 * r2 * log(r2);
   }
   __syncthreads();
   for (int m = tid; m < k; m += blockDim.x) {
     double v = m == nr ? 1.0 : m == nr + 1 ? ux : uy;
     if (m < nr) {
       v = 0.0;
-      for (int j = 0; j < k; ++j) v = fma(S.s[j], t.z[j * nr + m], v);
+      for (int j = 0; j < k; ++j) v = fma(s[j], t.z[j * nr + m], v);
     }
-    S.d[m] = v;
+    d[m] = v;
   }
   __syncthreads();
   for (int q = tid; q < nc; q += blockDim.x) {
     double f = 0.0;
-    for (int m = 0; m < k; ++m) f = fma(S.d[m], theta[q * k + m], f);
-    S.an[q] = static_cast<float>(f);
+    for (int m = 0; m < k; ++m) f = fma(d[m], theta[q * k + m], f);
+    an[q] = static_cast<float>(f);
   }
   __syncthreads();
   double part = 0.0;
   for (int i = tid; i < ks * ks; i += blockDim.x) {
     float v = 0.0f;
-    for (int q = 0; q < nc; ++q) v = __fmaf_rn(S.an[q], phi[static_cast<size_t>(q) * ks * ks + i], v);
+    for (int q = 0; q < nc; ++q) v = __fmaf_rn(an[q], phi[static_cast<size_t>(q) * ks * ks + i], v);
     kk[i] = v;
     part = fma(static_cast<double>(v), static_cast<double>(v), part);
   }
-  S.red[tid] = part;
+  red[tid] = part;
   __syncthreads();
   for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if (tid < o) S.red[tid] += S.red[tid + o];
+    if (tid < o) red[tid] += red[tid + o];
     __syncthreads();
   }
-  return S.red[0];
+  return red[0];
 }
 
 // The kernel of each cell and its zero-phase embedding into an n x n real image
@@ -939,10 +939,10 @@ __global__ void __launch_bounds__(256)
 k_local_kernels(FftGeom G, TpsDev t, const double* __restrict__ theta, int nc, const float* __restrict__ phi,
                 int ks, const double* __restrict__ centres, double* __restrict__ sumk2, float* __restrict__ dense,
                 float* __restrict__ kern_out) {
-  extern __shared__ float kk[];
-  __shared__ CellShared S;
+  extern __shared__ __align__(16) double lsm[];
+  float* kk = reinterpret_cast<float*>(lsm + cell_scratch(t.k, nc));  // ks x ks
   const int cell = blockIdx.x, n = G.n, r = ks / 2;
-  const double s2 = cell_kernel(S, t, theta, nc, phi, ks, centres[2 * cell], centres[2 * cell + 1], kk);
+  const double s2 = cell_kernel(lsm, t, theta, nc, phi, ks, centres[2 * cell], centres[2 * cell + 1], kk);
   for (int i = threadIdx.x; i < ks * ks; i += blockDim.x) {
     const int ky = i / ks, kx = i - ky * ks;
     const int gy = ((ky - r) % n + n) % n, gx = ((kx - r) % n + n) % n;
@@ -952,8 +952,8 @@ k_local_kernels(FftGeom G, TpsDev t, const double* __restrict__ theta, int nc, c
   if (threadIdx.x == 0 && sumk2) sumk2[cell] = s2;
 }
 
-__host__ __device__ constexpr int cp_lines(int n) {  // float2 of the column lines
-  const int lines = kCpCols * (n + 17), scratch = static_cast<int>((sizeof(CellShared) + 7) / 8);
+__host__ __device__ constexpr int cp_lines(int n, int k, int nc) {  // float2 of the column lines
+  const int lines = kCpCols * (n + 17), scratch = cell_scratch(k, nc);
   return lines > scratch ? lines : scratch;
 }
 
@@ -972,8 +972,7 @@ k_cell_power(FftGeom G, TpsDev t, const double* __restrict__ theta, int nc, cons
   constexpr int n = N, hn = n / 2, nb = hn + 1, C = kCpCols;
   const int r = ks / 2, zl = fft_ls(hn, false), ls = fft_ls(n, true);
   float2* x = fsm2;              // C x ls column lines; before them cell_kernel's scratch
-  float2* z = x + cp_lines(n);   // ks x zl row lines
-  CellShared& S = *reinterpret_cast<CellShared*>(x);
+  float2* z = x + cp_lines(n, t.k, nc);  // ks x zl row lines
   float2* tw = z + ks * zl;      // n/2
   float2* twh = tw + n / 2;      // hn/2
   float2* split = twh + hn / 2;  // nb
@@ -982,7 +981,7 @@ k_cell_power(FftGeom G, TpsDev t, const double* __restrict__ theta, int nc, cons
   copy_tw(twh, G.tw_tab + tw_off_fwd_hn(n), hn / 2);
   copy_tw(split, G.tw_tab + tw_off_split_fwd(n), nb);
   const int cell = blockIdx.x;
-  const double s2 = cell_kernel(S, t, theta, nc, phi, ks, centres[2 * cell], centres[2 * cell + 1], kk);
+  const double s2 = cell_kernel(reinterpret_cast<double*>(x), t, theta, nc, phi, ks, centres[2 * cell], centres[2 * cell + 1], kk);
   if (threadIdx.x == 0 && blockIdx.y == 0) sumk2[cell] = s2;
   for (int e = threadIdx.x; e < ks * hn; e += blockDim.x) {
     const int ky = e / hn, j = e - ky * hn;
@@ -1121,7 +1120,9 @@ void launch_local_kernels(cudaStream_t s, const FftGeom& g, int ncell, const Tps
                           const float* phi, int ks, const double* centres, double* sumk2, float* dense,
                           float* kern_out) {
   if (t.k > kCellKnots || nc > kCellFields) fail(DGPU_ERR_INVALID, "decorrelate: too many knots or components");
-  const size_t smem = sizeof(float) * static_cast<size_t>(ks) * ks;
+  // Sized by this call: kernels of up to 239 x 239 with up to 64 knots and 66 components.
+  const size_t smem = sizeof(double) * cell_scratch(t.k, nc) + sizeof(float) * static_cast<size_t>(ks) * ks;
+  if (smem > 227 * 1024) fail(DGPU_ERR_INVALID, "decorrelate: kernel radius too large");
   ensure_dynamic_smem(reinterpret_cast<const void*>(k_local_kernels), smem);
   k_local_kernels<<<ncell, 256, smem, s>>>(g, t, theta, nc, phi, ks, centres, sumk2, dense, kern_out);
   DGPU_LAUNCH("k_local_kernels");
@@ -1129,16 +1130,16 @@ void launch_local_kernels(cudaStream_t s, const FftGeom& g, int ncell, const Tps
 
 bool block_filter_fused(const FftGeom& g) { return g.n == kBfN && g.tw_tab != nullptr; }
 
-static size_t cell_power_smem(const FftGeom& g, int ks) {
+static size_t cell_power_smem(const FftGeom& g, int ks, int knots, int nc) {
   const int n = g.n, hn = n / 2;
-  return sizeof(float2) * (static_cast<size_t>(cp_lines(n)) + static_cast<size_t>(ks) * fft_ls(hn, false) +
+  return sizeof(float2) * (static_cast<size_t>(cp_lines(n, knots, nc)) + static_cast<size_t>(ks) * fft_ls(hn, false) +
                            n / 2 + hn / 2 + hn + 1) +
          sizeof(float) * ks * ks;
 }
 bool cell_power_fused(const FftGeom& g, int ks, int knots, int nc) {
   return (g.n == 128 || g.n == 256) && g.tw_tab != nullptr && ks <= g.n / 2 && knots <= kCellKnots &&
          nc <= kCellFields &&
-         cell_power_smem(g, ks) <= 160 * 1024;
+         cell_power_smem(g, ks, knots, nc) <= 160 * 1024;
 }
 void launch_cell_power(cudaStream_t s, const FftGeom& g, int ncell, const TpsDev& t, const double* theta, int nc,
                        const float* phi, int ks, const double* centres, double* sumk2, double* power) {
@@ -1147,7 +1148,7 @@ void launch_cell_power(cudaStream_t s, const FftGeom& g, int ncell, const TpsDev
   // cells: 1, 2, 3, 5 and 9 CTAs each take 141, 153, 149, 146 and 172 us).
   const int groups = (g.n / 2 + 1 + kCpCols - 1) / kCpCols;
   const int split = std::min(groups, std::max(1, 148 * 4 / std::max(ncell, 1)));
-  const size_t smem = cell_power_smem(g, ks);
+  const size_t smem = cell_power_smem(g, ks, t.k, nc);
   auto kern = g.n == 256 ? k_cell_power<256> : k_cell_power<128>;
   ensure_dynamic_smem(reinterpret_cast<const void*>(kern), smem);
   kern<<<dim3(ncell, split), 256, smem, s>>>(g, t, theta, nc, phi, ks, centres, sumk2, power);
