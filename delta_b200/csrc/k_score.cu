@@ -54,7 +54,8 @@ k_matched_filter_t(int w, int h, const float* __restrict__ img, const float* __r
   extern __shared__ __align__(16) float msm[];
   float* win = msm;                  // WH x WW
   float2* tap = reinterpret_cast<float2*>(win + G::WH * G::WW);  // PS x TS taps as (k, k), zero padded
-  const int bx = blockIdx.x * kMfBW, by = blockIdx.y * kMfBH;
+  const int tiles_x = (w + kMfBW - 1) / kMfBW;
+  const int bx = static_cast<int>(blockIdx.x % tiles_x) * kMfBW, by = static_cast<int>(blockIdx.x / tiles_x) * kMfBH;
   const int tid = threadIdx.x;
   for (int i = tid; i < PS * G::TS; i += blockDim.x) {
     const int r = i / G::TS, c = i - r * G::TS;
@@ -83,7 +84,7 @@ k_matched_filter_t(int w, int h, const float* __restrict__ img, const float* __r
       }
     }
   if (!__syncthreads_and(finite)) {
-    if (tid == 0) nf_tiles[atomicAdd(nf_count, 1)] = blockIdx.y * gridDim.x + blockIdx.x;
+    if (tid == 0) nf_tiles[atomicAdd(nf_count, 1)] = blockIdx.x;
     return;
   }
   const int c0 = (tid % kMfTX) * kMfC, r0 = (tid / kMfTX) * kMfR;
@@ -220,8 +221,9 @@ static void launch_mf_t(cudaStream_t s, int w, int h, const float* img, const fl
                         float sumpsf2, float* out, int* nf_buf) {
   auto kern = k_matched_filter_t<PS>;
   ensure_dynamic_smem(reinterpret_cast<const void*>(kern), MfGeom<PS>::smem);
-  dim3 grid(ceil_div(w, kMfBW), ceil_div(h, kMfBH));
-  kern<<<grid, kMfTX * kMfTY, MfGeom<PS>::smem, s>>>(w, h, img, var, psf_dev, sumpsf2, out, nf_buf, nf_buf + 1);
+  // All tiles along x: a grid's y takes 65535 of them, 4194240 rows.
+  const int tiles = ceil_div(w, kMfBW) * ceil_div(h, kMfBH);
+  kern<<<tiles, kMfTX * kMfTY, MfGeom<PS>::smem, s>>>(w, h, img, var, psf_dev, sumpsf2, out, nf_buf, nf_buf + 1);
   DGPU_LAUNCH("k_matched_filter");
 }
 
