@@ -3,16 +3,19 @@
 // score(x) = (sum_u psf(u) D(x+u)) / sqrt(var(x) * sum psf^2), zero-padded,
 // 0 where var <= 0.
 //
-// Common PSF sides (template PS): one CTA of 16 x 16 threads per 128 x 128
-// output tile, each thread an 8 x 8 block of outputs (8 rows of 8 adjacent
-// columns) in registers. The haloed D window and the taps (rows padded to a
-// multiple of 4) are staged in shared memory. The thread walks the window rows
-// of its block: it reads the row's 8 + PS - 1 values once (16-byte vector
-// loads) and, for every output row i whose tap row ly = wr - i is in range,
-// the 17-tap row ly (broadcast vector loads) and applies it to the 8 outputs
-// of that row. Each output therefore accumulates its taps in the reference's
-// (ly, lx) order with fused multiply-adds; the ratio of FMAs to shared loads
-// is about 24 to 1, so the kernel is FP32-FMA-bound.
+// Common PSF sides (template PS): one CTA of 8 x 16 threads per 64 x 64 output tile,
+// each thread a 4 x 8 block of outputs (4 rows of 8 adjacent columns, two columns to a
+// packed multiply-add) in registers. The haloed D window and the taps (rows padded to
+// a multiple of 4) are staged in shared memory. The thread walks the window rows of
+// its block: it reads the row's 8 + PS - 1 values once (16-byte loads), as pairs from
+// even and from odd columns on, and, for every output row i whose tap row ly = wr - i
+// is in range, that tap row (four taps to a broadcast 16-byte load) and applies it to
+// the 8 outputs of that row. Each output therefore accumulates its taps in the
+// reference's (ly, lx) order with fused multiply-adds. Bound by the FP32 pipe and the
+// shared loads beside it (a row of 17 taps: 26 loads for 272 packed multiply-adds, the
+// window's at two wavefronts each). 4096 x 4096, 17 and 21 taps a side: 267 and 363 us;
+// with each tap stored twice, as the pairs use it, 281 and 402 (44 loads for a row of
+// 21 taps); 128 x 128 tiles of scalar multiply-adds 317 and 384.
 //
 // With every staged value finite, a zero tap adds an exact +-0 to a sum that
 // is never -0, so skipping it (as the reference does) and not skipping it give
@@ -41,8 +44,8 @@ struct MfGeom {
   static constexpr int SEG4 = (kMfC + PS - 1 + 3) / 4;      // 16-byte loads per window row per thread
   static constexpr int WW = kMfBW - kMfC + 4 * SEG4;        // staged window width (floats, multiple of 4)
   static constexpr int WH = kMfBH + PS - 1;                 // staged window height
-  static constexpr int TS = (PS + 1) & ~1;                  // tap row stride (pairs)
-  static constexpr size_t smem = sizeof(float) * (static_cast<size_t>(WH) * WW + 2 * static_cast<size_t>(PS) * TS);
+  static constexpr int TS = (PS + 3) & ~3;                  // tap row stride
+  static constexpr size_t smem = sizeof(float) * (static_cast<size_t>(WH) * WW + static_cast<size_t>(PS) * TS);
 };
 
 template <int PS>
@@ -53,14 +56,13 @@ k_matched_filter_t(int w, int h, const float* __restrict__ img, const float* __r
   using G = MfGeom<PS>;
   extern __shared__ __align__(16) float msm[];
   float* win = msm;                  // WH x WW
-  float2* tap = reinterpret_cast<float2*>(win + G::WH * G::WW);  // PS x TS taps as (k, k), zero padded
+  float* tap = win + G::WH * G::WW;  // PS x TS, zero padded
   const int tiles_x = (w + kMfBW - 1) / kMfBW;
   const int bx = static_cast<int>(blockIdx.x % tiles_x) * kMfBW, by = static_cast<int>(blockIdx.x / tiles_x) * kMfBH;
   const int tid = threadIdx.x;
   for (int i = tid; i < PS * G::TS; i += blockDim.x) {
     const int r = i / G::TS, c = i - r * G::TS;
-    const float k = c < PS ? __ldg(psf + r * PS + c) : 0.0f;
-    tap[i] = make_float2(k, k);
+    tap[i] = c < PS ? __ldg(psf + r * PS + c) : 0.0f;
   }
   int finite = 1;
   constexpr int kRows = 8;  // rows of a warp in flight together
@@ -110,15 +112,19 @@ k_matched_filter_t(int w, int h, const float* __restrict__ img, const float* __r
     for (int i = 0; i < kMfR; ++i) {
       const int ly = wr - i;
       if (ly < 0 || ly >= PS) continue;  // the same for every thread
-      const float2* tp = tap + ly * G::TS;
+      const float* tp = tap + ly * G::TS;
 #pragma unroll
-      for (int lx = 0; lx < PS; lx += 2) {
-        const float4 q = *reinterpret_cast<const float4*>(tp + lx);
+      for (int l0 = 0; l0 < PS; l0 += 4) {
+        const float4 q = *reinterpret_cast<const float4*>(tp + l0);
+        const float k[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-        for (int c = 0; c < kMfC / 2; ++c) acc[i][c] = __ffma2_rn(make_float2(q.x, q.y), even[c + lx / 2], acc[i][c]);
-        if (lx + 1 < PS)
+        for (int u = 0; u < 4; ++u) {
+          if (l0 + u >= PS) break;
+          const float2 kk = make_float2(k[u], k[u]);
 #pragma unroll
-          for (int c = 0; c < kMfC / 2; ++c) acc[i][c] = __ffma2_rn(make_float2(q.z, q.w), odd[c + lx / 2], acc[i][c]);
+          for (int c = 0; c < kMfC / 2; ++c)
+            acc[i][c] = __ffma2_rn(kk, (u & 1) ? odd[c + (l0 + u) / 2] : even[c + (l0 + u) / 2], acc[i][c]);
+        }
       }
     }
   }
@@ -148,7 +154,7 @@ k_matched_filter_t(int w, int h, const float* __restrict__ img, const float* __r
 
 // Generic PSF sizes (taps in shared memory), and the non-finite tiles listed
 // by k_matched_filter_t: with `tiles` set, CTAs stride over the 64 x 32
-// sub-tiles of the *ntile listed 128 x 128 tiles instead of the grid.
+// sub-tiles of the *ntile listed 64 x 64 tiles instead of the grid.
 __global__ void __launch_bounds__(256)
 k_matched_filter_g(int w, int h, const float* __restrict__ img, const float* __restrict__ var,
                    const float* __restrict__ psf, int ps, float sumpsf2, float* __restrict__ out,
