@@ -15,6 +15,7 @@
 #include <cub/device/device_radix_sort.cuh>
 
 #include <algorithm>
+#include <cmath>
 #include <string>
 
 #include "dev_common.cuh"
@@ -204,13 +205,15 @@ __global__ void k_cand_keys(const unsigned* count, int cap, const int* __restric
 // is kept (it is out) or undecided (it waits there, and goes on from there when
 // that one is out); if none is left it is kept. The rounds follow the longest
 // chain of waiting candidates, 3 to 5 on star fields; the brightest undecided
-// candidate always decides, so 1024 bound them.
+// candidate always decides, so 1024 bound them. Where a frame has room for few
+// stamps (few_stamps) the chunk keeps one a round instead.
 constexpr int kIsoHeads = 1024;
 struct Isolation {
   int4 node[1024];  // x, y, next
   int head[kIsoHeads], khead[kIsoHeads];
   unsigned char state[1024];
   int wsum[32];
+  int4 first[2][32];  // each warp's brightest undecided candidate: thread, x, y
 };
 __device__ __forceinline__ int iso_bucket(int cx, int cy) {
   return static_cast<int>((static_cast<unsigned>(cx) * 0x9E3779B1u ^ static_cast<unsigned>(cy) * 0x85EBCA6Bu) >> 22);
@@ -228,7 +231,7 @@ __device__ __forceinline__ bool iso_near(int dx, int dy, int r, long long r2) {
 }
 
 // One chunk: thread t < n holds raster index idx. Returns the number kept so far.
-__device__ int isolate_chunk(Isolation& sh, int w, int n, int idx, int iso, int max_stamps, int nk, int* ks,
+__device__ int isolate_chunk(Isolation& sh, int w, int n, int idx, int iso, bool few, int max_stamps, int nk, int* ks,
                              int* __restrict__ kept) {
   enum : unsigned char { kOut, kKept, kOpen };
   volatile unsigned char* state = sh.state;
@@ -248,10 +251,27 @@ __device__ int isolate_chunk(Isolation& sh, int w, int n, int idx, int iso, int 
     for (int q = 0; q < 9 && open; ++q)
       for (int k = sh.khead[iso_bucket(cx - 1 + q % 3, cy - 1 + q / 3)]; k != kEnd && open; k = knext[k])
         open = !iso_near(x - ks[2 * k], y - ks[2 * k + 1], r, r2);
+  bool mine = false;
+  if (few) {
+    // Round by round the brightest candidate left is kept and the others drop out that
+    // lie near it.
+    for (int round = 0, left = max_stamps - nk; round < left; ++round) {
+      const unsigned vote = __ballot_sync(0xffffffffu, open);
+      if (vote ? lane == __ffs(vote) - 1 : lane == 0) sh.first[round & 1][warp] = make_int4(vote ? tid : 1024, x, y, 0);
+      __syncthreads();
+      const int4 f = sh.first[round & 1][lane];
+      const int best = __reduce_min_sync(0xffffffffu, f.x);
+      if (best == 1024) break;
+      const int from = best >> 5;
+      const int bx = __shfl_sync(0xffffffffu, f.y, from), by = __shfl_sync(0xffffffffu, f.z, from);
+      if (best == tid) mine = true;
+      open = open && best != tid && !iso_near(x - bx, y - by, r, r2);
+    }
+    open = false;
+  }
   state[tid] = open ? kOpen : kOut;
   if (open) sh.node[tid] = make_int4(x, y, atomicExch(&sh.head[iso_bucket(cx, cy)], tid), 0);
   __syncthreads();
-  bool mine = false;
   int q = 0, k = open ? sh.head[iso_bucket(cx - 1, cy - 1)] : kEnd;
   do {
     while (open) {
@@ -330,7 +350,7 @@ __device__ unsigned long long sort_1024(unsigned long long k, unsigned long long
 constexpr int kSortMost = 16384;
 constexpr int kSortStamps = 4096;  // the most stamps whose places fit beside the keys
 
-__global__ void __launch_bounds__(1024) k_sort_isolate(int w, DetectPair jobs, int iso, int max_stamps) {
+__global__ void __launch_bounds__(1024) k_sort_isolate(int w, DetectPair jobs, int iso, bool few, int max_stamps) {
   using u64 = unsigned long long;
   extern __shared__ __align__(16) u64 keys[];
   __shared__ Isolation sh;
@@ -416,7 +436,7 @@ __global__ void __launch_bounds__(1024) k_sort_isolate(int w, DetectPair jobs, i
     }
     __syncthreads();
     const u64 k = sort_1024(tid < n ? chunk[tid] : ~0ull, chunk);
-    nk = isolate_chunk(sh, w, n, tid < n ? static_cast<int>(k & 0xffffffffull) : 0, iso, max_stamps, nk, ks, j.kept);
+    nk = isolate_chunk(sh, w, n, tid < n ? static_cast<int>(k & 0xffffffffull) : 0, iso, few, max_stamps, nk, ks, j.kept);
     lo = end + 1;
     left -= n;
   }
@@ -425,7 +445,7 @@ __global__ void __launch_bounds__(1024) k_sort_isolate(int w, DetectPair jobs, i
 
 // Isolation of candidates sorted in global memory.
 __global__ void __launch_bounds__(1024)
-k_isolate(int w, DetectDev j, int cap, const int* __restrict__ sorted_idx, int iso, int max_stamps) {
+k_isolate(int w, DetectDev j, int cap, const int* __restrict__ sorted_idx, int iso, bool few, int max_stamps) {
   extern __shared__ int ks[];
   __shared__ Isolation sh;
   const int nc = min(static_cast<int>(j.count[0]), cap);
@@ -433,7 +453,7 @@ k_isolate(int w, DetectDev j, int cap, const int* __restrict__ sorted_idx, int i
   for (int base = 0; base < nc && nk < max_stamps; base += 1024) {
     const int n = min(nc - base, 1024);
     const int idx = static_cast<int>(threadIdx.x) < n ? sorted_idx[base + threadIdx.x] : 0;
-    nk = isolate_chunk(sh, w, n, idx, iso, max_stamps, nk, ks, j.kept);
+    nk = isolate_chunk(sh, w, n, idx, iso, few, max_stamps, nk, ks, j.kept);
   }
   if (threadIdx.x == 0) j.count[2] = static_cast<unsigned>(nk);
 }
@@ -697,6 +717,18 @@ static void launch_stamp_props(cudaStream_t s, int w, int h, const DetectParamsD
   DGPU_LAUNCH("k_stamp_props");
 }
 
+// Whether isolation keeps few stamps: at most one in a square of side radius / sqrt 2,
+// so (w / side + 1) (h / side + 1) bound them. Up to 640 the chunk is resolved a kept
+// stamp at a time (0.3 us each): the cells of the lists then hold many candidates that
+// wait for one another. 2000 stars at 1003 x 1531, up to 1000 stamps, by lists and by
+// rounds: radius 50 (1302) 83 and 114 us, 80 (525) 122 and 63, 200 (118) 739 and 29;
+// 8000 at 2048 x 2048: 80 (1384) 162 and 214, 120 (632) 189 and 149; 300 x 400 with 200
+// stars: 20 (650) 22 and 37, 30 (300) 33 and 27, 200 (12) 1129 and 11.
+static bool few_stamps(int w, int h, const DetectParamsDev& p) {
+  const double side = std::abs(static_cast<double>(p.isolation_radius)) / std::sqrt(2.0);
+  return side >= 1.0 && (w / side + 1.0) * (h / side + 1.0) <= 640.0;
+}
+
 // The general path of one image, for more candidates than one CTA sorts or more
 // stamps than it keeps in shared memory beside them: radix sort, isolation and
 // measurement, reading the kept count back in between. On entry j.hc[0] > 0.
@@ -717,7 +749,7 @@ static void detect_general(Context& c, int w, int h, const DetectParamsDev& p, D
   const size_t smem = iso_smem(p.max_stamps);
   if (sizeof(int) * 2 * std::max(p.max_stamps, 1) > 160 * 1024) fail(DGPU_ERR_INVALID, "detect_stamps: max_stamps above 20480 is not supported");
   ensure_dynamic_smem(reinterpret_cast<const void*>(k_isolate), smem);
-  k_isolate<<<1, 1024, smem, s>>>(w, d, cap, sorted, p.isolation_radius, p.max_stamps);
+  k_isolate<<<1, 1024, smem, s>>>(w, d, cap, sorted, p.isolation_radius, few_stamps(w, h, p), p.max_stamps);
   DGPU_LAUNCH("k_isolate");
   read_back(c, j.hc, d.count, sizeof(j.hc));
   sync_reads(c);
@@ -771,7 +803,7 @@ static void run_detect_jobs(Context& c, int w, int h, const DetectParamsDev& p, 
   DGPU_LAUNCH("k_footprint");
   if (fast) {
       ensure_dynamic_smem(reinterpret_cast<const void*>(k_sort_isolate), sort_smem);
-    k_sort_isolate<<<njobs, 1024, sort_smem, s>>>(w, jobs, p.isolation_radius, p.max_stamps);
+    k_sort_isolate<<<njobs, 1024, sort_smem, s>>>(w, jobs, p.isolation_radius, few_stamps(w, h, p), p.max_stamps);
     DGPU_LAUNCH("k_sort_isolate");
     if (most > 0) launch_stamp_props(s, w, h, p, jobs, njobs, most, most);
   }
