@@ -29,3 +29,40 @@ def test_isolation_of_few_stamps(count, iso, most):
     kx, ky = _greedy(xs, ys, values, size, iso, most)
     np.testing.assert_array_equal(got["x"], kx)
     np.testing.assert_array_equal(got["y"], ky)
+
+
+def _matched(a, b, radius, most):
+    """The pair's stamps from those of its images: each of the reference (in order) with
+    the nearest of the science image, the first of them on a tie."""
+    rows = []
+    for x, y, f in zip(b["x"], b["y"], b["fwhm"]):
+        d2 = (x - a["x"].astype(np.int64)) ** 2 + (y - a["y"].astype(np.int64)) ** 2
+        if len(d2) and d2.min() <= radius * radius:
+            rows.append((x, y, a["fwhm"][int(np.argmin(d2))], f))
+    return rows[:most]
+
+
+# Both images in one CTA's sort, one of them past it, one without candidates, and more
+# stamps than the one CTA keeps.
+@pytest.mark.parametrize("left,right,most", [(40, 30, 400), (1, 50, 400), (1, 1, 400), (7, 0, 400), (3, 4, 5000)])
+def test_pair_lists_are_those_of_its_images(left, right, most):
+    size, radius = 1024, 2
+    rng = np.random.default_rng(10 * left + right)
+    grid = np.arange(30, size - 30, 5)
+    xs, ys = (g.ravel() for g in np.meshgrid(grid, grid))
+
+    def image(step, jitter):
+        if step == 0:
+            return _image(np.zeros(0, int), np.zeros(0, int), np.zeros(0, np.float32), size)
+        x, y = xs[::step] + jitter, ys[::step]
+        return _image(x, y, (200.0 + rng.integers(0, 500, x.size)).astype(np.float32), size)
+
+    for sci, ref in ((image(left, 0), image(right, 1)), (image(right, 1), image(left, 0))):
+        kw = dict(stamp_radius=6, threshold_sigma=60.0, max_stamps=most, isolation_radius=12)
+        a, b = (_core.detect_stamps(i, **kw) for i in (sci, ref))
+        want = _matched(a, b, radius, len(b["x"]))
+        got = _core.select_stamps(sci, ref, match_radius=radius, **kw)
+        rows = list(zip(got["x"], got["y"], got["fwhm_science"], got["fwhm_reference"]))
+        assert len(rows) == len(want)
+        np.testing.assert_array_equal(np.array(rows, float).reshape(-1, 4), np.array(want, float).reshape(-1, 4))
+        assert left == 0 or right == 0 or len(rows) > 0
