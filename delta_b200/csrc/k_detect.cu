@@ -349,6 +349,7 @@ __device__ unsigned long long sort_1024(unsigned long long k, unsigned long long
 // sorted all keys).
 constexpr int kSortMost = 16384;
 constexpr int kSortStamps = 4096;  // the most stamps whose places fit beside the keys
+constexpr int kIsoStamps = 20480;  // and the most that fit without the keys
 
 __global__ void __launch_bounds__(1024) k_sort_isolate(int w, DetectPair jobs, int iso, bool few, int max_stamps) {
   using u64 = unsigned long long;
@@ -747,7 +748,7 @@ static void detect_general(Context& c, int w, int h, const DetectParamsDev& p, D
   void* tmp = c.slot(kSlotFft4, tmp_bytes + 16);
   DGPU_CUDA(cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, keys2, vals, sorted, nc, 0, 64, s));
   const size_t smem = iso_smem(p.max_stamps);
-  if (sizeof(int) * 2 * std::max(p.max_stamps, 1) > 160 * 1024) fail(DGPU_ERR_INVALID, "detect_stamps: max_stamps above 20480 is not supported");
+  if (p.max_stamps > kIsoStamps) fail(DGPU_ERR_INVALID, "detect_stamps: max_stamps above 20480 is not supported");
   ensure_dynamic_smem(reinterpret_cast<const void*>(k_isolate), smem);
   k_isolate<<<1, 1024, smem, s>>>(w, d, cap, sorted, p.isolation_radius, few_stamps(w, h, p), p.max_stamps);
   DGPU_LAUNCH("k_isolate");
@@ -774,8 +775,10 @@ static void run_detect_jobs(Context& c, int w, int h, const DetectParamsDev& p, 
   const size_t sort_smem = sizeof(unsigned long long) * kSortMost + iso_smem(most);
   const size_t psmem = sizeof(double) * static_cast<size_t>(2 * p.fwhm_radius + 1) * (2 * p.fwhm_radius + 1);
   const bool fast = most <= kSortStamps && psmem <= 200 * 1024;
-  const size_t kept_ints = (static_cast<size_t>(std::max(most, 1)) + 1) & ~size_t(1);
-  const size_t per = 64 + sizeof(int) * (2 * static_cast<size_t>(cap) + kept_ints) + sizeof(double) * 3 * std::max(most, 1);
+  // The general path keeps up to kIsoStamps (it refuses more) and measures elsewhere.
+  const size_t kept_ints = (static_cast<size_t>(std::clamp(most, 1, kIsoStamps)) + 1) & ~size_t(1);
+  const size_t per = 64 + sizeof(int) * (2 * static_cast<size_t>(cap) + kept_ints) +
+                     sizeof(double) * 3 * (fast ? static_cast<size_t>(std::max(most, 1)) : 0);
   char* buf = static_cast<char*>(c.slot(kSlotFft0, per * njobs));
   DetectPair jobs{};
   MedianJob med[kMedianJobs];
@@ -802,7 +805,7 @@ static void run_detect_jobs(Context& c, int w, int h, const DetectParamsDev& p, 
   k_footprint<<<dim3(148 * 4, njobs), 256, 0, s>>>(w, h, jobs, p, cap);
   DGPU_LAUNCH("k_footprint");
   if (fast) {
-      ensure_dynamic_smem(reinterpret_cast<const void*>(k_sort_isolate), sort_smem);
+    ensure_dynamic_smem(reinterpret_cast<const void*>(k_sort_isolate), sort_smem);
     k_sort_isolate<<<njobs, 1024, sort_smem, s>>>(w, jobs, p.isolation_radius, few_stamps(w, h, p), p.max_stamps);
     DGPU_LAUNCH("k_sort_isolate");
     if (most > 0) launch_stamp_props(s, w, h, p, jobs, njobs, most, most);

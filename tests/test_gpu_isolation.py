@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 from test_gpu_select_sizes import _greedy, _image
 
-from delta_b200 import _core
+from delta_b200 import _core, _lib
 
 pytestmark = pytest.mark.gpu
 
@@ -66,3 +66,32 @@ def test_pair_lists_are_those_of_its_images(left, right, most):
         assert len(rows) == len(want)
         np.testing.assert_array_equal(np.array(rows, float).reshape(-1, 4), np.array(want, float).reshape(-1, 4))
         assert left == 0 or right == 0 or len(rows) > 0
+
+
+@pytest.mark.parametrize("most", [20480, 20481, 2**31 - 1])
+def test_workspace_does_not_follow_the_most_stamps(most):
+    """A bound on the stamps far above what can be kept costs no memory; it is refused
+    only where there is a candidate."""
+    torch = pytest.importorskip("torch")
+    import ctypes
+
+    size = 256
+    ctx = _lib.context()
+    params = _core._detect_params(6, 60.0, most, 0.0, 0, 0, 0, 2)
+    out = [np.zeros(4, np.int32), np.zeros(4, np.int32), np.zeros(4), np.zeros(4), np.zeros(4)]
+    n = ctypes.c_int(-1)
+
+    def detect(img):
+        return _lib.lib().dgpu_detect_stamps(ctx.handle, _lib.MEM_HOST, ctypes.c_int64(size), ctypes.c_int64(size),
+                                             _lib.ptr(img), None, ctypes.byref(params), 4,
+                                             *[_lib.ptr(a) for a in out], ctypes.byref(n))
+
+    _core.detect_stamps(np.zeros((size, size), np.float32))
+    free = torch.cuda.mem_get_info()[0]
+    assert detect(np.zeros((size, size), np.float32)) == _lib.DGPU_OK and n.value == 0
+    assert free - torch.cuda.mem_get_info()[0] < 1 << 28
+    rc = detect(_image(np.array([100]), np.array([90]), np.float32(500.0), size))
+    if most > 20480:
+        assert rc == _lib.DGPU_ERR_INVALID
+    else:
+        assert rc == _lib.DGPU_OK and n.value == 1 and (out[0][0], out[1][0]) == (100, 90)
