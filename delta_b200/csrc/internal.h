@@ -121,7 +121,7 @@ struct Context {
   std::vector<int32_t> cat_i;   // 3 int32 columns x n
   std::vector<uint8_t> cat_u8;  // 7 uint8 columns x n
   int cat_count = 0;
-  int64_t cat_npix = 0;         // label image size of the last catalog
+  int64_t cat_npix = 0;         // label image size of the last catalog (-1: it failed half way)
 
   // Read-backs (read_back / sync_reads): a mapped pinned area that the host
   // logic's small device -> host copies reach by SM stores, and the copies

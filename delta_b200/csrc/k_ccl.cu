@@ -569,6 +569,10 @@ int run_catalog(Context& c, int w, int h, const float* score, const float* diff,
                 const double* bright_x, const double* bright_y, int n_bright) {
   cudaStream_t s = c.stream;
   const int64_t n = static_cast<int64_t>(w) * h;
+  // Until the list is complete there is nothing expand_labels could read: its indices
+  // come from the list, which the work below overwrites.
+  c.cat_npix = -1;
+  c.cat_count = 0;
   const SeedList sl = SeedList::at(static_cast<int*>(c.slot(kSlotLabels, sizeof(int) * SeedList::ints(n))), n);
   const bool neg = p.return_negative != 0;
   const int nb = static_cast<int>(SeedList::blocks(n));
