@@ -421,14 +421,16 @@ struct FinishParams {
 __device__ long lround_away(double v) { return static_cast<long>(v >= 0 ? floor(v + 0.5) : -floor(-v + 0.5)); }
 
 // summarize_component (src/catalog.cpp:337-418) finishing + dipole flag +
-// enrich_entries (src/catalog.cpp:476-596). A warp per component: its lanes load
-// the aperture's pixels together and every lane adds them in raster order.
+// enrich_entries (src/catalog.cpp:476-596). WARP: a warp per component, its lanes load
+// the aperture's pixels together and every lane adds them in raster order; else a
+// thread per component.
+template <bool WARP>
 __global__ void __launch_bounds__(128) k_comp_finish(int ncomp, int w, int h, const float* __restrict__ score,
                               const float* __restrict__ diff, const uint8_t* __restrict__ mask,
                               const float* __restrict__ variance, const float* __restrict__ psf,
                               const double* __restrict__ bx, const double* __restrict__ by, int nb,
                               CompStats cs, FinishParams fp, CompOut o) {
-  const int c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, c = WARP ? t >> 5 : t, lane = threadIdx.x & 31;
   if (c >= ncomp) return;
   const double kFwhmPerSigma = 2.354820045030949;
   const double kPi = 3.14159265358979323846;
@@ -464,20 +466,29 @@ __global__ void __launch_bounds__(128) k_comp_finish(int ncomp, int w, int h, co
     const double r2 = static_cast<double>(radius) * radius;
     const int64_t side = 2 * static_cast<int64_t>(radius) + 1, area = side * side;
     double fsum = 0.0;
-    for (int64_t e0 = 0; e0 < area; e0 += 32) {
-      const int64_t e = e0 + lane;
-      const int dy = static_cast<int>(e / side) - radius, dx = static_cast<int>(e % side) - radius;
-      const int yy = y0 + dy, xx = x0 + dx;
-      float v = 0.0f;
-      if (e < area && yy >= 0 && yy < h && xx >= 0 && xx < w && !(dx * dx + dy * dy > r2))
-        v = diff[static_cast<int64_t>(yy) * w + xx];
-      const unsigned in = __ballot_sync(0xffffffffu, v != 0.0f && isfinite(v));  // adding a zero changes nothing
-      for (unsigned left = in; left; left &= left - 1)
-        fsum += static_cast<double>(__shfl_sync(0xffffffffu, v, __ffs(left) - 1));
+    if constexpr (WARP) {
+      for (int64_t e0 = 0; e0 < area; e0 += 32) {
+        const int64_t e = e0 + lane;
+        const int dy = static_cast<int>(e / side) - radius, dx = static_cast<int>(e % side) - radius;
+        const int yy = y0 + dy, xx = x0 + dx;
+        float v = 0.0f;
+        if (e < area && yy >= 0 && yy < h && xx >= 0 && xx < w && !(dx * dx + dy * dy > r2))
+          v = diff[static_cast<int64_t>(yy) * w + xx];
+        const unsigned in = __ballot_sync(0xffffffffu, v != 0.0f && isfinite(v));  // adding a zero changes nothing
+        for (unsigned left = in; left; left &= left - 1)
+          fsum += static_cast<double>(__shfl_sync(0xffffffffu, v, __ffs(left) - 1));
+      }
+    } else {
+      for (int dy = max(-radius, -y0); dy <= min(radius, h - 1 - y0); ++dy)
+        for (int dx = max(-radius, -x0); dx <= min(radius, w - 1 - x0); ++dx) {
+          if (dx * dx + dy * dy > r2) continue;
+          const float v = diff[static_cast<int64_t>(y0 + dy) * w + x0 + dx];
+          if (isfinite(v)) fsum += static_cast<double>(v);
+        }
     }
     o.flux[c] = fsum;
   }
-  if (lane != 0) return;
+  if (WARP && lane != 0) return;
   uint8_t q = 0;
   if (!consistent) q |= 1u;
   if (mflags != 0) q |= 4u;
@@ -554,8 +565,17 @@ __global__ void __launch_bounds__(128) k_comp_finish(int ncomp, int w, int h, co
 // Host driver
 // ---------------------------------------------------------------------------
 
-// Blocks of the kernels that walk the seed list (its length is on the device).
-constexpr int kListBlocks = 148 * 2;
+// Blocks of the kernels that walk the seed list (its length is on the device): as many
+// as the chip holds, twice for the merge, whose searches take uneven time. Two blocks
+// an SM save 1 us on a list of a few thousand and lose on long ones (4096 x 4096 of
+// noise, threshold 0.3 sigma, 6e6 seeds: merge 1729 us, now 414; a comb of one
+// component with 2e6 seeds 1649, now 366).
+constexpr int kListBlocks = 148 * 8;
+constexpr int kMergeBlocks = 148 * 16;
+// Components that get a warp each for their finish: half the chip's warps. 4096 x 4096,
+// a warp and a thread each: 66 components 10 and 18 us, 4100 15 and 26, 22933 57 and 28,
+// 348091 776 and 68; 1001 x 1001: 1360 10 and 19, 6152 20 and 19.
+constexpr int kFinishWarps = 148 * 32;
 
 void expand_labels(Context& c, int64_t n, int* labels) {
   const SeedList sl = SeedList::at(static_cast<int*>(c.slot_ptr[kSlotLabels]), n);
@@ -591,7 +611,7 @@ int run_catalog(Context& c, int w, int h, const float* score, const float* diff,
     StageTimer t(c, neg ? "catalog: label negative" : "catalog: label positive");
     k_seed_list<<<nb, kSeedBlock / 32, 0, s>>>(n, nb, sl);
     DGPU_LAUNCH("k_seed_list");
-    k_label_merge<<<kListBlocks, 256, 0, s>>>(w, sl, c.d_status, c.label_loop_cap);
+    k_label_merge<<<kMergeBlocks, 256, 0, s>>>(w, sl, c.d_status, c.label_loop_cap);
     DGPU_LAUNCH("k_label_merge");
     k_label_flatten<<<kListBlocks, 256, 0, s>>>(sl, c.d_status, c.label_loop_cap);
     DGPU_LAUNCH("k_label_flatten");
@@ -674,8 +694,10 @@ int run_catalog(Context& c, int w, int h, const float* score, const float* diff,
   fp.shape_tol = p.shape_chi2_tolerance;
   fp.bright_radius = p.bright_star_radius > 0.0 ? p.bright_star_radius : 3.0 * p.expected_fwhm;
   fp.psf_size = psf_size;
-  k_comp_finish<<<(ncomp + 3) / 4, 128, 0, s>>>(ncomp, w, h, score, diff, mask, variance, psf,
-                                                     bright_x, bright_y, n_bright, cs, fp, o);
+  const bool warps = ncomp <= kFinishWarps;
+  auto kern = warps ? k_comp_finish<true> : k_comp_finish<false>;
+  kern<<<warps ? (ncomp + 3) / 4 : (ncomp + 127) / 128, 128, 0, s>>>(ncomp, w, h, score, diff, mask, variance, psf,
+                                                                     bright_x, bright_y, n_bright, cs, fp, o);
   DGPU_LAUNCH("k_comp_finish");
   // Bring the columns back into the context (host).
   std::vector<char> host(out_bytes);
