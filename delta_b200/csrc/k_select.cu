@@ -2,7 +2,9 @@
 //
 // Up to 2^19 values (every background sample, and the fill values of frames up
 // to 3.6 Mpix): a cluster of eight CTAs per sample holds the keys in shared memory
-// and selects without leaving it. A subsample of 512 keys first brackets the
+// (the first 425984; each pass re-reads the rest, six loads in flight: one by one they
+// made a pass over 523776 values 12 load latencies long) and selects without leaving
+// it. A subsample of 512 keys first brackets the
 // wanted rank (4 sigma of its rank: about a sixth of the keys), so that one
 // pass of comparisons counts the keys below and only the bracket's keys enter the
 // shared-memory histograms, spread over their digits; the leading bits of a sky
@@ -163,7 +165,14 @@ __global__ void __cluster_dims__(kCtas, 1, 1) __launch_bounds__(kThreads, 1) k_c
         f(q.z);
         f(q.w);
       }
-      for (int i = held + tid; i < count; i += kThreads) f(which == 1 ? distance(source(i)) : source(i));
+      constexpr int kTail = 6;  // loads in flight (the largest sample's tail is 12 a thread)
+      for (int i = held + tid; i < count; i += kTail * kThreads) {
+        uint32_t k[kTail];
+#pragma unroll
+        for (int u = 0; u < kTail; ++u) k[u] = i + u * kThreads < count ? source(i + u * kThreads) : kNone;
+#pragma unroll
+        for (int u = 0; u < kTail; ++u) f(which == 1 ? distance(k[u]) : k[u]);
+      }
     };
     if (tid < kSub / kCtas)
       mine[tid] = held > 0 ? keys[sub_place(tid, kSub / kCtas, held)] : kNone;
