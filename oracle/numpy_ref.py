@@ -338,8 +338,40 @@ def reference_fill_value(ref: np.ndarray, ref_mask) -> np.float32:
 
 
 # ---------------------------------------------------------------------------
-# Convolution engine (src/convolve.cpp), float64 accumulation of float32 inputs
+# Convolution engine (src/convolve.cpp): in float64 (convolve_x, convolve_y), and as
+# the reference sums it, in float32 with fused multiply-adds (basis_convolve)
 # ---------------------------------------------------------------------------
+
+
+def fma32(a, b, c):
+    """float32(a * b + c) rounded once, for finite float32 operands.
+
+    The product of two float32 values is exact in float64. Its sum with c is brought
+    to odd (Boldo & Melquiond 2008): rounded to nearest, then, where that was inexact
+    and left the last bit even, moved to the neighbour on the side of the error. A
+    value so rounded to 53 bits rounds to 24 as the exact sum does."""
+    p = np.multiply(a, b, dtype=np.float64)
+    c = np.asarray(c, np.float64)
+    s = p + c
+    t = s - p
+    err = (p - (s - t)) + (c - t)  # exact (Knuth's two-sum)
+    even = (s.view(np.int64) & 1) == 0
+    s = np.where((err != 0) & even, np.nextafter(s, np.where(err > 0, np.inf, -np.inf)), s)
+    return s.astype(np.float32)
+
+
+def _convolve_x32(img: np.ndarray, k: np.ndarray) -> np.ndarray:
+    """convolve_x with the reference's sums: float32, the taps j ascending, each a fused
+    multiply-add; samples off the frame add an exact zero."""
+    ks, (h, w) = k.size, img.shape
+    hh = (ks - 1) // 2
+    pad = np.zeros((h, w + 2 * hh), np.float32)
+    pad[:, hh : hh + w] = img
+    out = np.zeros((h, w), np.float32)
+    for j in range(ks):
+        sh = hh - j
+        out = fma32(k[j], pad[:, hh + sh : hh + sh + w], out)
+    return out
 
 
 def convolve_x(img: np.ndarray, k: np.ndarray) -> np.ndarray:
@@ -363,12 +395,13 @@ def convolve_y(img: np.ndarray, k: np.ndarray) -> np.ndarray:
 
 
 def basis_convolve(image: np.ndarray, beta: float, n_max: int, radius: int = 0) -> np.ndarray:
-    """(nc, H, W) B_n stack.  src/convolve.cpp:90-113 (float32 taps)."""
+    """(nc, H, W) B_n stack, float32 as the reference's.  src/convolve.cpp:90-113."""
     r = resolve_radius(beta, n_max, radius)
     b1d = gauss_hermite_basis1d(beta, n_max, r)
     k1 = b1d.astype(np.float32)
-    tx = [convolve_x(image, k1[n]) for n in range(n_max + 1)]
-    return np.stack([convolve_y(tx[nx], k1[ny]) for nx, ny in basis_orders(n_max)])
+    img = np.asarray(image, np.float32)
+    tx = [_convolve_x32(img, k1[n]) for n in range(n_max + 1)]
+    return np.stack([_convolve_x32(np.ascontiguousarray(tx[nx].T), k1[ny]).T for nx, ny in basis_orders(n_max)])
 
 
 # ---------------------------------------------------------------------------
@@ -960,7 +993,7 @@ def fit_kernel(science, reference, knots, stamp_x, stamp_y, stamp_radius, beta, 
     ks = 2 * r + 1
     if basis_convolve_fn is None:
         def basis_convolve_fn(patch):
-            return basis_convolve(patch, beta, n_max, r).astype(np.float32)
+            return basis_convolve(patch, beta, n_max, r)
     g = gather_stamps(science, reference, stamp_x, stamp_y, stamp_radius, b1d, n_max, r,
                       science_var, reference_var, science_mask, reference_mask, basis_convolve_fn)
     npix_all = g["target"].size

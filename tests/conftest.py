@@ -24,6 +24,22 @@ def pytest_configure(config):
     config.addinivalue_line("markers", "slow: long-running")
 
 
+# Holds an FP64 oracle to 1e-9 of the effective degrees of freedom. The device's B_n are
+# float32 as the reference's: at the stamps that the reference selects that moves them
+# by less, at the fixed ones used without it by 1.6e-8 (49.801186822 in FP64 rows,
+# 49.801187657 in float32 rows, 49.801187648 on the device).
+NEEDS_REFERENCE_STAMPS = "test_stamp_gcv_matches_fp64_oracle_and_central_differences"
+
+
+def pytest_collection_modifyitems(items):
+    """Without the oracle built from the reference that test misses its bound: it runs
+    last, so that a run that stops at the first failure has run all the others."""
+    from oracle import refbuild
+
+    if not refbuild.available():
+        items.sort(key=lambda item: item.name == NEEDS_REFERENCE_STAMPS)
+
+
 @pytest.fixture
 def rng():
     return np.random.default_rng(12345)
