@@ -417,7 +417,7 @@ int dgpu_subtract(dgpu_context* ctx, int mem, int64_t width, int64_t height, con
     float* scal = static_cast<float*>(c.slot(kSlotScratch1, 64));  // [0] ref fill, [1] diff fill
     {
       StageTimer t(c, "subtract: sanitise reference");
-      launch_strided_median(c, kSampleReference, static_cast<int64_t>(n), ref, rm, scal);
+      launch_strided_median(c, static_cast<int64_t>(n), ref, rm, scal);
     }
     {
       const auto taps = b.taps();
@@ -460,7 +460,7 @@ int dgpu_subtract(dgpu_context* ctx, int mem, int64_t width, int64_t height, con
       StageTimer t(c, "subtract: mask growth");
       uint8_t* eb = static_cast<uint8_t*>(c.slot(kSlotExactBad, n));
       launch_mask(s, w, h, sci, ref, sm, rm, saturation, b.radius, diff, mask, eb);
-      launch_strided_median(c, kSampleDifference, static_cast<int64_t>(n), diff, mask, scal + 1);
+      launch_strided_median(c, static_cast<int64_t>(n), diff, mask, scal + 1);
       launch_mask_fill(s, static_cast<int64_t>(n), mask, eb, scal + 1, diff, var);
     }
     stage_out(c, mem, out_difference, diff, 4 * n);

@@ -756,7 +756,7 @@ int dgpu_fit_kernel(dgpu_context* ctx, int mem, int64_t width, int64_t height, c
     float* fill = static_cast<float*>(c.slot(kSlotScratch2, 64));
     {
       StageTimer t(c, "fit: stamp B_n convolve");
-      launch_strided_median(c, kSampleReference, static_cast<int64_t>(npx), ref, rm, fill);
+      launch_strided_median(c, static_cast<int64_t>(npx), ref, rm, fill);
       int* dsx = up(c, kSlotBright, reinterpret_cast<const int*>(stamp_x), static_cast<size_t>(n_stamps));
       int* dsy = static_cast<int*>(c.slot(kSlotCompOut, sizeof(int) * std::max(n_stamps, 1)));
       DGPU_CUDA(h2d_async(dsy, stamp_y, sizeof(int) * n_stamps, st));
@@ -947,7 +947,7 @@ int dgpu_stamp_gcv(dgpu_context* ctx, int mem, int64_t width, int64_t height, co
     E.alloc_rows();
     const int rk = E.rk;
     float* fill = static_cast<float*>(c.slot(kSlotScratch2, 64));
-    launch_strided_median(c, kSampleReference, static_cast<int64_t>(npx), ref, rm, fill);
+    launch_strided_median(c, static_cast<int64_t>(npx), ref, rm, fill);
     int* dsx = up(c, kSlotBright, reinterpret_cast<const int*>(stamp_x), static_cast<size_t>(n_stamps));
     int* dsy = up(c, kSlotCompOut, reinterpret_cast<const int*>(stamp_y), static_cast<size_t>(n_stamps));
     // Taps: x tables carry the scale (u_c = s B_n), y tables do not.

@@ -76,7 +76,7 @@ int dgpu_kernel_chi2(dgpu_context* ctx, int mem, int64_t width, int64_t height, 
     const auto* rm = static_cast<const uint8_t*>(stage_in(c, mem, reference_mask, n, kSlotInMaskR));
     const DevFields F = build_fields(c, tp, model->theta, nf, w, h);
     float* scal = static_cast<float*>(c.slot(kSlotScratch1, 64));
-    launch_strided_median(c, kSampleReference, static_cast<int64_t>(n), ref, rm, scal);
+    launch_strided_median(c, static_cast<int64_t>(n), ref, rm, scal);
 
     // Shifted taps and their derivatives (float32 copies of the FP64 values).
     std::vector<double> gxd, dgxd, gyd, dgyd;

@@ -43,8 +43,6 @@ void launch_block_var(cudaStream_t s, const FftGeom& g, int nitems, int nextra, 
 void launch_local_kernels(cudaStream_t s, const FftGeom& g, int ncell, const TpsDev& t, const double* theta, int nc,
                           const float* phi, int ks, const double* centres, double* sumk2, float* dense,
                           float* kern_out);
-void launch_ola_normalise(cudaStream_t s, int w, int h, const double* wx_total, const double* wy_total, float* acc,
-                          float* var_acc);
 // Overlap-add of the raw block outputs `bout` (item x n x n) into acc / var_acc,
 // in the reference's colour order, normalised by the weight sums.
 void launch_ola_gather(cudaStream_t s, int w, int h, int n, const int* oxs, int nox, const int* oys, int noy,

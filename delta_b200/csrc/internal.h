@@ -78,9 +78,9 @@ enum Slot : int {
   kSlotInSci, kSlotInRef, kSlotInVarS, kSlotInVarR, kSlotInMaskS, kSlotInMaskR,
   kSlotOutDiff, kSlotOutVar, kSlotOutMask, kSlotOutScore,
   kSlotLattice, kSlotLatticeF, kSlotCellX, kSlotCellY, kSlotTaps, kSlotPhi, kSlotFullFields,
-  kSlotTheta, kSlotKnots, kSlotZ,
+  kSlotTheta, kSlotZ,
   kSlotExactBad, kSlotSamples, kSlotSelect, kSlotPsf,
-  kSlotSeedPos, kSlotSeedNeg, kSlotLabels, kSlotLabelsNeg, kSlotRootRank, kSlotBlockCounts,
+  kSlotSeedPos, kSlotSeedNeg, kSlotLabels, kSlotRootRank, kSlotBlockCounts,
   kSlotCompStats, kSlotCompOut, kSlotBright, kSlotScratch0, kSlotScratch1, kSlotScratch2,
   kSlotFit0, kSlotFit1, kSlotFit2, kSlotFit3, kSlotFit4, kSlotFit5, kSlotFit6, kSlotFit7,
   kSlotFit8, kSlotFit9, kSlotFit10, kSlotFit11, kSlotFit12, kSlotFit13, kSlotFit14, kSlotFit15,
@@ -383,7 +383,6 @@ struct SubtractArgs {
   const float* fill;  // device scalar (reference fill value)
   float* diff;
 };
-void launch_model_convolve(cudaStream_t s, const SubtractArgs& a, const Basis& b);
 void launch_variance(cudaStream_t s, int w, int h, const DevFields& F, const float* phi, int rk,
                      int nc, const float* var_s, const float* var_r, float* var_out);
 void launch_mask(cudaStream_t s, int w, int h, const float* sci, const float* ref,
@@ -404,20 +403,14 @@ void launch_negate(cudaStream_t s, int64_t n, float* v);
 // (no allocation); out2 (host) = {median, MAD}. Synchronises `s`.
 void background_noalloc(int64_t n, const float* img, const uint8_t* mask, cudaStream_t s, float* out2);
 
-// Upper median (element size/2 of the sorted sample) of values[7j] that pass a
-// predicate, via radix select. Result written to a device float.
-enum SampleKind { kSampleReference = 0, kSampleDifference = 1 };
-void launch_strided_median(Context& c, int kind, int64_t n, const float* values, const uint8_t* mask,
-                           float* d_result);
+// Upper median (element size/2 of the sorted sample) of the finite values[7j] whose
+// mask byte is 0, via radix select. Result written to a device float.
+void launch_strided_median(Context& c, int64_t n, const float* values, const uint8_t* mask, float* d_result);
 
 void launch_matched_filter(cudaStream_t s, int w, int h, const float* img, const float* var, const float* psf_dev,
                            int ps, float sumpsf2, float* out, int* nf_buf);
 
-void launch_basis_convolve(cudaStream_t s, int w, int h, const float* img, const Basis& b,
-                           const float* taps, float* out);
-
 // Catalog (k_ccl.cu)
-struct CatalogDevResult;
 // Label image (n int32, device) of the last run_catalog, which saw n pixels.
 void expand_labels(Context& c, int64_t n, int* labels);
 int run_catalog(Context& c, int w, int h, const float* score, const float* diff,

@@ -1019,24 +1019,6 @@ k_cell_power(FftGeom G, TpsDev t, const double* __restrict__ theta, int nc, cons
   }
 }
 
-// Normalise by the separable Hann weight sum (src/noise.cpp:458-479).
-__global__ void k_ola_normalise(int w, int h, const double* __restrict__ wx_total, const double* __restrict__ wy_total,
-                                float* __restrict__ acc, float* __restrict__ var_acc) {
-  const int64_t n = static_cast<int64_t>(w) * h;
-  for (int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n;
-       i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    const int x = static_cast<int>(i % w), y = static_cast<int>(i / w);
-    const double ws = wy_total[y] * wx_total[x];
-    if (ws > 0.0) {
-      acc[i] = static_cast<float>(static_cast<double>(acc[i]) / ws);
-      var_acc[i] = static_cast<float>(static_cast<double>(var_acc[i]) / ws);
-    } else {
-      acc[i] = 0.0f;
-      var_acc[i] = 0.0f;
-    }
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Launchers
 // ---------------------------------------------------------------------------
@@ -1176,14 +1158,6 @@ void launch_ola_gather(cudaStream_t s, int w, int h, int n, const int* oxs, int 
   k_ola_gather<<<grid, kOlaTW, 0, s>>>(w, h, n, oxs, nox, oys, noy, hwin, bout, bnum, wx_total, wy_total, acc,
                                        var_acc);
   DGPU_LAUNCH("k_ola_gather");
-}
-
-void launch_ola_normalise(cudaStream_t s, int w, int h, const double* wx_total, const double* wy_total, float* acc,
-                          float* var_acc) {
-  const int64_t n = static_cast<int64_t>(w) * h;
-  const int blocks = static_cast<int>(std::min<int64_t>((n + 255) / 256, 148 * 16));
-  k_ola_normalise<<<blocks, 256, 0, s>>>(w, h, wx_total, wy_total, acc, var_acc);
-  DGPU_LAUNCH("k_ola_normalise");
 }
 
 }  // namespace dgpu

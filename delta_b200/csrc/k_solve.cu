@@ -362,14 +362,6 @@ __device__ __forceinline__ double* e_tile(const Sys& y, int c, int tj) {
 }
 __device__ __forceinline__ double* d_tile(const Sys& y, int j) { return y.Dv + static_cast<size_t>(j) * kTS; }
 
-// Initial value of E (row, col): rhs in row 0, F^T below, zero padding.
-__device__ __forceinline__ double e_init(const Sys& y, int row, int col) {
-  if (row == 0) return col < y.P ? y.rhs[col] : 0.0;
-  if (row > y.nfr) return 0.0;
-  const int fb = (row - 1) / y.r, jj = (row - 1) - fb * y.r, m = col - fb * y.k;
-  return (m >= 0 && m < y.k) ? y.fk[m * y.r + jj] : 0.0;
-}
-
 // Does A tile (ti, tj) hold an element of a diagonal field block (penalised)?
 __device__ __forceinline__ bool a_pen_tile(const Sys& y, int ti, int tj) {
   const int r0 = ti * kT, c0 = tj * kT;

@@ -132,10 +132,6 @@ constexpr int kMcXPT = 4;   // output columns per thread in the x pass
 // both passes read them as 16-byte vectors (the y pass reads 8 taps at j0 + 0..7).
 __host__ __device__ constexpr int mc_tap_stride(int ks) { return (ks + 7) & ~7; }
 
-struct McSmem {
-  int nrows, gbw_pad, lat_nx, lat_ny, cx0, cy0;
-};
-
 template <int NX, bool STACK>
 __global__ void __launch_bounds__(256)
 k_model_convolve(int w, int h, const float* __restrict__ sci, const float* __restrict__ ref,
@@ -920,9 +916,7 @@ void launch_mask_fill(cudaStream_t s, int64_t n, const uint8_t* mask, const uint
 // Upper median of a stride-7 sample (std::nth_element(size / 2); an empty sample
 // yields 0): the good finite reference pixels (src/subtract.cpp:20-51), or the
 // unmasked finite difference pixels under the grown mask (915-945).
-void launch_strided_median(Context& c, int kind, int64_t n, const float* values, const uint8_t* mask,
-                           float* d_result) {
-  (void)kind;
+void launch_strided_median(Context& c, int64_t n, const float* values, const uint8_t* mask, float* d_result) {
   launch_upper_median(c, n, 7, values, mask, d_result);
 }
 
