@@ -1,9 +1,9 @@
 // chi^2 tiles of the kernel model (see k_grad.cu) for the common basis shapes:
 // NX = n_max + 1 components per direction and the taps padded with zeros to
-// KSP = 8 KB, both known at compile time, as in k_model_convolve_fast.cu. A
-// zero tap times a finite staged value adds an exact zero, and every sum keeps
-// the generic kernel's order (x taps, y taps and components ascending), so the
-// per-pixel values are its values bit for bit.
+// KSP = 8 KB, both known at compile time. The x pass takes its taps in pairs: the one
+// after the last is a zero, which times a finite staged value adds an exact zero. The y
+// pass stops at the last tap. Every sum keeps the generic kernel's order (x taps, y taps
+// and components ascending), so the per-pixel values are its values bit for bit.
 //
 // Value only (GRAD false): C_c alone. x sums as one float per column, y pass
 // with 2 columns x 4 rows per thread in packed FMAs, 32 x 64 tiles, two CTAs
@@ -15,7 +15,7 @@
 // by side as one float2 per column, so one 8-byte load feeds the packed FMA
 // (C, C^x) += g_y (t, t') and the scalar C^y += g'_y t; a thread holds 1 column
 // x 8 rows, whose sliding window makes 15 loads serve 192 FMAs (with 4 rows the
-// loads would bound it). The two buffers take 169 KB at 32 x 64, so one CTA of
+// loads would bound it). The two buffers take 154 KB at 32 x 64, so one CTA of
 // 256 threads per SM: 1.78 ms with the generic kernel, 0.81 ms now. FP32 FMA
 // bound: 2500 FMA per pixel with the halo rows, 0.28 ms at 37.2 TFMA/s.
 #include <cuda_runtime.h>
@@ -30,7 +30,6 @@ namespace dgpu {
 namespace {
 
 constexpr int kTW = 32;       // tile columns
-constexpr int kPadRows = 8;   // zero rows above the x sums (the padded taps of the y pass read up to 7 of them)
 constexpr int kPadCols = 8;   // zero columns left of the reference window
 constexpr int kThreads = 256;
 
@@ -45,7 +44,7 @@ struct Layout {
   static size_t floats(int TH, int ks, int lat) {
     const int nrows = TH + ks - 1;
     return 2 * static_cast<size_t>((nrows + 1) / 2) * window_cols(ks) +
-           static_cast<size_t>(NX) * (nrows + kPadRows) * kTW * V + static_cast<size_t>(NX) * KSP * 3 * V + lat;
+           static_cast<size_t>(NX) * nrows * kTW * V + static_cast<size_t>(NX) * KSP * 3 * V + lat;
   }
 };
 
@@ -62,11 +61,11 @@ __global__ void __launch_bounds__(kThreads, GRAD ? 1 : 2) k_chi2_f(Chi2Args a, i
   constexpr int KSP = L::KSP, V = L::V;
   extern __shared__ __align__(16) float smem[];
   const int ks = a.ks, kh = (ks - 1) / 2, w = a.w, h = a.h, nc = a.nc;
-  const int nrows = TH + 2 * kh, wcols = kTW + 2 * kh, rw = window_cols(ks), trows = nrows + kPadRows;
+  const int nrows = TH + 2 * kh, wcols = kTW + 2 * kh, rw = window_cols(ks);
   const int npair = (nrows + 1) / 2;
   float* win = smem;                         // npair x rw row pairs; column kPadCols + c <-> frame column bx - kh + c
-  float* tx = win + 2 * npair * rw;          // NX x trows x kTW x V
-  float* gy = tx + NX * trows * kTW * V;     // NX x KSP, then (GRAD) g'_y
+  float* tx = win + 2 * npair * rw;          // NX x nrows x kTW x V
+  float* gy = tx + NX * nrows * kTW * V;     // NX x KSP, then (GRAD) g'_y
   float* gx2 = gy + NX * KSP * V;            // NX x KSP pairs, then (GRAD) g'_x
   float* slat = gx2 + 2 * NX * KSP * V;      // nf x lly x llx
   const int bx = blockIdx.x * kTW, by = blockIdx.y * TH, tid = threadIdx.x;
@@ -97,10 +96,6 @@ __global__ void __launch_bounds__(kThreads, GRAD ? 1 : 2) k_chi2_f(Chi2Args a, i
       reinterpret_cast<float2*>(gx2)[NX * KSP + i] =
           in ? make_float2(a.dgx[q * ks + j], a.dgx[q * ks + j]) : make_float2(0.0f, 0.0f);
     }
-  }
-  for (int i = tid; i < NX * kPadRows * kTW * V; i += kThreads) {
-    const int q = i / (kPadRows * kTW * V);
-    tx[q * trows * kTW * V + (i - q * kPadRows * kTW * V)] = 0.0f;
   }
   for (int i = tid; i < 2 * npair * rw; i += kThreads) {
     const int r = i / rw, cc = i - r * rw, c = cc - kPadCols;
@@ -148,7 +143,7 @@ __global__ void __launch_bounds__(kThreads, GRAD ? 1 : 2) k_chi2_f(Chi2Args a, i
     const int r = 2 * rp;
 #pragma unroll
     for (int q = 0; q < NX; ++q) {
-      float* o = tx + ((q * trows + kPadRows + r) * kTW + c0) * V;
+      float* o = tx + ((q * nrows + r) * kTW + c0) * V;
       if (GRAD) {
         *reinterpret_cast<float4*>(o) = make_float4(acc[0][q][0].x, acc[V - 1][q][0].x, acc[0][q][1].x, acc[V - 1][q][1].x);
         if (r + 1 < nrows)
@@ -222,10 +217,10 @@ __global__ void __launch_bounds__(kThreads, GRAD ? 1 : 2) k_chi2_f(Chi2Args a, i
     for (int i = 0; i < R; ++i)
 #pragma unroll
       for (int u = 0; u < COLS; ++u) m0[i][u] = mx[i][u] = my[i][u] = 0.0f;
-    const int base = kPadRows + ly + 2 * kh;  // x-sum row of output row 0, tap 0
+    const int base = ly + 2 * kh;  // x-sum row of output row 0, tap 0
     for (int c = 0; c < nc; ++c) {
       const int2 o = a.orders[c];
-      const float2* col = reinterpret_cast<const float2*>(tx + static_cast<size_t>(o.x) * trows * kTW * V + lx * V);
+      const float2* col = reinterpret_cast<const float2*>(tx + static_cast<size_t>(o.x) * nrows * kTW * V + lx * V);
       const float* g0 = gy + o.y * KSP;
       float2 cc[R];  // GRAD: (C, C^x) of row i; else C of the two columns
       float cy[R];
