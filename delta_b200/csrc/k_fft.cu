@@ -962,8 +962,9 @@ __host__ __device__ constexpr int cp_lines(int n, int k, int nc) {  // float2 of
 // zero) and the column transforms, C columns at a time, none of it through global
 // memory; CTA y of a cell takes every gridDim.y-th group of columns. The arithmetic
 // is that of the passes it replaces (k_local_kernels, k_rows_fwd, k_cols), which
-// wrote and read the dense image and the whole spectrum: 141 us at 465 cells of 256 x
-// 256, where they took 426 us. Bound as k_block_filter is, by the line transforms.
+// wrote and read the dense image and the whole spectrum: 123 us at 465 cells of 256 x
+// 256, where they took 426 us. Bound as k_block_filter is, by the line transforms. Three
+// CTAs an SM leave 80 registers, 32 bytes a thread of them spilled.
 template <int N>
 __global__ void __launch_bounds__(256, 3)
 k_cell_power(FftGeom G, TpsDev t, const double* __restrict__ theta, int nc, const float* __restrict__ phi, int ks,
@@ -1126,8 +1127,10 @@ bool cell_power_fused(const FftGeom& g, int ks, int knots, int nc) {
 void launch_cell_power(cudaStream_t s, const FftGeom& g, int ncell, const TpsDev& t, const double* theta, int nc,
                        const float* phi, int ks, const double* centres, double* sumk2, double* power) {
   // Column groups over several CTAs per cell while there are fewer than four per SM;
-  // with more cells each CTA would repeat the kernel and its rows for nothing (465
-  // cells: 1, 2, 3, 5 and 9 CTAs each take 141, 153, 149, 146 and 172 us).
+  // with more cells each CTA would repeat the kernel and its rows for nothing. us for 1,
+  // 2, 3, 5 and 9 CTAs a cell: 961 cells 196, 262, 281, 293, 314; 465 cells 123, 124,
+  // 124, 123, 150; 128 cells 54, 38, 34, 41, 46 (the rule's 4: 41); 32 cells 54, 34, 24,
+  // 20, 16.
   const int groups = (g.n / 2 + 1 + kCpCols - 1) / kCpCols;
   const int split = std::min(groups, std::max(1, 148 * 4 / std::max(ncell, 1)));
   const size_t smem = cell_power_smem(g, ks, t.k, nc);
